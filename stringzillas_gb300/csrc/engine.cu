@@ -90,11 +90,15 @@ static scope_t *as_scope(void *handle) noexcept {
 }
 
 static int visible_devices() noexcept {
-    int count = 0;
+    // A process's visible devices do not change once the runtime has found any; until then every call asks again.
+    static std::atomic<int> found {0};
+    int count = found.load(std::memory_order_relaxed);
+    if (count > 0) return count;
     if (cudaGetDeviceCount(&count) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
+    found.store(count, std::memory_order_relaxed);
     return count;
 }
 
@@ -1990,6 +1994,9 @@ struct fingerprint_engine_t {
     std::uint32_t magic = fingerprint_magic_k;
     std::uint32_t dimensions = 0;
     std::vector<fingerprint_dim_t> params;
+    std::vector<fingerprint_weights_t> weights;
+    std::vector<fingerprint_group_t> group_list; // groups of 64 dimensions, class by class
+    fingerprint_groups_t groups {};
     device_context_t devices[max_devices_k];
     device_buffer_t params_device[max_devices_k];
     device_buffer_t outputs[max_devices_k];
@@ -2032,8 +2039,12 @@ sz_status_t create_fingerprints(std::size_t dimensions, std::size_t alphabet_siz
     engine->dimensions = (std::uint32_t)dimensions;
     bool const sliced = dimensions % widths_count == 0 && (dimensions / widths_count) % 64 == 0;
     engine->params.resize(dimensions);
+    engine->weights.resize(dimensions);
     for (std::size_t d = 0; d < dimensions; ++d)
-        engine->params[d] = fingerprint_dimension(d, widths[(sliced ? d / 64 : d) % widths_count], seed);
+        engine->params[d] = fingerprint_dimension(d, widths[(sliced ? d / 64 : d) % widths_count], seed,
+                                                  engine->weights[d]);
+    engine->group_list.resize((dimensions + fingerprint_group_k - 1) / fingerprint_group_k);
+    engine->groups = fingerprint_groups(engine->params.data(), engine->dimensions, engine->group_list.data());
     *engine_out = engine;
     return report({}, error_message);
 }
@@ -2073,11 +2084,22 @@ sz_status_t fingerprint_call(void *engine_handle, void *scope_handle, tape_view_
     // Parameters, once per device.
     device_buffer_t &params = engine->params_device[device];
     std::size_t const params_bytes = engine->params.size() * sizeof(fingerprint_dim_t);
-    if (params.bytes < params_bytes) {
-        status = params.reserve(params_bytes, stream);
+    std::size_t const weights_at = align_up(params_bytes, 256);
+    std::size_t const weights_bytes = engine->weights.size() * sizeof(fingerprint_weights_t);
+    std::size_t const list_at = align_up(weights_at + weights_bytes, 256);
+    std::size_t const list_bytes = engine->group_list.size() * sizeof(fingerprint_group_t);
+    if (params.bytes < list_at + list_bytes) {
+        status = params.reserve(list_at + list_bytes, stream);
         if (!status.ok()) return report(status, error_message);
-        cudaError_t const copied = cudaMemcpyAsync(params.data, engine->params.data(), params_bytes,
-                                                   cudaMemcpyHostToDevice, stream);
+        auto *area = static_cast<unsigned char *>(params.data);
+        cudaError_t copied =
+            cudaMemcpyAsync(area, engine->params.data(), params_bytes, cudaMemcpyHostToDevice, stream);
+        if (copied == cudaSuccess)
+            copied = cudaMemcpyAsync(area + weights_at, engine->weights.data(), weights_bytes, cudaMemcpyHostToDevice,
+                                     stream);
+        if (copied == cudaSuccess)
+            copied = cudaMemcpyAsync(area + list_at, engine->group_list.data(), list_bytes, cudaMemcpyHostToDevice,
+                                     stream);
         if (copied != cudaSuccess) return report(from_cuda(copied), error_message);
     }
     // Outputs: in place when device-reachable, else through a dense device buffer and 2-D copies.
@@ -2093,9 +2115,12 @@ sz_status_t fingerprint_call(void *engine_handle, void *scope_handle, tape_view_
         if (!counts_on_device)
             counts_target = reinterpret_cast<std::uint32_t *>(area + dense_bytes), counts_pitch = row_bytes;
     }
-    cudaError_t error = launch_fingerprints(staged, static_cast<fingerprint_dim_t const *>(params.data),
-                                            engine->dimensions, hashes_target, hashes_pitch, counts_target,
-                                            counts_pitch, context->sm_count, stream);
+    auto const *area = static_cast<unsigned char const *>(params.data);
+    cudaError_t error = launch_fingerprints(
+        staged, reinterpret_cast<fingerprint_dim_t const *>(area),
+        reinterpret_cast<fingerprint_weights_t const *>(area + weights_at), engine->dimensions,
+        reinterpret_cast<fingerprint_group_t const *>(area + list_at), engine->groups, hashes_target, hashes_pitch,
+        counts_target, counts_pitch, context->sm_count, stream);
     if (error == cudaSuccess && !hashes_on_device)
         error = cudaMemcpy2DAsync(hashes, hashes_stride, hashes_target, row_bytes, row_bytes, texts.count,
                                   cudaMemcpyDeviceToHost, stream);

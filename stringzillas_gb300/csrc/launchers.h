@@ -31,16 +31,41 @@ cudaError_t launch_myers_direct(plan_args_t const &args, std::int64_t *out, std:
 cudaError_t launch_scatter_output(plan_args_t const &args, std::int64_t const *results, std::int64_t *out,
                                   std::uint64_t stride, int sm_count, cudaStream_t stream);
 
+constexpr int fingerprint_tensor_width_k = 32; // widest window the tensor-core kernel takes
+constexpr int fingerprint_group_k = 64;        // dimensions a warp of that kernel scores
+
 /** One Min-Hash dimension: modulus m (2^42 < m < 2^43), multiplier a (< 640), D = -a^w mod m, the quotient
- *  estimate's constant mu = floor(2^74 / m) (< 2^32), window width w. */
+ *  estimate's constant mu = floor(2^74 / m) (< 2^32), window width w; for windows of up to 32 bytes the scale of the
+ *  estimates (2^shift) and, in units of 2^-32, the constant of the centred bytes and the bound of the weights'
+ *  rounding. 40 bytes: the rolling kernel's warps read them for every text, and 1,024 of them have to stay in L1. */
 struct fingerprint_dim_t {
     std::uint64_t modulo, discard;
-    std::uint32_t multiplier, mu, width, reserved;
+    std::uint32_t multiplier, mu, width, margin, offset, shift;
+};
+/** The weights 2^shift * a^(w-1-i) / m of a window's bytes as two signed digits in half precision (high, low: units of
+ *  2^-11 and 2^-22), zero from w on. */
+struct fingerprint_weights_t {
+    std::uint16_t digits[2][fingerprint_tensor_width_k];
 };
 /** The reference's parameters of dimension @p dim for a window of @p width bytes and a reproducibility @p seed. */
-fingerprint_dim_t fingerprint_dimension(std::uint64_t dim, std::uint64_t width, std::uint64_t seed);
-/** Min-Hash fingerprints of every text: rows `hashes_stride` / `counts_stride` bytes apart, `dimensions` columns. */
-cudaError_t launch_fingerprints(tape_t const &texts, fingerprint_dim_t const *params, std::uint32_t dimensions,
+fingerprint_dim_t fingerprint_dimension(std::uint64_t dim, std::uint64_t width, std::uint64_t seed,
+                                        fingerprint_weights_t &weights);
+/** A group of 64 consecutive dimensions and the width of its widest window. */
+struct fingerprint_group_t {
+    std::uint32_t index, widest;
+};
+/** How many groups have windows of up to 16 bytes, up to 32, and wider ones. */
+struct fingerprint_groups_t {
+    std::uint32_t count[3];
+};
+/** Fills @p groups (one entry per 64 dimensions), class by class. */
+fingerprint_groups_t fingerprint_groups(fingerprint_dim_t const *params, std::uint32_t dimensions,
+                                        fingerprint_group_t *groups);
+/** Min-Hash fingerprints of every text: rows `hashes_stride` / `counts_stride` bytes apart, `dimensions` columns;
+ *  `group_list` is the device copy of what `fingerprint_groups` filled. */
+cudaError_t launch_fingerprints(tape_t const &texts, fingerprint_dim_t const *params,
+                                fingerprint_weights_t const *weights, std::uint32_t dimensions,
+                                fingerprint_group_t const *group_list, fingerprint_groups_t const &groups,
                                 std::uint32_t *hashes, std::uint64_t hashes_stride, std::uint32_t *counts,
                                 std::uint64_t counts_stride, int sm_count, cudaStream_t stream);
 

@@ -183,3 +183,34 @@ def test_reference_test_shapes(szs, ndim):
     again_h, again_c = engine(szs.Strs(texts))
     np.testing.assert_array_equal(again_h, hashes)
     np.testing.assert_array_equal(again_c, counts)
+
+
+@pytest.mark.parametrize("dimensions,widths", [
+    (128, [16, 17]),          # sliced: one group per tensor-core kernel
+    (256, [1, 16, 32, 33]),   # sliced: both tensor-core kernels and the rolling one
+    (70, [2, 15, 16]),        # mixed widths in a group, a ragged last group
+    (65, [31, 32]),
+    (64, [40]),
+])
+def test_window_and_chunk_edges_match_oracle(szs, dimensions, widths):
+    """Texts around the edges of the tensor-core kernel's tiles (16 windows) and chunks (256), with repeats: random
+    bytes, few letters, a period, one byte (more candidates than a chunk's list holds), and a late minimum."""
+    rng = np.random.default_rng(dimensions)
+    texts = []
+    for windows in (1, 15, 16, 17, 63, 64, 65, 255, 256, 257, 511, 512, 513, 1030):
+        for width in widths:
+            length = windows + width - 1
+            texts.append(rng.integers(0, 256, length).astype(np.uint8))
+            texts.append(rng.integers(0, 2, length).astype(np.uint8) * 255)
+            texts.append(np.resize(rng.integers(0, 256, 37), length).astype(np.uint8))
+            texts.append(np.full(length, 255, np.uint8))
+            texts.append(np.concatenate([np.full(length // 2, 120), rng.integers(0, 256, length - length // 2)])
+                         .astype(np.uint8))
+    offsets = np.zeros(len(texts) + 1, dtype=np.uint64)
+    offsets[1:] = np.cumsum([len(t) for t in texts])
+    data = np.concatenate(texts)
+    engine = szs.Fingerprints(dimensions, np.array(widths, dtype=np.uint64), seed=3)
+    hashes, counts = engine(_strs(szs, data, offsets))
+    want_h, want_c = oracle.fingerprints(dimensions, (data, offsets), widths, 3)
+    np.testing.assert_array_equal(hashes, want_h)
+    np.testing.assert_array_equal(counts, want_c)
