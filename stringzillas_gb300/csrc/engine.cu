@@ -691,6 +691,12 @@ static status_t transcode_utf8(device_context_t *context, cudaStream_t stream, t
  *  @param defer  pairwise calls with host results only: return once the work is queued, without waiting for it;
  *                `finish_deferred` later waits and fills @p stats (the pipelined driver keeps two chunks in flight).
  */
+// Groups of CTAs for a batch's largest pairs: the share of an average CTA's cells one of them should take, and the most
+// scratch the GPU's CTA slots may need (the groups' rings come on top of the single CTAs').
+constexpr double band_largest_share_k = 0.55;
+constexpr double band_largest_mean_k = 1.85; // the least cells of a grouped class, in means of the batch
+constexpr std::size_t band_largest_scratch_k = std::size_t(4) << 30;
+
 constexpr std::uint64_t alphabet_sample_bytes_k = std::uint64_t(1) << 20; // bytes per tape of a guessed alphabet
 
 static status_t run_on(engine_t const &engine, device_context_t *context, cudaStream_t stream, call_t const &call,
@@ -1032,6 +1038,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         std::size_t state_offset = 0;  // grouped band jobs: the groups' state records in the scratch buffer
         std::size_t state_bytes = 0;
         bool fills = true;             // the grid takes every resident CTA slot of its kernel on the device
+        bool first = false;            // a batch's largest pairs: launched before everything else
     };
     job_t jobs[64];
     int job_count = 0;
@@ -1057,14 +1064,77 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         group_ctas = (int)size;
         ctas = (int)(std::min<std::uint64_t>(pairs_here, slots / group_ctas) * group_ctas);
     };
+    auto band_job = [&](job_kind_t kind, int key_begin, int key_end, std::uint64_t pairs_here, int ctas, int group_ctas,
+                        dp_launch_shape_t const &shape, std::size_t bytes_per_cta) {
+        std::size_t const bytes = align_up(bytes_per_cta * (std::size_t)ctas, 256);
+        job_t job {kind, kind == job_band16_k ? 16 : 32, 0, key_begin, key_end, pairs_here, ctas, scratch_total, bytes};
+        job.fills = group_ctas > 1 || ctas >= context->sm_count * shape.ctas_per_sm;
+        job.rows = shape.rows_per_lane;
+        scratch_total += bytes;
+        if (group_ctas > 1) {
+            job.group_ctas = group_ctas, job.state_offset = scratch_total;
+            job.state_bytes = align_up((std::size_t)(ctas / group_ctas) * band_group_state_bytes(), 256);
+            scratch_total += job.state_bytes;
+        }
+        jobs[job_count++] = job;
+    };
+    // Enough long pairs to fill the GPU, but of very different sizes: a pair of many times the average CTA's share of the
+    // cells would still be running long after the others (1,024 pairs of 1,000-30,000: one of 9e8 cells against a share
+    // of 2.4e8, 46 ms on one CTA of which the other CTAs work 19; 22.6 ms with groups). So the 16-bit band's largest size
+    // classes (octaves of cells) get groups of CTAs, as many as bring a pair to about half a share, but no more than the
+    // class's smallest patterns have strips for, while they hold less than half of the call's cells and their pairs
+    // nearly twice the mean (pairs of like sizes balance by themselves: 160 pairs of 5,000-12,000 take 6.0 ms single,
+    // 8.6 ms with their largest in groups; 300 of 2,000-16,000 log-uniform 13.4 ms single, 9.6 ms). Not the 32-bit band, whose single CTAs score more per step than its groups (400 pairs of
+    // 1,100-6,000: 5.1 ms single, 7.5 ms grouped). Returns the first bin left to single CTAs; calls with few pairs are
+    // left to `band_groups`.
+    auto band_largest = [&](std::uint64_t pairs_here, dp_launch_shape_t const &shape, std::uint64_t strip_rows,
+                            std::size_t bytes_per_cta) -> int {
+        int const key_begin = bin_band16_begin_k, key_end = key_begin + bin_dp_classes_k;
+        if (schedule == szs_gb300_schedule_plain_k || shape.group_ctas_per_sm <= 0) return key_begin;
+        std::uint64_t const slots = (std::uint64_t)context->sm_count * shape.group_ctas_per_sm;
+        if (pairs_here * 2 <= slots || bytes_per_cta * slots > band_largest_scratch_k) return key_begin;
+        auto smallest = [&](int key) { return std::ldexp(1.0, 10 + bin_dp_classes_k - 1 - (key - key_begin)); };
+        double total = 0, grouped = 0;
+        for (int key = key_begin; key < key_end; ++key) total += 1.5 * smallest(key) * plan.count[key];
+        double const share = total / (double)slots;
+        std::uint64_t left = slots;
+        // A CTA alone on its SM scores nearly twice as fast as beside another: with fewer pairs than slots, two CTAs per
+        // pair gain nothing.
+        std::uint64_t const least = pairs_here < slots ? 3 : 2;
+        int key = key_begin;
+        for (; key < key_end; ++key) {
+            if (!plan.count[key]) continue;
+            grouped += 1.5 * smallest(key) * plan.count[key];
+            double const strips = smallest(key) / (double)plan.max_cols / (double)strip_rows;
+            std::uint64_t const size = std::min<std::uint64_t>(
+                {(std::uint64_t)(1.5 * smallest(key) / (band_largest_share_k * share)),
+                 (std::uint64_t)std::ceil(strips / band_warps_per_cta()), (std::uint64_t)band_group_max_ctas(), left});
+            if (size < least || grouped * 2 > total ||
+                smallest(key) < band_largest_mean_k * total / (double)pairs_here)
+                break;
+            std::uint64_t const groups = std::min<std::uint64_t>(plan.count[key], left / size);
+            band_job(job_band16_k, key, key + 1, plan.count[key], (int)(groups * size), (int)size, shape, bytes_per_cta);
+            jobs[job_count - 1].first = true;
+            left -= groups * size;
+        }
+        return key;
+    };
     {
-        std::uint64_t const pairs_here = pairs_in(bin_band16_begin_k, bin_band16_begin_k + bin_dp_classes_k);
-        if (pairs_here) {
+        std::uint64_t const all_pairs = pairs_in(bin_band16_begin_k, bin_band16_begin_k + bin_dp_classes_k);
+        if (all_pairs) {
             dp_launch_shape_t shape =
                 band16_shape(engine.kind, costs.affine != 0, packed_costs.classes, compare_mode, wide, 8);
             if (shape.ctas_per_sm <= 0) return {sz_status_unknown_k, "16-bit band kernel cannot be resident"};
+            // Local scores keep room for a 32-bit ring: a pair that reaches the 16-bit limit is scored again.
+            std::size_t const ring_scale = engine.kind == kind_smith_waterman_k ? 2 : 1;
+            std::size_t const bytes_per_cta =
+                band16_words_per_slot * 4 * ring_scale * (std::size_t)band_warps_per_cta();
+            int const rest = band_largest(all_pairs, shape, 2u * 32u * (std::uint64_t)shape.rows_per_lane, bytes_per_cta);
+            int const end = bin_band16_begin_k + bin_dp_classes_k;
+            std::uint64_t const pairs_here = pairs_in(rest, end);
             int ctas = 0, group_ctas = 1;
-            band_groups(pairs_here, shape, 2u * 32u * (std::uint64_t)shape.rows_per_lane, ctas, group_ctas);
+            if (pairs_here)
+                band_groups(pairs_here, shape, 2u * 32u * (std::uint64_t)shape.rows_per_lane, ctas, group_ctas);
             // Groups limited by their pairs' super-strips while the GPU has CTA slots to spare (a handful of long
             // pairs) take 4 rows per lane: twice the super-strips, so a pair spreads over twice the warps, each step
             // about half as long. Groups that fill the GPU keep 8 rows, which do more cells per step's overhead.
@@ -1076,21 +1146,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
                     band_groups(pairs_here, narrow, 2u * 32u * 4u, narrow_ctas, narrow_group);
                 if (narrow_group > group_ctas) shape = narrow, ctas = narrow_ctas, group_ctas = narrow_group;
             }
-            // Local scores keep room for a 32-bit ring: a pair that reaches the 16-bit limit is scored again.
-            std::size_t const ring_scale = engine.kind == kind_smith_waterman_k ? 2 : 1;
-            std::size_t const bytes = align_up(band16_words_per_slot * 4 * ring_scale * (std::size_t)ctas *
-                                                   (std::size_t)band_warps_per_cta(), 256);
-            job_t job {job_band16_k, 16, 0, bin_band16_begin_k, bin_band16_begin_k + bin_dp_classes_k, pairs_here,
-                       ctas, scratch_total, bytes};
-            job.fills = group_ctas > 1 || ctas >= context->sm_count * shape.ctas_per_sm;
-            job.rows = shape.rows_per_lane;
-            scratch_total += bytes;
-            if (group_ctas > 1) {
-                job.group_ctas = group_ctas, job.state_offset = scratch_total;
-                job.state_bytes = align_up((std::size_t)(ctas / group_ctas) * band_group_state_bytes(), 256);
-                scratch_total += job.state_bytes;
-            }
-            jobs[job_count++] = job;
+            if (pairs_here) band_job(job_band16_k, rest, end, pairs_here, ctas, group_ctas, shape, bytes_per_cta);
         }
     }
     {
@@ -1109,19 +1165,8 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
                 if (narrow.ctas_per_sm > 0) band_groups(pairs_here, narrow, 32u * 4u, narrow_ctas, narrow_group);
                 if (narrow_group > group_ctas) shape = narrow, ctas = narrow_ctas, group_ctas = narrow_group;
             }
-            std::size_t const bytes =
-                align_up(cells_per_warp * 4 * (std::size_t)ctas * (std::size_t)band_warps_per_cta(), 256);
-            job_t job {job_band_k, 32, 0, bin_band_begin_k, bin_band_begin_k + bin_dp_classes_k, pairs_here, ctas,
-                       scratch_total, bytes};
-            job.fills = group_ctas > 1 || ctas >= context->sm_count * shape.ctas_per_sm;
-            job.rows = shape.rows_per_lane;
-            scratch_total += bytes;
-            if (group_ctas > 1) {
-                job.group_ctas = group_ctas, job.state_offset = scratch_total;
-                job.state_bytes = align_up((std::size_t)(ctas / group_ctas) * band_group_state_bytes(), 256);
-                scratch_total += job.state_bytes;
-            }
-            jobs[job_count++] = job;
+            band_job(job_band_k, bin_band_begin_k, bin_band_begin_k + bin_dp_classes_k, pairs_here, ctas, group_ctas,
+                     shape, cells_per_warp * 4 * (std::size_t)band_warps_per_cta());
         }
     }
     for (int cell_bits : {64, 32}) {
@@ -1236,7 +1281,8 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
     // last pair, so a small job launched after it would only start at the end and add its whole time to the call.
     // Launched first, it takes its few slots and runs beside the large grids, which balance over their cursor.
     if (schedule != szs_gb300_schedule_plain_k)
-        std::stable_partition(jobs, jobs + job_count, [](job_t const &job) { return !job.fills; });
+        std::stable_partition(jobs, jobs + job_count, [](job_t const &job) { return job.first || !job.fills; }),
+            std::stable_partition(jobs, jobs + job_count, [](job_t const &job) { return job.first; });
     if (scratch_total) {
         status = context->scratch.reserve(scratch_total, stream);
         if (!status.ok()) return status;

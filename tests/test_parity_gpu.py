@@ -1084,3 +1084,22 @@ def test_long_unit_levenshtein_chain_waves(szs, port):
     second = [bytes(rng.choice(DNA, size=int(n) + int(rng.integers(0, 200)))) for n in lengths]
     got = szs.LevenshteinDistances().pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
     np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_costs(), tape(first), tape(second)))
+
+
+@pytest.mark.parametrize("family,costs,alphabet,count", [("sw", (-5, -2), DNA, 360), ("lev", (0, 2, 3, 1), None, 170)])
+def test_largest_pairs_of_a_batch_take_groups(szs, port, family, costs, alphabet, count):
+    """Batches that fill the GPU's CTA slots (or half of them) with 16-bit band pairs, a few of them many times the mean:
+    the largest size classes take groups of CTAs beside the others' single CTAs, with both kernels in one call. Local
+    scores past the 16-bit limit (identical strings) among them."""
+    rng = np.random.default_rng(count)
+    b2c, table = dna_tables()
+    letters = np.arange(32, 127, dtype=np.uint8) if alphabet is None else alphabet
+    lengths = [(int(rng.integers(2050, 2400)), int(rng.integers(2050, 2600))) for _ in range(count)]
+    lengths += [(9000, 9500), (8200, 16000), (12000, 8500)] if family == "sw" else [(7000, 7100), (6900, 7300)]
+    first = [bytes(rng.choice(letters, size=n)) for n, _ in lengths]
+    second = [bytes(rng.choice(letters, size=m)) for _, m in lengths]
+    if family == "sw":
+        first.append(first[-1] * 2), second.append(first[-1])  # gain 2 x 24,000: rescored on 32-bit cells
+    engine, oracle_costs = make_engine(szs, family, costs, b2c, table)
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    np.testing.assert_array_equal(got, port.pairs(oracle_costs, tape(first), tape(second)))
