@@ -1,16 +1,24 @@
 /**
  *  @file direct.cu
- *  @brief Cross products of short tokens under unit-cost Levenshtein: one thread per output cell, no planning.
+ *  @brief Cross products under unit-cost Levenshtein: one thread per output cell, a query's match masks shared by the
+ *         CTA, no planning.
  *
- *  A cross-product call over strings of at most 64 bytes spends most of its time in planning when it
- *  takes the general path: the pair enumeration, binning and task scatter touch every pair, and a host round trip
- *  separates planning from scoring. When every string of both tapes has at most 64 bytes, each output cell is one
- *  bit-parallel distance over a pattern of at most two 32-bit words, cheap enough to compute where it lands. So one
- *  kernel takes one cell per thread (a query per grid row, candidates across the row, so no division per cell): it
- *  reads the two strings through the tapes' offsets, lays the shorter one's bytes out as 8 bit planes of one or two
- *  words, runs the Myers / Hyyrö step over the longer one's bytes (match masks from the planes, one logic operation
- *  per plane and word), and writes the distance into the caller's matrix. A string longer than 64 bytes raises a
- *  flag instead; the host then runs the general path for the whole call, which writes every cell again.
+ *  In a cross product every query meets every candidate, so what the pairwise kernels prepare per pair (code planes or
+ *  match masks of the pattern, a task record, a bin) is the same for a whole row of cells. Here a CTA takes one query
+ *  as the pattern and a block of candidates: it writes the query's match masks once into a shared table indexed by the
+ *  byte itself (no alphabet pass), each thread runs the Myers / Hyyrö step over its candidate with the pattern's deltas
+ *  in registers (up to 1,024 rows in 32 words), and writes the distance where it lands in the caller's matrix. A text
+ *  column costs one shared load per four words (16-byte loads; rows of the table are an odd number of 16-byte units
+ *  apart, so the few letters of a DNA text fall into different banks), and ten integer operations per word, which bound
+ *  the kernel: the warp-per-pair kernel spends about 45 on a step of one word per lane.
+ *
+ *  Measured (device-resident, whole calls): 197 x 198 strings of 1,000 bytes 3.16 ms on the planned warp-per-pair route,
+ *  1.01 ms here; 2,048 x 2,048 tokens of 4-16 bytes 0.25 ms with the pattern's bit planes built by every thread, 0.12 ms
+ *  here; 197 x 198 of 100 bytes 112 us planned, 52 us here.
+ *
+ *  Either side may be the pattern: the queries, unless they are longer than 1,024 bytes and the candidates are not.
+ *  Words are chosen per pattern inside a kernel, in steps that fit its class (up to 128, 512 and 1,024 rows), which the
+ *  host picks by the longest pattern; classes keep the registers of the long patterns off the short ones.
  *
  *  Counterpart of the reference's single-word direct path for tiny-token cross products
  *  (include/stringzillas/similarities/cuda.cuh:3892-3936); the distances are those of the serial engine
@@ -42,39 +50,43 @@ __device__ __forceinline__ void direct_string(tape_t const &tape, std::uint64_t 
     length = end - begin;
 }
 
-/** Unit-cost edit distance of a pattern of 1..32 x `words_` bytes against a text of 1..64 bytes. */
+/** Bytes between two rows of the match-mask table of patterns of `words` words. */
+__host__ __device__ constexpr int direct_row_bytes(int words) {
+    return words <= 2 ? 4 * words : 16 * (((words + 3) / 4) | 1);
+}
+
+/** The unit-cost edit distance of the CTA's pattern (n rows, masks in `table`) and a text of 1 or more bytes. */
 template <int words_>
-__device__ __forceinline__ std::uint32_t direct_distance(std::uint8_t const *pattern, std::uint32_t n,
+__device__ __forceinline__ std::uint32_t direct_distance(unsigned char const *table, std::uint32_t n,
                                                         std::uint8_t const *text, std::uint32_t m) {
-    constexpr int W = words_;
-    std::uint32_t planes[8][W];
-#pragma unroll
-    for (int w = 0; w < W; ++w) {
-#pragma unroll
-        for (int b = 0; b < 8; ++b) planes[b][w] = 0u;
-        std::uint32_t const rows = n > 32u * w ? min(32u, n - 32u * w) : 0u;
-        for (std::uint32_t k = 0; k < rows; ++k) {
-            std::uint32_t const byte = pattern[32u * w + k];
-#pragma unroll
-            for (int b = 0; b < 8; ++b) planes[b][w] |= ((byte >> b) & 1u) << k;
-        }
-    }
+    constexpr int W = words_, Q = (W + 3) / 4;
     std::uint32_t pv[W], mv[W];
 #pragma unroll
     for (int w = 0; w < W; ++w) pv[w] = 0xFFFFFFFFu, mv[w] = 0u;
-    for (std::uint32_t j = 0; j < m; ++j) {
-        std::uint32_t const byte = text[j];
-        std::uint32_t eq[W], xv[W], sum[W];
+    auto column = [&](std::uint32_t byte) {
+        unsigned char const *masks = table + byte * direct_row_bytes(W);
+        std::uint32_t eq[4 * Q], xv[W], sum[W];
+        if constexpr (W == 1) eq[0] = *reinterpret_cast<std::uint32_t const *>(masks);
+        else if constexpr (W == 2) {
+            uint2 const v = *reinterpret_cast<uint2 const *>(masks);
+            eq[0] = v.x, eq[1] = v.y;
+        }
+        else {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                uint4 const v = *reinterpret_cast<uint4 const *>(masks + 16 * q);
+                eq[4 * q] = v.x, eq[4 * q + 1] = v.y, eq[4 * q + 2] = v.z, eq[4 * q + 3] = v.w;
+            }
+        }
 #pragma unroll
         for (int w = 0; w < W; ++w) {
-            eq[w] = 0xFFFFFFFFu;
-#pragma unroll
-            for (int b = 0; b < 8; ++b) eq[w] &= planes[b][w] ^ (((byte >> b) & 1u) - 1u);
             xv[w] = eq[w] | mv[w];
             sum[w] = eq[w] & pv[w];
         }
-        if constexpr (W == 1) sum[0] += pv[0];
-        else asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;" : "+r"(sum[0]), "+r"(sum[1]) : "r"(pv[0]), "r"(pv[1]));
+        // Multi-word (Eq & Pv) + Pv: one add per word, the carry rippling upwards through the carry flag.
+        asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(sum[0]) : "r"(pv[0]));
+#pragma unroll
+        for (int w = 1; w < W; ++w) asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(sum[w]) : "r"(pv[w]));
         std::uint32_t ph_prev = 1u << 31, mh_prev = 0u; // +1 shifted into row 0
 #pragma unroll
         for (int w = 0; w < W; ++w) {
@@ -87,7 +99,22 @@ __device__ __forceinline__ std::uint32_t direct_distance(std::uint8_t const *pat
             mv[w] = ph_shifted & xv[w];
             ph_prev = ph, mh_prev = mh;
         }
+    };
+    // The text four bytes at a time from aligned words (never past the one holding its last byte), shifted to the
+    // text's own alignment so that a warp's lanes step together whatever theirs; the next word is in flight meanwhile.
+    std::uintptr_t const address = reinterpret_cast<std::uintptr_t>(text);
+    std::uint32_t const *aligned = reinterpret_cast<std::uint32_t const *>(address & ~std::uintptr_t(3));
+    std::uint32_t const skew = (std::uint32_t)(address & 3), last = (skew + m - 1) >> 2;
+    std::uint32_t low = __ldg(aligned), high = last >= 1 ? __ldg(aligned + 1) : 0u;
+    for (std::uint32_t c = 0; c < m / 4; ++c) {
+        std::uint32_t const four = __funnelshift_r(low, high, 8 * skew);
+        low = high;
+        if (c + 2 <= last) high = __ldg(aligned + c + 2);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) column(__byte_perm(four, 0u, 0x4440u + k));
     }
+    std::uint32_t rest = __funnelshift_r(low, high, 8 * skew);
+    for (std::uint32_t j = 0; j < (m & 3u); ++j, rest >>= 8) column(rest & 0xFFu);
     // D[n][m] = m + (rows 1..n of the last column's +1 deltas) - (its -1 deltas).
     std::uint32_t distance = m;
 #pragma unroll
@@ -99,46 +126,119 @@ __device__ __forceinline__ std::uint32_t direct_distance(std::uint8_t const *pat
     return distance;
 }
 
-/** One output cell per thread: queries along the grid's y dimension, candidates along x (no division per cell). */
-__global__ void __launch_bounds__(256) myers_direct_kernel(plan_args_t const args, std::int64_t *__restrict__ out,
-                                                           std::uint64_t stride, std::uint32_t *__restrict__ flag) {
-    std::uint64_t const queries = args.queries.count, candidates = args.candidates_count;
-    for (std::uint64_t q = blockIdx.y; q < queries; q += gridDim.y) {
-        std::uint8_t const *first;
+/** A pattern's row of cells with the fewest words of the class that hold it (`words_`, or steps above). */
+template <int words_, int step_, int most_, typename visit_>
+__device__ __forceinline__ void direct_with_words(std::uint32_t words, visit_ &&visit) {
+    if constexpr (words_ + step_ <= most_)
+        if (words > words_) return direct_with_words<words_ + step_, step_, most_>(words, visit);
+    visit(std::integral_constant<int, words_> {});
+}
+
+/**
+ *  One pattern per CTA and round, one cell per thread and round: patterns along the grid's y dimension, texts along x.
+ *  `swapped`: the patterns are the candidates.
+ */
+template <int first_, int step_, int most_>
+__global__ void __launch_bounds__(256, most_ <= 4 ? 5 : (most_ <= 16 ? 3 : 2))
+    myers_direct_kernel(tape_t const patterns, tape_t const texts, int const swapped, std::int64_t *__restrict__ out,
+                        std::uint64_t const stride) {
+    extern __shared__ __align__(16) unsigned char masks_s[];
+    for (std::uint64_t p = blockIdx.y; p < patterns.count; p += gridDim.y) {
+        std::uint8_t const *pattern;
         std::uint64_t n;
-        direct_string(args.queries, q, first, n);
-        for (std::uint64_t c = (std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < candidates;
-             c += (std::uint64_t)gridDim.x * blockDim.x) {
-            std::uint8_t const *second;
-            std::uint64_t m;
-            direct_string(args.candidates, c, second, m);
-            if (n > 64u || m > 64u) {
-                atomicOr(flag, 1u);
-                continue;
+        direct_string(patterns, p, pattern, n);
+        direct_with_words<first_, step_, most_>((std::uint32_t)((n + 31) / 32), [&](auto words) {
+            constexpr int W = decltype(words)::value;
+            constexpr int row_words = direct_row_bytes(W) / 4;
+            auto *table = reinterpret_cast<std::uint32_t *>(masks_s);
+            __syncthreads(); // the previous pattern's readers are done
+            for (std::uint32_t i = threadIdx.x; i < 256u * row_words; i += blockDim.x) table[i] = 0u;
+            __syncthreads();
+            for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+                atomicOr(&table[(std::uint32_t)pattern[i] * row_words + (i >> 5)], 1u << (i & 31u));
+            __syncthreads();
+            for (std::uint64_t t = (std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < texts.count;
+                 t += (std::uint64_t)gridDim.x * blockDim.x) {
+                std::uint8_t const *text;
+                std::uint64_t m;
+                direct_string(texts, t, text, m);
+                std::uint32_t const distance =
+                    n && m ? direct_distance<W>(masks_s, (std::uint32_t)n, text, (std::uint32_t)m)
+                           : (std::uint32_t)(n + m);
+                out[swapped ? t * stride + p : p * stride + t] = distance;
             }
-            std::uint32_t distance;
-            bool const swap = m < n;
-            std::uint8_t const *pattern = swap ? second : first, *text = swap ? first : second;
-            std::uint32_t const rows = (std::uint32_t)(swap ? m : n), cols = (std::uint32_t)(swap ? n : m);
-            if (rows == 0) distance = cols;
-            else if (rows <= 32u) distance = direct_distance<1>(pattern, rows, text, cols);
-            else distance = direct_distance<2>(pattern, rows, text, cols);
-            out[q * stride + c] = distance;
-        }
+        });
+    }
+}
+
+/** The longest string of each tape (one CTA each), and its data's bytes, straight into page-locked host memory. */
+__global__ void __launch_bounds__(1024) direct_extents_kernel(tape_t const queries, tape_t const candidates,
+                                                              std::uint64_t *__restrict__ extents) {
+    __shared__ unsigned long long longest_s;
+    if (threadIdx.x == 0) longest_s = 0;
+    __syncthreads();
+    tape_t const &tape = blockIdx.x ? candidates : queries;
+    unsigned long long longest = 0;
+#pragma unroll 8
+    for (std::uint64_t i = threadIdx.x; i < tape.count; i += blockDim.x) {
+        std::uint8_t const *start;
+        std::uint64_t length;
+        direct_string(tape, i, start, length);
+        longest = max(longest, (unsigned long long)length);
+    }
+#pragma unroll
+    for (int distance = 16; distance; distance >>= 1)
+        longest = max(longest, __shfl_xor_sync(0xFFFFFFFFu, longest, distance));
+    if ((threadIdx.x & 31) == 0) atomicMax(&longest_s, longest);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        std::uint8_t const *first, *end;
+        std::uint64_t length;
+        direct_string(tape, 0, first, length);
+        direct_string(tape, tape.count - 1, end, length);
+        extents[2 * blockIdx.x] = longest_s;
+        extents[2 * blockIdx.x + 1] = (std::uint64_t)(end + length - first);
     }
 }
 
 } // namespace
 
-cudaError_t launch_myers_direct(plan_args_t const &args, std::int64_t *out, std::uint64_t stride,
-                                std::uint32_t *flag, int sm_count, cudaStream_t stream) {
-    if (args.mode != mode_cross_k) return cudaErrorInvalidValue;
-    std::uint64_t const columns = (args.candidates_count + 255) / 256;
-    unsigned const grid_x = (unsigned)(columns < 64 ? (columns ? columns : 1) : 64);
-    std::uint64_t const rows_wanted = ((std::uint64_t)sm_count * 16 + grid_x - 1) / grid_x;
-    unsigned const grid_y = (unsigned)std::min<std::uint64_t>(std::min<std::uint64_t>(args.queries.count, rows_wanted),
-                                                              65535);
-    myers_direct_kernel<<<dim3(grid_x, grid_y ? grid_y : 1), 256, 0, stream>>>(args, out, stride, flag);
+cudaError_t launch_direct_extents(tape_t const &queries, tape_t const &candidates, std::uint64_t *extents,
+                                  cudaStream_t stream) {
+    direct_extents_kernel<<<2, 1024, 0, stream>>>(queries, candidates, extents);
+    return cudaGetLastError();
+}
+
+bool myers_direct_takes(std::uint64_t longest_query, std::uint64_t longest_candidate, std::uint64_t pairs,
+                        bool &swapped) {
+    swapped = longest_query > direct_max_rows_k && longest_candidate <= direct_max_rows_k;
+    std::uint64_t const rows = swapped ? longest_candidate : longest_query;
+    if (rows > direct_max_rows_k || longest_query >= (1ull << 31) || longest_candidate >= (1ull << 31)) return false;
+    return rows <= 512 || pairs >= direct_min_pairs_k;
+}
+
+cudaError_t launch_myers_direct(tape_t const &queries, tape_t const &candidates, bool swapped, std::uint64_t longest_rows,
+                                std::int64_t *out, std::uint64_t stride, int sm_count, cudaStream_t stream) {
+    tape_t const &patterns = swapped ? candidates : queries, &texts = swapped ? queries : candidates;
+    // Small CTAs while there are few cells for the SMs, so that the last round is even; larger ones share a pattern's
+    // table among more threads.
+    unsigned threads = 256;
+    while (threads > 64 && patterns.count * ((texts.count + threads - 1) / threads) < (std::uint64_t)sm_count * 8)
+        threads /= 2;
+    std::uint64_t const columns = (texts.count + threads - 1) / threads;
+    unsigned const grid_x = (unsigned)std::min<std::uint64_t>(columns, 1024);
+    std::uint64_t const wanted = ((std::uint64_t)sm_count * 32 + grid_x - 1) / grid_x;
+    unsigned const grid_y = (unsigned)std::min<std::uint64_t>({patterns.count, wanted, 65535});
+    dim3 const grid(grid_x, grid_y);
+    int const set = swapped ? 1 : 0;
+    if (longest_rows <= 128)
+        myers_direct_kernel<1, 1, 4><<<grid, threads, 256 * direct_row_bytes(4), stream>>>(patterns, texts, set, out, stride);
+    else if (longest_rows <= 512)
+        myers_direct_kernel<2, 2, 16><<<grid, threads, 256 * direct_row_bytes(16), stream>>>(patterns, texts, set, out,
+                                                                                            stride);
+    else
+        myers_direct_kernel<4, 4, 32><<<grid, threads, 256 * direct_row_bytes(32), stream>>>(patterns, texts, set, out,
+                                                                                            stride);
     return cudaGetLastError();
 }
 

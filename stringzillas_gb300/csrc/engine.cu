@@ -287,11 +287,7 @@ struct device_context_t {
     batch_alphabet_t *alphabet_host() const noexcept {
         return reinterpret_cast<batch_alphabet_t *>(static_cast<unsigned char *>(readback.data) + sizeof(plan_bins_t));
     }
-    /** 256 spare bytes after the plan and the alphabet, on the device and in the pinned readback area. */
-    std::uint32_t *spare_device() const noexcept {
-        return reinterpret_cast<std::uint32_t *>(static_cast<unsigned char *>(control.data) + sizeof(plan_bins_t) +
-                                                 sizeof(batch_alphabet_t));
-    }
+    /** 256 spare bytes after the plan and the alphabet of the pinned readback area. */
     std::uint64_t *spare_host() const noexcept {
         return reinterpret_cast<std::uint64_t *>(static_cast<unsigned char *>(readback.data) + sizeof(plan_bins_t) +
                                                  sizeof(batch_alphabet_t));
@@ -763,45 +759,45 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         args.wide = wide ? 1 : 0;
     }
 
-    // Cross products of short tokens under unit costs, into device-resident results: when both tapes hold at most 64
-    // bytes per string on average, one kernel scores every cell in place (one thread per cell, no planning); a
-    // string longer than 64 bytes raises its flag, and the general path below scores the call.
-    if (engine.unit_levenshtein && !engine.utf8 && call.mode == mode_cross_k && schedule != szs_gb300_schedule_plain_k &&
-        !defer && device_accessible(call.out)) {
-        std::uint64_t *ends = context->spare_host(); // offsets[0] and offsets[count] of both tapes
-        tape_t const *tapes[2] = {&args.queries, &args.candidates};
-        for (int k = 0; k < 2; ++k) {
-            std::size_t const width = tapes[k]->offset_bits == 32 ? 4 : 8;
-            auto const *offsets = static_cast<unsigned char const *>(tapes[k]->offsets);
-            ends[2 * k] = ends[2 * k + 1] = 0;
-            SZS_TRY_CUDA(cudaMemcpyAsync(&ends[2 * k], offsets, width, cudaMemcpyDefault, stream));
-            SZS_TRY_CUDA(cudaMemcpyAsync(&ends[2 * k + 1], offsets + tapes[k]->count * width, width, cudaMemcpyDefault,
-                                         stream));
-        }
+    // Cross products under unit costs: one thread per cell with the query's match masks shared by its CTA, without
+    // planning, when one side's strings are short enough. Device-resident results are written in place.
+    if (engine.unit_levenshtein && !wide && call.mode == mode_cross_k && schedule != szs_gb300_schedule_plain_k && !defer) {
+        std::uint64_t *seen = context->spare_host();
+        SZS_TRY_CUDA(cudaEventRecord(context->start, stream));
+        SZS_TRY_CUDA(launch_direct_extents(args.queries, args.candidates, seen, stream));
         SZS_TRY_CUDA(cudaStreamSynchronize(stream));
-        std::uint64_t const query_bytes = ends[1] - ends[0], candidate_bytes = ends[3] - ends[2];
-        if (query_bytes <= 64 * queries_count && candidate_bytes <= 64 * candidates_count) {
-            std::uint32_t *flag = context->spare_device();
-            SZS_TRY_CUDA(cudaEventRecord(context->start, stream));
-            SZS_TRY_CUDA(cudaMemsetAsync(flag, 0, sizeof(std::uint32_t), stream));
+        bool swapped = false;
+        if (myers_direct_takes(seen[0], seen[2], args.pairs, swapped)) {
+            bool const in_place = device_accessible(call.out);
+            std::int64_t *target = call.out;
+            if (!in_place) {
+                status = context->work.reserve(args.pairs * sizeof(std::int64_t), stream);
+                if (status.ok()) status = context->results_host.reserve(args.pairs * sizeof(std::int64_t));
+                if (!status.ok()) return status;
+                target = static_cast<std::int64_t *>(context->work.data);
+            }
             SZS_TRY_CUDA(cudaEventRecord(context->compute_start, stream));
-            SZS_TRY_CUDA(launch_myers_direct(args, call.out, call.stride, flag, context->sm_count, stream));
+            SZS_TRY_CUDA(launch_myers_direct(args.queries, args.candidates, swapped, swapped ? seen[2] : seen[0], target,
+                                             in_place ? call.stride : candidates_count, context->sm_count, stream));
             SZS_TRY_CUDA(cudaEventRecord(context->compute_stop, stream));
-            auto *flag_host = reinterpret_cast<std::uint32_t *>(ends + 4);
-            *flag_host = 0;
-            SZS_TRY_CUDA(cudaMemcpyAsync(flag_host, flag, sizeof(std::uint32_t), cudaMemcpyDeviceToHost, stream));
+            auto *dense = static_cast<std::int64_t *>(context->results_host.data);
+            if (!in_place)
+                SZS_TRY_CUDA(cudaMemcpyAsync(dense, target, args.pairs * sizeof(std::int64_t), cudaMemcpyDeviceToHost,
+                                             stream));
             SZS_TRY_CUDA(cudaEventRecord(context->stop, stream));
             SZS_TRY_CUDA(cudaStreamSynchronize(stream));
-            if (*flag_host == 0) {
-                float elapsed = 0, compute = 0;
-                cudaEventElapsedTime(&elapsed, context->start, context->stop);
-                cudaEventElapsedTime(&compute, context->compute_start, context->compute_stop);
-                stats.last_call_ms = elapsed, stats.last_compute_ms = compute;
-                stats.last_cells = query_bytes * candidate_bytes; // sum over cells of n x m
-                stats.last_launches = 1;
-                stats.kernel_launches += 1;
-                return {};
-            }
+            if (!in_place)
+                for (std::uint64_t q = 0; q < queries_count; ++q)
+                    std::memcpy(call.out + q * call.stride, dense + q * candidates_count,
+                                candidates_count * sizeof(std::int64_t));
+            float elapsed = 0, compute = 0;
+            cudaEventElapsedTime(&elapsed, context->start, context->stop);
+            cudaEventElapsedTime(&compute, context->compute_start, context->compute_stop);
+            stats.last_call_ms = elapsed, stats.last_compute_ms = compute;
+            stats.last_cells = seen[1] * seen[3]; // sum over cells of n x m
+            stats.last_launches = 2;
+            stats.kernel_launches += 2;
+            return {};
         }
     }
 

@@ -23,11 +23,22 @@ cudaError_t launch_plan(plan_args_t const &args, plan_bins_t *bins, pair_task_t 
 cudaError_t launch_alphabet(tape_t const &queries, tape_t const &candidates, bool has_candidates,
                             batch_alphabet_t *alphabet, int sm_count, cudaStream_t stream,
                             std::uint64_t sample_bytes = 0);
-/** Unit-cost Levenshtein over a cross product (`args.mode == mode_cross_k`) straight into `out` (row stride in
- *  elements), one thread per cell; sets `*flag` to 1 if a string has more than 64 bytes (its cells are then not
- *  written). */
-cudaError_t launch_myers_direct(plan_args_t const &args, std::int64_t *out, std::uint64_t stride,
-                                std::uint32_t *flag, int sm_count, cudaStream_t stream);
+constexpr std::uint64_t direct_max_rows_k = 1024; // longest pattern of the direct cross-product kernels
+/** Fewest cells of a cross product for the direct kernels with patterns of 513 to 1,024 rows: one thread per cell takes
+ *  about 0.33 ms for a pair of 1,000 bytes however few there are, where the warp-per-pair kernel spreads few pairs over
+ *  more SMs (256 pairs 0.28 ms, 2,560 0.45 ms, 3,600 0.54 ms). */
+constexpr std::uint64_t direct_min_pairs_k = 1536;
+/** The longest string of both tapes and the bytes of their data into `extents` (4 values in page-locked host memory:
+ *  longest query, query bytes, longest candidate, candidate bytes). */
+cudaError_t launch_direct_extents(tape_t const &queries, tape_t const &candidates, std::uint64_t *extents,
+                                  cudaStream_t stream);
+/** Whether the direct kernels take a unit-cost cross product with these longest strings; `swapped`: with the
+ *  candidates as patterns. */
+bool myers_direct_takes(std::uint64_t longest_query, std::uint64_t longest_candidate, std::uint64_t pairs, bool &swapped);
+/** Unit-cost Levenshtein over a cross product straight into `out` (row stride in elements), one thread per cell;
+ *  `longest_rows` is the longest pattern (at most `direct_max_rows_k`). */
+cudaError_t launch_myers_direct(tape_t const &queries, tape_t const &candidates, bool swapped, std::uint64_t longest_rows,
+                                std::int64_t *out, std::uint64_t stride, int sm_count, cudaStream_t stream);
 cudaError_t launch_scatter_output(plan_args_t const &args, std::int64_t const *results, std::int64_t *out,
                                   std::uint64_t stride, int sm_count, cudaStream_t stream);
 

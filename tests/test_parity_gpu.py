@@ -1103,3 +1103,34 @@ def test_largest_pairs_of_a_batch_take_groups(szs, port, family, costs, alphabet
     engine, oracle_costs = make_engine(szs, family, costs, b2c, table)
     got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
     np.testing.assert_array_equal(got, port.pairs(oracle_costs, tape(first), tape(second)))
+
+
+@pytest.mark.parametrize("longest", [4, 32, 33, 64, 96, 128, 129, 320, 512, 513, 1000, 1024, 1025])
+def test_direct_cross_product_edges(szs, port, longest):
+    """Unit-cost cross products around the direct kernels' word counts and classes: patterns of every edge up to
+    `longest` (beyond 1,024 the candidates become the patterns), empty strings, every byte value, texts at every
+    alignment, host and strided device results, 32- and 64-bit offsets, and few cells (the planned routes from 513
+    rows on)."""
+    import torch
+    rng = np.random.default_rng(longest)
+    letters = np.arange(256, dtype=np.uint8)
+    edges = [n for n in (0, 1, 3, 31, 32, 33, 63, 64, 65, 127, 128, 255, 256, 257, 511, 1023) if n < longest] + [longest]
+    lengths = edges + [int(n) for n in rng.integers(0, longest + 1, 66)]
+    queries = [bytes(rng.choice(letters if i % 2 else DNA, size=n)) for i, n in enumerate(lengths)]
+    candidates = [bytes(rng.choice(letters if i % 3 else DNA, size=int(n)))
+                  for i, n in enumerate(list(rng.integers(0, min(longest, 700) + 1, 60)) + [0, 1, 33])]
+    candidates += [q[:40] + q[41:][:600] for q in queries[:6]]
+    want = port.cross(oracle.levenshtein_costs(), tape(queries), tape(candidates))
+    engine = szs.LevenshteinDistances()
+    np.testing.assert_array_equal(engine(szs.Strs(queries), szs.Strs(candidates)).astype(np.int64), want)
+    np.testing.assert_array_equal(engine(szs.Strs(queries[:5]), szs.Strs(candidates[:7])).astype(np.int64), want[:5, :7])
+    for kind in (np.int32, np.int64):
+        def device(items):
+            data, offsets = tape(items)
+            return szs.Strs.from_buffers(torch.from_numpy(data.copy()).cuda(),
+                                         torch.from_numpy(offsets.astype(kind)).cuda())
+        out = torch.full((len(queries), len(candidates) + 3), -1, dtype=torch.int64, device="cuda")
+        engine(device(queries), device(candidates), out=out)
+        got = out.cpu().numpy()
+        np.testing.assert_array_equal(got[:, :len(candidates)], want)
+        assert (got[:, len(candidates):] == -1).all()
