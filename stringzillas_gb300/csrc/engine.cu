@@ -219,6 +219,8 @@ struct device_context_t {
     cudaStream_t lanes[lanes_k] = {nullptr};
     cudaEvent_t fork = nullptr;
     cudaEvent_t joins[lanes_k] = {nullptr};
+    static constexpr int near_jobs_k = 3; // near-diagonal jobs of one call at most
+    cudaEvent_t near_done[near_jobs_k] = {nullptr};
     cudaEvent_t trace_events[64] = {nullptr};
     graph_cache_t prologue_graphs; // alphabet + plan + plan readback
     graph_cache_t launch_graphs;   // the scoring kernels of a plan
@@ -256,6 +258,7 @@ struct device_context_t {
         SZS_TRY_CUDA(cudaEventCreate(&compute_stop));
         for (auto &event : trace_events) SZS_TRY_CUDA(cudaEventCreate(&event));
         SZS_TRY_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        for (auto &event : near_done) SZS_TRY_CUDA(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
         SZS_TRY_CUDA(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
         // Timed only under SZS_GB300_TRACE or SZS_GB300_TRACE_CHUNKS, which print each pipelined chunk's timeline.
         unsigned const copied_flags = std::getenv("SZS_GB300_TRACE") || std::getenv("SZS_GB300_TRACE_CHUNKS")
@@ -323,6 +326,8 @@ struct device_context_t {
             if (joins[i]) cudaEventDestroy(joins[i]);
         }
         if (fork) cudaEventDestroy(fork);
+        for (auto &event : near_done)
+            if (event) cudaEventDestroy(event);
         if (compute_start) cudaEventDestroy(compute_start);
         if (compute_stop) cudaEventDestroy(compute_stop);
         if (own_stream) cudaStreamDestroy(own_stream);
@@ -373,12 +378,14 @@ static engine_t *as_engine(void *handle, int kind) noexcept {
 static int cost_abs(int x) noexcept { return x < 0 ? -x : x; }
 
 // Per plane count, built from kernels_myers.cu once per count: (words, exact, tasks, bins, key_begin, key_end,
-// alphabet, results, ctas, stream), and the warp forms without `exact`.
+// alphabet, results, list, ctas, stream), and the warp forms without `exact`.
 #define SZS_DECLARE_MYERS_PLANES(planes)                                                                            \
     cudaError_t launch_myers_planes##planes(int, bool, pair_task_t const *, plan_bins_t const *, int, int,           \
-                                            batch_alphabet_t const *, std::int64_t *, int, cudaStream_t);           \
+                                            batch_alphabet_t const *, std::int64_t *, std::uint32_t const *, int,    \
+                                            cudaStream_t);                                                           \
     cudaError_t launch_myers_warp_planes##planes(int, pair_task_t const *, plan_bins_t *, int, int,                 \
-                                                 batch_alphabet_t const *, std::int64_t *, int, cudaStream_t);
+                                                 batch_alphabet_t const *, std::int64_t *, std::uint32_t const *,    \
+                                                 int, cudaStream_t);
 SZS_DECLARE_MYERS_PLANES(2)
 SZS_DECLARE_MYERS_PLANES(3)
 SZS_DECLARE_MYERS_PLANES(5)
@@ -397,24 +404,32 @@ int myers_threads_per_cta() { return 128; }
 /** Warp-per-pair bit-parallel kernel over bins [key_begin, key_end) with `words` words per lane. */
 static cudaError_t launch_myers_warp(int words, int planes, pair_task_t const *tasks, plan_bins_t *bins,
                                      int key_begin, int key_end, batch_alphabet_t const *alphabet,
-                                     std::int64_t *results, int ctas, cudaStream_t stream) {
+                                     std::int64_t *results, std::uint32_t const *list, int ctas, cudaStream_t stream) {
     switch (planes) {
-    case 2: return launch_myers_warp_planes2(words, tasks, bins, key_begin, key_end, alphabet, results, ctas, stream);
-    case 3: return launch_myers_warp_planes3(words, tasks, bins, key_begin, key_end, alphabet, results, ctas, stream);
-    case 5: return launch_myers_warp_planes5(words, tasks, bins, key_begin, key_end, alphabet, results, ctas, stream);
-    case 8: return launch_myers_warp_planes8(words, tasks, bins, key_begin, key_end, alphabet, results, ctas, stream);
+    case 2: return launch_myers_warp_planes2(words, tasks, bins, key_begin, key_end, alphabet, results, list, ctas,
+                                             stream);
+    case 3: return launch_myers_warp_planes3(words, tasks, bins, key_begin, key_end, alphabet, results, list, ctas,
+                                             stream);
+    case 5: return launch_myers_warp_planes5(words, tasks, bins, key_begin, key_end, alphabet, results, list, ctas,
+                                             stream);
+    case 8: return launch_myers_warp_planes8(words, tasks, bins, key_begin, key_end, alphabet, results, list, ctas,
+                                             stream);
     default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t launch_myers(int words, int planes, bool exact, pair_task_t const *tasks, plan_bins_t const *bins,
-                         int key_begin, int key_end, batch_alphabet_t const *alphabet, std::int64_t *results, int ctas,
-                         cudaStream_t stream) {
+                         int key_begin, int key_end, batch_alphabet_t const *alphabet, std::int64_t *results,
+                         std::uint32_t const *list, int ctas, cudaStream_t stream) {
     switch (planes) {
-    case 2: return launch_myers_planes2(words, exact, tasks, bins, key_begin, key_end, alphabet, results, ctas, stream);
-    case 3: return launch_myers_planes3(words, exact, tasks, bins, key_begin, key_end, alphabet, results, ctas, stream);
-    case 5: return launch_myers_planes5(words, exact, tasks, bins, key_begin, key_end, alphabet, results, ctas, stream);
-    case 8: return launch_myers_planes8(words, exact, tasks, bins, key_begin, key_end, alphabet, results, ctas, stream);
+    case 2: return launch_myers_planes2(words, exact, tasks, bins, key_begin, key_end, alphabet, results, list, ctas,
+                                        stream);
+    case 3: return launch_myers_planes3(words, exact, tasks, bins, key_begin, key_end, alphabet, results, list, ctas,
+                                        stream);
+    case 5: return launch_myers_planes5(words, exact, tasks, bins, key_begin, key_end, alphabet, results, list, ctas,
+                                        stream);
+    case 8: return launch_myers_planes8(words, exact, tasks, bins, key_begin, key_end, alphabet, results, list, ctas,
+                                        stream);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -845,6 +860,13 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         args.packed_step_cost[choice] = engine.tuning.packed_step_cost[choice]
                                             ? engine.tuning.packed_step_cost[choice]
                                             : (std::uint16_t)packed_step_cost_k[choice];
+    // Unit costs: whether most pairs look alike decides if they are tried near their diagonal first. Plans made before
+    // the strings have landed (pipelined chunks) cannot look at them and try.
+    bool const planned_ahead = call.scoring_after && call.plan_after != call.scoring_after;
+    args.near_sample_stride =
+        engine.unit_levenshtein && schedule != szs_gb300_schedule_plain_k && !planned_ahead
+            ? (std::uint32_t)std::max<std::uint64_t>(args.pairs / near_samples_k, 1)
+            : 0;
     bool const levenshtein = engine.kind == kind_levenshtein_k;
     bool const dense = !engine.dense.empty();
     // Both score over the batch's own byte codes; 16-bit codes are already dense.
@@ -1020,7 +1042,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
     // The launch list, longest pairs first (64- and 32-bit wavefront, packed with the most rows per lane, then the
     // bit-parallel kernels by word count), so the routes' tails overlap each other instead of adding up.
     enum job_kind_t { job_dp_k, job_dp16_k, job_myers_k, job_band_k, job_band16_k, job_myers_warp_k, job_short_k,
-                      job_myers_chain_k };
+                      job_myers_chain_k, job_near_k };
     struct job_t {
         job_kind_t kind;
         int variant; // cell bits, rows per lane, or words
@@ -1035,6 +1057,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         std::size_t state_bytes = 0;
         bool fills = true;             // the grid takes every resident CTA slot of its kernel on the device
         bool first = false;            // a batch's largest pairs: launched before everything else
+        bool listed = false;           // scores what the near-diagonal jobs listed, after them
     };
     job_t jobs[64];
     int job_count = 0;
@@ -1218,6 +1241,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         jobs[job_count - 1].fills = needed >= (std::uint64_t)context->sm_count * shape.ctas_per_sm;
     }
     int myers_planes = 0;
+    std::size_t near_list_at = 0; // the near-diagonal kernels' list of task indices in the scratch buffer
     std::uint32_t chain_strips = 0, chain_wave = 0; // warps per chained pair, pairs per cooperative launch
     std::uint64_t chain_link_stride = 0;
     if (engine.unit_levenshtein) {
@@ -1248,6 +1272,33 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         // The plain form keeps each bit-parallel route in one bin and launches the word count of the batch's longest
         // pattern on it (the binned form launches each bin with its own word count).
         bool const plain = schedule == szs_gb300_schedule_plain_k;
+        // Pairs that are alike are scored near their diagonal first (myers_near.cuh); the jobs of their bins then score
+        // what those kernels list. A window of three words pays from five words of pattern on, and for 16-bit codes also
+        // against the warp route's one word per lane; the nine-word window of long DNA-like reads keeps a thread per
+        // pair busy for long, so it takes batches of more pairs than the warp route scores at once (two CTAs of eight
+        // warps per SM).
+        int near_words = myers_max_words_k + 1, near_per_lane = 0; // first words, most words per lane it takes
+        // A pair given up early costs about an eighth of its full score, one found saves a third or more.
+        if (!plain && (!args.near_sample_stride || plan.near_alike * 3 > plan.near_sampled)) {
+            auto near_job = [&](int half, int key_begin, int key_end) {
+                std::uint64_t const pairs_here = pairs_in(key_begin, key_end);
+                if (!pairs_here) return;
+                std::uint64_t const needed = (pairs_here + myers_near_threads() - 1) / myers_near_threads();
+                int const ctas = (int)std::min<std::uint64_t>(needed, (std::uint64_t)context->sm_count * 16);
+                if (!near_list_at) {
+                    near_list_at = scratch_total + 256;
+                    scratch_total = near_list_at + align_up(args.pairs * sizeof(std::uint32_t), 256);
+                }
+                jobs[job_count++] = {job_near_k, half, 0, key_begin, key_end, pairs_here, ctas, 0, 0};
+            };
+            int const warp_end = bin_myers_warp_begin_k + myers_warp_max_words_k * myers_warp_classes_k;
+            near_words = near_min_words_k;
+            near_job(1, bin_myers_begin_k + near_words * 16, bin_myers_begin_k + (myers_max_words_k + 1) * 16);
+            int const one_per_lane = warp_end - myers_warp_classes_k;
+            if (wide && pairs_in(one_per_lane, warp_end)) near_per_lane = 1, near_job(1, one_per_lane, warp_end);
+            if (myers_planes == 2 && pairs_in(bin_myers_warp_begin_k, warp_end) >= (std::uint64_t)context->sm_count * 16)
+                near_per_lane = myers_warp_max_words_k, near_job(4, bin_myers_warp_begin_k, warp_end);
+        }
         // Longer patterns first: one warp per pair, most words per lane first.
         for (int words = myers_warp_max_words_k; words >= 1; --words) {
             int const key_begin = bin_myers_warp_begin_k + (myers_warp_max_words_k - words) * myers_warp_classes_k;
@@ -1260,6 +1311,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             jobs[job_count++] = {job_myers_warp_k, launch_words, 0, key_begin, key_begin + myers_warp_classes_k,
                                  pairs_here, ctas, 0, 0};
             jobs[job_count - 1].fills = needed >= (std::uint64_t)context->sm_count * 2;
+            jobs[job_count - 1].listed = words <= near_per_lane;
         }
         for (int words = myers_max_words_k; words >= 1; --words) {
             int const key_begin = bin_myers_begin_k + words * 16;
@@ -1271,14 +1323,20 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             int const ctas = (int)std::min<std::uint64_t>(needed, (std::uint64_t)context->sm_count * 16);
             jobs[job_count++] = {job_myers_k, launch_words, 0, key_begin, key_begin + 16, pairs_here, ctas, 0, 0};
             jobs[job_count - 1].fills = needed >= (std::uint64_t)context->sm_count * 16;
+            jobs[job_count - 1].listed = words >= near_words;
         }
     }
     // Jobs whose grids leave slots free go first: a persistent grid that fills the device holds its slots until its
     // last pair, so a small job launched after it would only start at the end and add its whole time to the call.
     // Launched first, it takes its few slots and runs beside the large grids, which balance over their cursor.
+    // The largest pairs' groups go before everything else, and the near-diagonal jobs before those that wait for them.
     if (schedule != szs_gb300_schedule_plain_k)
-        std::stable_partition(jobs, jobs + job_count, [](job_t const &job) { return job.first || !job.fills; }),
-            std::stable_partition(jobs, jobs + job_count, [](job_t const &job) { return job.first; });
+        std::stable_sort(jobs, jobs + job_count, [](job_t const &a, job_t const &b) {
+            auto rank = [](job_t const &job) {
+                return job.first ? 0 : job.kind == job_near_k ? 1 : job.listed ? 4 : job.fills ? 3 : 2;
+            };
+            return rank(a) < rank(b);
+        });
     if (scratch_total) {
         status = context->scratch.reserve(scratch_total, stream);
         if (!status.ok()) return status;
@@ -1303,21 +1361,30 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             key_append(launch_key, jobs[i].key_begin), key_append(launch_key, jobs[i].key_end);
             key_append(launch_key, jobs[i].ctas), key_append(launch_key, jobs[i].scratch_offset);
             key_append(launch_key, jobs[i].group_ctas), key_append(launch_key, jobs[i].state_offset);
-            key_append(launch_key, jobs[i].rows);
+            key_append(launch_key, jobs[i].rows), key_append(launch_key, jobs[i].listed);
         }
         key_append(launch_key, packed_costs), key_append(launch_key, call_costs);
         key_append(launch_key, tasks), key_append(launch_key, bins), key_append(launch_key, results);
         key_append(launch_key, context->scratch.data), key_append(launch_key, alphabet);
         key_append(launch_key, cells_per_warp), key_append(launch_key, myers_planes), key_append(launch_key, wide);
+        key_append(launch_key, near_list_at);
         key_append(launch_key, schedule), key_append(launch_key, lanes_used);
         key_append(launch_key, engine.kind), key_append(launch_key, compare_mode);
     }
     auto issue_jobs = [&](cudaStream_t s) -> status_t {
         SZS_TRY_CUDA(cudaEventRecord(context->fork, s));
         for (int lane = 0; lane < lanes_used; ++lane) SZS_TRY_CUDA(cudaStreamWaitEvent(context->lanes[lane], context->fork, 0));
+        auto *near_list = near_list_at ? reinterpret_cast<std::uint32_t *>(
+                                             static_cast<unsigned char *>(context->scratch.data) + near_list_at)
+                                       : nullptr;
+        int near_jobs = 0;
         for (int i = 0; i < job_count; ++i) {
             job_t const &job = jobs[i];
             cudaStream_t const lane_stream = context->lanes[i % lanes_used];
+            if (job.listed)
+                for (int k = 0; k < near_jobs; ++k)
+                    SZS_TRY_CUDA(cudaStreamWaitEvent(lane_stream, context->near_done[k], 0));
+            std::uint32_t const *list = job.listed ? near_list : nullptr;
             bool const traced = tracing && 2 * i + 1 < 64;
             if (traced) cudaEventRecord(context->trace_events[2 * i], lane_stream);
             void *scratch = static_cast<unsigned char *>(context->scratch.data) + job.scratch_offset;
@@ -1355,21 +1422,26 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
                 SZS_TRY_CUDA(launch_short(engine.kind, costs.affine != 0, job.variant, job.key_begin, job.key_end,
                                           tasks, bins, packed_costs, results, job.ctas, job.warps, lane_stream,
                                           compare_mode));
+            else if (job.kind == job_near_k) {
+                SZS_TRY_CUDA(launch_myers_near(job.variant, myers_planes, tasks, bins, job.key_begin, job.key_end, alphabet,
+                                               results, near_list, job.ctas, lane_stream));
+                SZS_TRY_CUDA(cudaEventRecord(context->near_done[near_jobs++], lane_stream));
+            }
             else if (job.kind == job_myers_warp_k && wide)
                 SZS_TRY_CUDA(launch_myers_warp_wide(job.variant, tasks, bins, job.key_begin, job.key_end, results,
-                                                    job.ctas, lane_stream));
+                                                    list, job.ctas, lane_stream));
             else if (job.kind == job_myers_warp_k)
                 SZS_TRY_CUDA(launch_myers_warp(job.variant, myers_planes, tasks, bins, job.key_begin, job.key_end,
-                                               alphabet, results, job.ctas, lane_stream));
+                                               alphabet, results, list, job.ctas, lane_stream));
             else if (wide)
                 SZS_TRY_CUDA(launch_myers_wide(job.variant, schedule != szs_gb300_schedule_plain_k, tasks, bins,
-                                               job.key_begin, job.key_end, results, job.ctas, lane_stream));
+                                               job.key_begin, job.key_end, results, list, job.ctas, lane_stream));
             else if (myers_planes == 2)
                 SZS_TRY_CUDA(launch_myers_table(job.variant, job.key_begin, job.key_end, tasks, bins, alphabet,
-                                                results, job.ctas, lane_stream));
+                                                results, list, job.ctas, lane_stream));
             else
                 SZS_TRY_CUDA(launch_myers(job.variant, myers_planes, schedule != szs_gb300_schedule_plain_k, tasks,
-                                          bins, job.key_begin, job.key_end, alphabet, results, job.ctas,
+                                          bins, job.key_begin, job.key_end, alphabet, results, list, job.ctas,
                                           lane_stream));
             if (traced) cudaEventRecord(context->trace_events[2 * i + 1], lane_stream);
         }
@@ -1453,8 +1525,9 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
     stats.last_compute_ms = compute;
     if (tracing) {
         static char const *const names[] = {"wavefront bits", "packed16 rows", "bit-parallel words", "band bits",
-                                            "band16 bits", "warp bit-parallel", "short shape", "chained words"};
-        static_assert(sizeof(names) / sizeof(names[0]) == job_myers_chain_k + 1, "a name per job kind");
+                                            "band16 bits", "warp bit-parallel", "short shape", "chained words",
+                                            "near diagonal"};
+        static_assert(sizeof(names) / sizeof(names[0]) == job_near_k + 1, "a name per job kind");
         for (int i = 0; i < job_count && 2 * i + 1 < 64; ++i) {
             float ms = 0, offset = 0;
             cudaEventElapsedTime(&ms, context->trace_events[2 * i], context->trace_events[2 * i + 1]);

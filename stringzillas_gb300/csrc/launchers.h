@@ -204,27 +204,37 @@ cudaError_t launch_myers_chain(int words, int planes, pair_task_t const *tasks, 
                                batch_alphabet_t const *alphabet, std::int64_t *results, void *scratch,
                                std::uint64_t link_stride, std::uint32_t wait_polls, cudaStream_t stream);
 
+/** The near-diagonal bit-parallel kernel (`half` blocks of 32 rows either side of the diagonal: 1, or 4 for at most four
+ *  symbol codes) over bins [key_begin, key_end) of the thread and warp routes: scores similar pairs, and lists the others'
+ *  task indices in `list` (one entry per task, from the first task of each class on; `bins->listed` counts them). */
+cudaError_t launch_myers_near(int half, int planes, pair_task_t const *tasks, plan_bins_t *bins, int key_begin,
+                              int key_end, batch_alphabet_t const *alphabet, std::int64_t *results,
+                              std::uint32_t *list, int ctas, cudaStream_t stream);
+int myers_near_threads();
+
+/** The bit-parallel kernels below score all pairs of their bins, or with `list` only those the near-diagonal kernel
+ *  listed. */
 /** Bit-parallel kernels over strings of 16-bit codes (UTF-8 calls over more than 256 code points, 16 code planes):
  *  thread per pair over the bins of `words` words (1..8), and warp per pair over the warp bins (1..8 words per
  *  lane). */
 cudaError_t launch_myers_wide(int words, bool exact, pair_task_t const *tasks, plan_bins_t const *bins, int key_begin,
-                              int key_end, std::int64_t *results, int ctas, cudaStream_t stream);
+                              int key_end, std::int64_t *results, std::uint32_t const *list, int ctas, cudaStream_t stream);
 cudaError_t launch_myers_warp_wide(int words, pair_task_t const *tasks, plan_bins_t *bins, int key_begin, int key_end,
-                                   std::int64_t *results, int ctas, cudaStream_t stream);
+                                   std::int64_t *results, std::uint32_t const *list, int ctas, cudaStream_t stream);
 
 /** Runs the bit-parallel kernel over bins [key_begin, key_end) with `words` words (1..16) and `planes` code planes
  *  (2, 3, 5 or 8). `exact` = every pair in the bins needs exactly `words` words (the binned schedule); otherwise
  *  pairs may be shorter (the plain schedule puts every bit-parallel pair in one bin and launches the word count of
  *  the batch's longest pattern). */
 cudaError_t launch_myers(int words, int planes, bool exact, pair_task_t const *tasks, plan_bins_t const *bins,
-                         int key_begin, int key_end, batch_alphabet_t const *alphabet, std::int64_t *results, int ctas,
+                         int key_begin, int key_end, batch_alphabet_t const *alphabet, std::int64_t *results, std::uint32_t const *list, int ctas,
                          cudaStream_t stream);
 int myers_threads_per_cta();
 /** The shared-table bit-parallel kernel for batches over at most four symbol codes: bins [key_begin, key_end),
  *  patterns of at most 32 x `words` rows (1..16). A pair holding a byte outside `alphabet->present` sets bit 1 of
  *  `bins->error_flags` (its score is then not valid). */
 cudaError_t launch_myers_table(int words, int key_begin, int key_end, pair_task_t const *tasks,
-                               plan_bins_t *bins, batch_alphabet_t const *alphabet, std::int64_t *results,
+                               plan_bins_t *bins, batch_alphabet_t const *alphabet, std::int64_t *results, std::uint32_t const *list,
                                int ctas, cudaStream_t stream);
 /** Planes actually instantiated for a requested minimum. */
 int myers_planes_for(int bits_needed);

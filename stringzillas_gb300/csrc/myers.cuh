@@ -134,12 +134,17 @@ __device__ __forceinline__ std::uint32_t myers_distance(std::uint8_t const *patt
 }
 
 /** Thread-per-pair kernel over bins [key_begin, key_end), patterns of at most 32 x `words_` rows (exactly that many
- *  words when `exact_`). */
+ *  words when `exact_`); with `list` (pairs the near-diagonal kernel left), over the listed tasks of its words. */
 template <int words_, int bits_, bool exact_>
 __global__ void __launch_bounds__(128) myers_kernel(pair_task_t const *__restrict__ tasks,
                                                     plan_bins_t const *__restrict__ bins, int key_begin, int key_end,
                                                     batch_alphabet_t const *__restrict__ alphabet,
-                                                    std::int64_t *__restrict__ results) {
+                                                    std::int64_t *__restrict__ results,
+                                                    std::uint32_t const *__restrict__ list) {
+    std::uint32_t const begin = bins->begin[key_begin];
+    std::uint32_t const count =
+        list ? bins->listed[words_] : bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
+    if (blockIdx.x * blockDim.x >= count) return;
     __shared__ std::uint8_t code_s[256];
     __shared__ plane_selectors_t<bits_> selectors_s;
     for (int i = threadIdx.x; i < 256; i += blockDim.x) {
@@ -149,11 +154,9 @@ __global__ void __launch_bounds__(128) myers_kernel(pair_task_t const *__restric
         for (int b = 0; b < bits_; ++b) selectors_s.select[i][b] = ((c >> b) & 1u) ? 0u : 0xFFFFFFFFu;
     }
     __syncthreads();
-    std::uint32_t const begin = bins->begin[key_begin];
-    std::uint32_t const count = bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
     for (std::uint32_t index = blockIdx.x * blockDim.x + threadIdx.x; index < count;
          index += gridDim.x * blockDim.x) {
-        pair_task_t const task = tasks[begin + index];
+        pair_task_t const task = tasks[list ? list[begin + index] : begin + index];
         results[task.slot] =
             myers_distance<words_, bits_, exact_>(task.rows, task.rows_length, task.cols, task.cols_length, code_s,
                                                   selectors_s);
@@ -175,13 +178,15 @@ __device__ __forceinline__ void code_selectors(std::uint32_t code, std::uint32_t
 template <int words_, bool exact_>
 __global__ void __launch_bounds__(128) myers_wide_kernel(pair_task_t const *__restrict__ tasks,
                                                          plan_bins_t const *__restrict__ bins, int key_begin,
-                                                         int key_end, std::int64_t *__restrict__ results) {
+                                                         int key_end, std::int64_t *__restrict__ results,
+                                                         std::uint32_t const *__restrict__ list) {
     constexpr int W = words_, B = myers_wide_planes_k;
     std::uint32_t const begin = bins->begin[key_begin];
-    std::uint32_t const count = bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
+    std::uint32_t const count =
+        list ? bins->listed[words_] : bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
     for (std::uint32_t index = blockIdx.x * blockDim.x + threadIdx.x; index < count;
          index += gridDim.x * blockDim.x) {
-        pair_task_t const task = tasks[begin + index];
+        pair_task_t const task = tasks[list ? list[begin + index] : begin + index];
         auto const *pattern = reinterpret_cast<std::uint16_t const *>(task.rows);
         std::uint32_t const n = task.rows_length, m = task.cols_length;
         myers_state_t<W, B, exact_> state;

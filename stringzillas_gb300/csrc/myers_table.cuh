@@ -23,6 +23,8 @@
  *  that met a marker sets bit 1 of the plan's error word, on which the host scores the call again with the exact
  *  alphabet. Known codes (0..3) and offsets (multiples of 2,048) never carry the marker bit.
  *
+ *  With `list` (pairs the near-diagonal kernel left) the kernel scores the listed tasks of its words instead of all.
+ *
  *  Per text character and pattern word the step is ten ALU operations (Xv, Eq & Pv, the carried add, Xh, Ph, Mh,
  *  two funnel shifts, Pv, Mv). The kernel takes its bins as a key range, so the plain form can run every pair with
  *  the word count of the batch's longest pattern (rows past a pattern's end are masked out of the final count).
@@ -98,13 +100,17 @@ template <int words_>
 __global__ void __launch_bounds__(myers_table_threads_k, myers_table_min_ctas(words_))
     myers_table_kernel(pair_task_t const *__restrict__ tasks, plan_bins_t *__restrict__ bins, int key_begin,
                        int key_end, batch_alphabet_t const *__restrict__ alphabet,
-                       std::int64_t *__restrict__ results) {
+                       std::int64_t *__restrict__ results, std::uint32_t const *__restrict__ list) {
     constexpr int W = words_, Q = (words_ + 3) / 4;
     constexpr unsigned code_stride = myers_table_threads_k * 16;                         // bytes between codes
     constexpr unsigned group_stride = myers_table_symbols_k * myers_table_threads_k * 16; // between word groups
     extern __shared__ __align__(16) unsigned char table_s[];
     __shared__ std::uint32_t offset_s[256]; // byte -> code * code_stride
     __shared__ std::uint8_t code_s[256];
+    std::uint32_t const begin = bins->begin[key_begin];
+    std::uint32_t const count =
+        list ? bins->listed[words_] : bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
+    if (blockIdx.x * blockDim.x >= count) return;
     for (int i = threadIdx.x; i < 256; i += blockDim.x) {
         std::uint32_t const c = alphabet->code[i] & (myers_table_symbols_k - 1);
         bool const known = (alphabet->present[i >> 5] >> (i & 31)) & 1u;
@@ -113,11 +119,9 @@ __global__ void __launch_bounds__(myers_table_threads_k, myers_table_min_ctas(wo
     }
     __syncthreads();
     unsigned char *const mine = table_s + threadIdx.x * 16u;
-    std::uint32_t const begin = bins->begin[key_begin];
-    std::uint32_t const count = bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
     for (std::uint32_t index = blockIdx.x * blockDim.x + threadIdx.x; index < count;
          index += gridDim.x * blockDim.x) {
-        pair_task_t const task = tasks[begin + index];
+        pair_task_t const task = tasks[list ? list[begin + index] : begin + index];
         std::uint8_t const *pattern = task.rows;
         std::uint32_t const n = task.rows_length, m = task.cols_length;
 

@@ -113,12 +113,13 @@ __device__ __forceinline__ std::uint32_t myers_warp_distance(pair_task_t const &
 }
 
 /** Warp-per-pair kernel over bins [key_begin, key_end) with at most `words_` words per lane; warps pull pairs from
- *  the first bin's cursor. */
+ *  the first bin's cursor. With `list` (pairs the near-diagonal kernel left), over the listed tasks of its words. */
 template <int words_, int bits_>
 __global__ void __launch_bounds__(256) myers_warp_kernel(pair_task_t const *__restrict__ tasks,
                                                          plan_bins_t *__restrict__ bins, int key_begin, int key_end,
                                                          batch_alphabet_t const *__restrict__ alphabet,
-                                                         std::int64_t *__restrict__ results) {
+                                                         std::int64_t *__restrict__ results,
+                                                         std::uint32_t const *__restrict__ list) {
     __shared__ std::uint8_t code_s[256];
     __shared__ plane_selectors_t<bits_> selectors_s;
     for (int i = threadIdx.x; i < 256; i += blockDim.x) {
@@ -130,13 +131,14 @@ __global__ void __launch_bounds__(256) myers_warp_kernel(pair_task_t const *__re
     __syncthreads();
     int const lane = threadIdx.x & 31;
     std::uint32_t const begin = bins->begin[key_begin];
-    std::uint32_t const count = bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
+    std::uint32_t const count = list ? bins->listed[myers_max_words_k + words_]
+                                     : bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
     while (true) {
         std::uint32_t index = 0;
         if (lane == 0) index = atomicAdd(&bins->cursor[key_begin], 1u);
         index = __shfl_sync(0xFFFFFFFFu, index, 0);
         if (index >= count) break;
-        pair_task_t const task = tasks[begin + index];
+        pair_task_t const task = tasks[list ? list[begin + index] : begin + index];
         std::uint32_t const distance = myers_warp_distance<words_, bits_>(task, code_s, &selectors_s);
         if (lane == 0) results[task.slot] = distance;
     }
@@ -146,16 +148,18 @@ __global__ void __launch_bounds__(256) myers_warp_kernel(pair_task_t const *__re
 template <int words_>
 __global__ void __launch_bounds__(256) myers_warp_wide_kernel(pair_task_t const *__restrict__ tasks,
                                                               plan_bins_t *__restrict__ bins, int key_begin,
-                                                              int key_end, std::int64_t *__restrict__ results) {
+                                                              int key_end, std::int64_t *__restrict__ results,
+                                                              std::uint32_t const *__restrict__ list) {
     int const lane = threadIdx.x & 31;
     std::uint32_t const begin = bins->begin[key_begin];
-    std::uint32_t const count = bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
+    std::uint32_t const count = list ? bins->listed[myers_max_words_k + words_]
+                                     : bins->begin[key_end - 1] + bins->count[key_end - 1] - begin;
     while (true) {
         std::uint32_t index = 0;
         if (lane == 0) index = atomicAdd(&bins->cursor[key_begin], 1u);
         index = __shfl_sync(0xFFFFFFFFu, index, 0);
         if (index >= count) break;
-        pair_task_t const task = tasks[begin + index];
+        pair_task_t const task = tasks[list ? list[begin + index] : begin + index];
         std::uint32_t const distance = myers_warp_distance<words_, myers_wide_planes_k, true>(
             task, nullptr, static_cast<plane_selectors_t<myers_wide_planes_k> const *>(nullptr));
         if (lane == 0) results[task.slot] = distance;

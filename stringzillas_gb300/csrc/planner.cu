@@ -212,6 +212,22 @@ __device__ __forceinline__ pair_route_info_t route_of_pair(plan_args_t const &ar
     return route_pair(args, first, first_length, second, second_length);
 }
 
+/** Whether two strings of `n` <= `m` symbols look so alike that their distance should be at most `distance`: by the
+ *  share of their first 16 symbols, or of their last 16, that are the same in place (one insertion hides the rest of one
+ *  end, seldom both), at least 9 (unrelated DNA agrees in 4). Decides only which kernel tries first, never a score. */
+template <typename symbol_>
+__device__ __forceinline__ bool looks_alike(symbol_ const *rows, std::uint32_t n, symbol_ const *cols, std::uint32_t m,
+                                            std::uint32_t distance) {
+    std::uint32_t head = 0, tail = 0;
+#pragma unroll
+    for (std::uint32_t k = 0; k < 16; ++k) {
+        head += rows[k] == cols[k];
+        tail += rows[n - 1 - k] == cols[m - 1 - k];
+    }
+    std::uint32_t const same = max(head, tail);
+    return same >= 9 && (std::uint64_t)(16 - same) * m <= 16ull * distance;
+}
+
 /** Pass 1: answer trivial pairs, count pairs per bin, track the longest column string and total cells. */
 __global__ void plan_count_kernel(plan_args_t const args, plan_bins_t *__restrict__ bins,
                                   std::int64_t *__restrict__ results) {
@@ -277,27 +293,66 @@ __global__ void plan_count_kernel(plan_args_t const args, plan_bins_t *__restric
     }
 }
 
-/** Pass 2: exclusive scan of bin counts (one CTA of `bin_keys_k / 2` threads, two adjacent keys each). */
-__global__ void plan_scan_kernel(plan_bins_t *__restrict__ bins) {
-    constexpr int threads = bin_keys_k / 2;
-    __shared__ std::uint32_t scan[threads];
-    int const i = threadIdx.x;
+/** Whether pair @p p is one that the near-diagonal kernels would try (patterns of at least five words, up to 32 or 128
+ *  symbols of difference in length), and if it is, whether it looks like a distance well inside their limits of 64 and
+ *  256. */
+__device__ __forceinline__ bool near_candidate(plan_args_t const &args, std::uint64_t p, bool &alike) {
+    std::uint64_t q, c;
+    pair_indices(args, p, q, c);
+    std::uint8_t const *first, *second;
+    std::uint64_t first_length, second_length;
+    tape_string(args.queries, q, first, first_length, args.wide);
+    tape_string(args.mode == mode_symmetric_k ? args.queries : args.candidates, c, second, second_length, args.wide);
+    bool const swap = second_length < first_length;
+    std::uint8_t const *rows = swap ? second : first, *cols = swap ? first : second;
+    std::uint64_t const n = swap ? second_length : first_length, m = swap ? first_length : second_length;
+    std::uint32_t const blocks = n <= 32u * myers_max_words_k ? 1u : 4u;
+    if (n <= 32u * (near_min_words_k - 1) || n > 32u * 32u * myers_warp_max_words_k || m - n > 32u * blocks) return false;
+    alike = args.wide ? looks_alike(reinterpret_cast<std::uint16_t const *>(rows), (std::uint32_t)n,
+                                    reinterpret_cast<std::uint16_t const *>(cols), (std::uint32_t)m, 40u * blocks)
+                      : looks_alike(rows, (std::uint32_t)n, cols, (std::uint32_t)m, 40u * blocks);
+    return true;
+}
+
+/** Pass 2: exclusive scan of bin counts (one CTA of `bin_keys_k / 2` threads, two adjacent keys each). A second CTA
+ *  samples the pairs' likeness meanwhile, one pair per thread. */
+__global__ void __launch_bounds__(bin_keys_k / 2) plan_scan_kernel(plan_args_t const args, plan_bins_t *__restrict__ bins) {
+    if (blockIdx.x == 1) {
+        std::uint64_t const p = (std::uint64_t)threadIdx.x * args.near_sample_stride;
+        bool alike = false;
+        bool const sampled = threadIdx.x < near_samples_k && p < args.pairs && near_candidate(args, p, alike);
+        int const samples = __syncthreads_count(sampled), similar = __syncthreads_count(sampled && alike);
+        if (threadIdx.x == 0) bins->near_sampled = (std::uint32_t)samples, bins->near_alike = (std::uint32_t)similar;
+        return;
+    }
+    constexpr int warps = bin_keys_k / 2 / 32;
+    static_assert(warps <= 32, "one warp scans the warps' totals");
+    __shared__ std::uint32_t totals[warps];
+    int const i = threadIdx.x, lane = i & 31, warp = i >> 5;
     std::uint32_t const first = bins->count[2 * i], second = bins->count[2 * i + 1];
     std::uint32_t const own = first + second;
-    scan[i] = own;
+    auto inclusive = [&](std::uint32_t value) {
+#pragma unroll
+        for (int offset = 1; offset < 32; offset <<= 1) {
+            std::uint32_t const below = __shfl_up_sync(0xFFFFFFFFu, value, offset);
+            if (lane >= offset) value += below;
+        }
+        return value;
+    };
+    std::uint32_t const scan = inclusive(own);
+    if (lane == 31) totals[warp] = scan;
     __syncthreads();
-    for (int offset = 1; offset < threads; offset <<= 1) {
-        std::uint32_t const add = i >= offset ? scan[i - offset] : 0u;
-        __syncthreads();
-        scan[i] += add;
-        __syncthreads();
+    if (warp == 0) {
+        std::uint32_t const total = inclusive(lane < warps ? totals[lane] : 0u);
+        if (lane < warps) totals[lane] = total;
     }
-    std::uint32_t const before = scan[i] - own;
+    __syncthreads();
+    std::uint32_t const before = scan - own + (warp ? totals[warp - 1] : 0u);
     bins->begin[2 * i] = before;
     bins->begin[2 * i + 1] = before + first;
     bins->fill[2 * i] = bins->fill[2 * i + 1] = 0;
     bins->cursor[2 * i] = bins->cursor[2 * i + 1] = 0;
-    if (i == threads - 1) bins->scheduled = scan[i];
+    if (i == bin_keys_k / 2 - 1) bins->scheduled = before + own;
 }
 
 /**
@@ -421,22 +476,30 @@ __global__ void alphabet_mark_kernel(tape_t const first_tape, tape_t const secon
     }
 }
 
-/** Dense codes for the marked bytes; `bits` = planes the Myers kernel needs (1..8). Clears the mask afterwards so
- *  the next call starts from zero. */
-__global__ void alphabet_codes_kernel(std::uint32_t *__restrict__ symbol_mask,
-                                      batch_alphabet_t *__restrict__ alphabet) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    std::uint32_t next = 0;
-    for (int b = 0; b < 256; ++b) {
-        bool const present = (symbol_mask[b >> 5] >> (b & 31)) & 1u;
-        alphabet->code[b] = present ? (std::uint8_t)next : 0;
-        next += present;
+/** Dense codes for the marked bytes, one byte per thread; `bits` = planes the Myers kernel needs (1..8). Clears the mask
+ *  afterwards so the next call starts from zero. */
+__global__ void __launch_bounds__(256) alphabet_codes_kernel(std::uint32_t *__restrict__ symbol_mask,
+                                                             batch_alphabet_t *__restrict__ alphabet) {
+    int const b = threadIdx.x, word = b >> 5, bit = b & 31;
+    std::uint32_t mask[8], below = 0, symbols = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        mask[k] = symbol_mask[k];
+        symbols += __popc(mask[k]);
+        if (k < word) below += __popc(mask[k]);
     }
-    std::uint32_t bits = 1;
-    while ((1u << bits) < next) ++bits;
-    alphabet->symbols = next;
-    alphabet->bits = bits;
-    for (int k = 0; k < 8; ++k) alphabet->present[k] = symbol_mask[k], symbol_mask[k] = 0;
+    std::uint32_t own = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (k == word) own = mask[k];
+    bool const present = (own >> bit) & 1u;
+    alphabet->code[b] = present ? (std::uint8_t)(below + __popc(own & ((1u << bit) - 1u))) : (std::uint8_t)0;
+    __syncthreads();
+    if (bit == 0) alphabet->present[word] = own, symbol_mask[word] = 0;
+    if (b == 0) {
+        alphabet->symbols = symbols;
+        alphabet->bits = symbols <= 2 ? 1u : 32u - (std::uint32_t)__clz((int)(symbols - 1));
+    }
 }
 
 /** Dense per-pair results into the caller's matrix (device-resident output). */
@@ -490,7 +553,7 @@ cudaError_t launch_plan(plan_args_t const &args, plan_bins_t *bins, pair_task_t 
     if (args.pairs == 0) return cudaSuccess;
     status = launch_prioritised(plan_count_kernel, grid_for(args.pairs, 256, sm_count), 256, stream, args, bins, results);
     if (status != cudaSuccess) return status;
-    status = launch_prioritised(plan_scan_kernel, 1, bin_keys_k / 2, stream, bins);
+    status = launch_prioritised(plan_scan_kernel, args.near_sample_stride ? 2 : 1, bin_keys_k / 2, stream, args, bins);
     if (status != cudaSuccess) return status;
     return launch_prioritised(plan_scatter_kernel, grid_for(args.pairs, 256, sm_count), 256, stream, args, bins, tasks);
 }
@@ -506,7 +569,7 @@ cudaError_t launch_alphabet(tape_t const &queries, tape_t const &candidates, boo
                                                   stream, queries, has_candidates ? candidates : queries, per_tape,
                                                   sample_bytes, mask);
     if (status != cudaSuccess) return status;
-    return launch_prioritised(alphabet_codes_kernel, 1, 32, stream, mask, alphabet);
+    return launch_prioritised(alphabet_codes_kernel, 1, 256, stream, mask, alphabet);
 }
 
 cudaError_t launch_scatter_output(plan_args_t const &args, std::int64_t const *results, std::int64_t *out,

@@ -66,6 +66,9 @@ constexpr int short_max_rows_k = 128;  // default: shorter sides up to this take
 static_assert(bin_short_begin_k + short_shapes_k * short_m_classes_k <= bin_keys_k, "bin layout exceeds the key space");
 constexpr int bin_myers_chain_k = bin_short_begin_k + short_shapes_k * short_m_classes_k; // 1824
 static_assert(bin_myers_chain_k < bin_keys_k, "bin layout exceeds the key space");
+constexpr int near_min_words_k = 5; // patterns of the thread route that the near-diagonal kernel tries
+constexpr std::uint32_t near_samples_k = 128; // pairs sampled per call
+constexpr std::uint32_t near_trial_k = 4096; // pairs tried near the diagonal before a batch may be found unrelated
 constexpr std::uint32_t myers_chain_max_rows_k = 1u << 20; // longest pattern a chain of warps takes
 
 /** Which pairs a call scores. */
@@ -108,6 +111,7 @@ struct plan_args_t {
     std::uint16_t packed_step_cost[4];  // relative cost of one lane step with 4, 8, 12, 16 rows per lane
     std::uint32_t band_min_rows_compare; // the same for compare-mode Levenshtein pairs (no profile)
     std::uint32_t short_max_rows;        // 16x2 pairs whose shorter side is at most this take the short route
+    std::uint32_t near_sample_stride;    // unit-cost calls: every so many pairs one is sampled for likeness (0: none)
 };
 
 /** Per-bin counters the planner fills. */
@@ -123,7 +127,10 @@ struct plan_bins_t {
     std::uint32_t max_myers_rows;      // longest pattern on the thread-per-pair bit-parallel route
     std::uint32_t max_myers_warp_rows; // longest pattern on the warp-per-pair bit-parallel route
     std::uint32_t max_chain_rows;      // longest pattern on the chained bit-parallel route
+    std::uint32_t near_tried, near_failed; // pairs the near-diagonal kernel has tried, and those it had to list
+    std::uint32_t near_sampled, near_alike; // pairs the planner sampled for likeness, and those found alike
     std::uint32_t reserved;
+    std::uint32_t listed[32];              // pairs it listed per class of full kernel (words; 16 + words per lane)
 };
 
 } // namespace szs_gb300

@@ -1134,3 +1134,80 @@ def test_direct_cross_product_edges(szs, port, longest):
         got = out.cpu().numpy()
         np.testing.assert_array_equal(got[:, :len(candidates)], want)
         assert (got[:, len(candidates):] == -1).all()
+
+
+def near_diagonal_pairs(rng, alphabet, count, low, high, shifts):
+    """Pairs whose optimal paths run along and just past the window of the near-diagonal kernel: a run of `s` symbols
+    inserted early and `t` deleted late (or the other way round), plus a few substitutions; near-identical, unrelated and
+    unequal pairs among them; the first symbol of the alphabet in runs."""
+    first, second = [], []
+    for i in range(count):
+        n = int(rng.integers(low, high + 1))
+        a = rng.choice(alphabet, size=n)
+        if i % 11 == 0:
+            a[: n // 2] = alphabet[0]
+        b = a.copy()
+        s, t = int(rng.choice(shifts)), int(rng.choice(shifts))
+        if i % 7 == 0:
+            b = rng.choice(alphabet, size=max(1, n + int(rng.integers(-40, 41))))
+        elif i % 7 < 5:
+            at = int(rng.integers(0, max(1, n // 3)))
+            b = np.concatenate([b[:at], rng.choice(alphabet, size=s), b[at:]])
+            late = len(b) - int(rng.integers(0, max(1, n // 3)))
+            b = np.concatenate([b[: max(late - t, at)], b[late:]])
+        where = rng.random(len(b)) < rng.choice([0.0, 0.01, 0.05, 0.2])
+        b[where] = rng.choice(alphabet, size=int(where.sum()))
+        if i % 2:
+            a, b = b, a
+        first.append(a), second.append(b)
+    return first, second
+
+
+@pytest.mark.parametrize("name,alphabet,low,high", [
+    ("dna", DNA, 100, 512), ("dna-n", np.frombuffer(b"ACGTN", np.uint8), 120, 300),
+    ("bytes", np.arange(256, dtype=np.uint8), 128, 330), ("two", np.array([0, 255], np.uint8), 120, 200)])
+def test_near_diagonal_pairs(szs, port, name, alphabet, low, high):
+    rng = np.random.default_rng(zlib_seed(name))
+    first, second = near_diagonal_pairs(rng, alphabet, 3000, low, high, [0, 1, 15, 30, 31, 32, 33, 34])
+    first, second = [bytes(a) for a in first], [bytes(b) for b in second]
+    engine = szs.LevenshteinDistances()
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_costs(), tape(first), tape(second)))
+
+
+def test_near_diagonal_long_reads(szs, port):
+    """The nine-word window (128 rows either side) of long DNA reads, which takes batches larger than the warp route
+    scores at once; every words-per-lane class, with some pairs listed back to it."""
+    rng = np.random.default_rng(99)
+    first, second = near_diagonal_pairs(rng, DNA, 2700, 520, 1300, [0, 3, 60, 100, 126, 127, 128, 129, 130])
+    for n in (2047, 3100, 5000, 8192):
+        more = near_diagonal_pairs(rng, DNA, 8, n - 40, n, [0, 100, 128, 200])
+        first += more[0]
+        second += more[1]
+    first, second = [bytes(a) for a in first], [bytes(b) for b in second]
+    engine = szs.LevenshteinDistances()
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_costs(), tape(first), tape(second)))
+
+
+def test_near_diagonal_unrelated_batch(szs, port):
+    """Unrelated strings: after the first pairs tried in vain, the rest of the batch goes to the full kernels untried."""
+    rng = np.random.default_rng(5)
+    first = random_strings(rng, 40000, 129, 200, DNA)
+    second = random_strings(rng, 40000, 129, 200, DNA)
+    engine = szs.LevenshteinDistances()
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_costs(), tape(first), tape(second)))
+
+
+@pytest.mark.parametrize("points", [300, 3000])
+def test_near_diagonal_code_points(szs, port, points):
+    """UTF-8 pairs over 16-bit codes: three-word windows over 16 planes on both the thread and the warp route's bins."""
+    rng = np.random.default_rng(points)
+    alphabet = np.arange(0x4E00, 0x4E00 + points, dtype=np.uint32)
+    first, second = near_diagonal_pairs(rng, alphabet, 900, 120, 420, [0, 1, 31, 32, 33])
+    first = ["".join(map(chr, a)) for a in first]
+    second = ["".join(map(chr, b)) for b in second]
+    engine = szs.LevenshteinDistancesUTF8()
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_utf8_costs(), tape(first), tape(second)))
