@@ -47,7 +47,7 @@ __device__ __forceinline__ void direct_string(tape_t const &tape, std::uint64_t 
         begin = offsets[index], end = offsets[index + 1];
     }
     start = tape.base + begin;
-    length = end - begin;
+    length = tape.lengths ? tape.lengths[index] : end - begin;
 }
 
 /** Bytes between two rows of the match-mask table of patterns of `words` words. */
@@ -171,34 +171,29 @@ __global__ void __launch_bounds__(256, most_ <= 4 ? 5 : (most_ <= 16 ? 3 : 2))
     }
 }
 
-/** The longest string of each tape (one CTA each), and its data's bytes, straight into page-locked host memory. */
+/** The longest string of each tape (one CTA each), and the sum of their lengths, straight into page-locked host memory. */
 __global__ void __launch_bounds__(1024) direct_extents_kernel(tape_t const queries, tape_t const candidates,
                                                               std::uint64_t *__restrict__ extents) {
-    __shared__ unsigned long long longest_s;
-    if (threadIdx.x == 0) longest_s = 0;
+    __shared__ unsigned long long longest_s, sum_s;
+    if (threadIdx.x == 0) longest_s = 0, sum_s = 0;
     __syncthreads();
     tape_t const &tape = blockIdx.x ? candidates : queries;
-    unsigned long long longest = 0;
+    unsigned long long longest = 0, sum = 0;
 #pragma unroll 8
     for (std::uint64_t i = threadIdx.x; i < tape.count; i += blockDim.x) {
         std::uint8_t const *start;
         std::uint64_t length;
         direct_string(tape, i, start, length);
-        longest = max(longest, (unsigned long long)length);
+        longest = max(longest, (unsigned long long)length), sum += length;
     }
 #pragma unroll
-    for (int distance = 16; distance; distance >>= 1)
+    for (int distance = 16; distance; distance >>= 1) {
         longest = max(longest, __shfl_xor_sync(0xFFFFFFFFu, longest, distance));
-    if ((threadIdx.x & 31) == 0) atomicMax(&longest_s, longest);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        std::uint8_t const *first, *end;
-        std::uint64_t length;
-        direct_string(tape, 0, first, length);
-        direct_string(tape, tape.count - 1, end, length);
-        extents[2 * blockIdx.x] = longest_s;
-        extents[2 * blockIdx.x + 1] = (std::uint64_t)(end + length - first);
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, distance);
     }
+    if ((threadIdx.x & 31) == 0) atomicMax(&longest_s, longest), atomicAdd(&sum_s, sum);
+    __syncthreads();
+    if (threadIdx.x == 0) extents[2 * blockIdx.x] = longest_s, extents[2 * blockIdx.x + 1] = sum_s;
 }
 
 } // namespace

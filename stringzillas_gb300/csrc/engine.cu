@@ -573,6 +573,7 @@ static status_t stage_tape(tape_view_t const &tape, staging_plan_t const &plan, 
                            tape_t &staged, cudaStream_t stream) noexcept {
     staged.count = tape.count;
     staged.offset_bits = tape.offset_bits;
+    staged.lengths = nullptr;
     unsigned char *cursor = area;
     if (plan.offsets_on_device) staged.offsets = tape.offsets;
     else {
@@ -642,57 +643,53 @@ static status_t finish_deferred(device_context_t *context, szs_gb300_stats_t &st
 static status_t transcode_utf8(device_context_t *context, cudaStream_t stream, tape_t &queries, tape_t &candidates,
                                bool has_candidates, bool &wide) noexcept {
     tape_t *tapes[2] = {&queries, has_candidates ? &candidates : nullptr};
-    std::uint64_t first[2] = {0, 0}, end[2] = {0, 0};
-    // The tapes' extents: the transcoded data can hold no more runes than bytes.
-    for (int t = 0; t < 2; ++t) {
-        if (!tapes[t]) continue;
-        std::size_t const size = tapes[t]->offset_bits == 32 ? 4 : 8;
-        auto const *offsets = static_cast<unsigned char const *>(tapes[t]->offsets);
-        SZS_TRY_CUDA(cudaMemcpyAsync(&first[t], offsets, size, cudaMemcpyDeviceToHost, stream));
-        SZS_TRY_CUDA(cudaMemcpyAsync(&end[t], offsets + tapes[t]->count * size, size, cudaMemcpyDeviceToHost, stream));
-    }
+    // The tapes' extents: a string has no more code points than bytes, so its codes fit at its bytes' positions.
+    std::uint64_t const *extents = context->spare_host();
+    SZS_TRY_CUDA(launch_utf8_extents(queries, has_candidates ? candidates : queries, context->spare_host(), stream));
     SZS_TRY_CUDA(cudaStreamSynchronize(stream));
-    std::size_t layout[2][3] = {}; // counts, offsets, data
+    std::uint64_t const first[2] = {extents[0], extents[2]}, end[2] = {extents[1], extents[3]};
+    std::size_t layout[2][3] = {}; // counts, 16-bit values, one-byte codes
     std::size_t cursor = align_up(sizeof(rune_set_t), 256);
-    std::size_t scan_bytes = 0;
     for (int t = 0; t < 2; ++t) {
         if (!tapes[t]) continue;
-        std::uint64_t const count = tapes[t]->count;
-        layout[t][0] = cursor, cursor += align_up((count + 1) * 8, 256);
-        layout[t][1] = cursor, cursor += align_up((count + 1) * 8, 256);
-        // Room for two bytes per code (more than 256 code points) and a whole 8-byte chunk past the end.
-        layout[t][2] = cursor, cursor += align_up(2 * (end[t] - first[t]) + 8, 256);
-        scan_bytes = std::max(scan_bytes, utf8_scan_scratch_bytes(count));
+        // Room for a whole 8-byte chunk past the end of both.
+        layout[t][0] = cursor, cursor += align_up(tapes[t]->count * 8, 256);
+        layout[t][1] = cursor, cursor += align_up(2 * (end[t] - first[t]) + 8, 256);
+        layout[t][2] = cursor, cursor += align_up(end[t] - first[t] + 8, 256);
     }
-    std::size_t const scan_at = cursor;
-    status_t status = context->utf8.reserve(cursor + align_up(scan_bytes, 256), stream);
+    status_t status = context->utf8.reserve(cursor, stream);
     if (!status.ok()) return status;
     auto *area = static_cast<unsigned char *>(context->utf8.data);
     auto *set = reinterpret_cast<rune_set_t *>(area);
-    SZS_TRY_CUDA(cudaMemsetAsync(set, 0, sizeof(rune_set_t), stream));
-    for (int t = 0; t < 2; ++t) {
-        if (!tapes[t]) continue;
-        auto *counts = reinterpret_cast<std::uint64_t *>(area + layout[t][0]);
-        SZS_TRY_CUDA(cudaMemsetAsync(counts, 0, (tapes[t]->count + 1) * 8, stream));
-        SZS_TRY_CUDA(launch_utf8_count(*tapes[t], end[t], counts, set, context->sm_count, stream));
-    }
+    SZS_TRY_CUDA(cudaMemsetAsync(set->present, 0, sizeof(set->present), stream));
+    SZS_TRY_CUDA(cudaMemsetAsync(&set->symbols, 0, sizeof(set->symbols) + sizeof(set->beyond), stream));
+    for (int t = 0; t < 2; ++t)
+        if (tapes[t])
+            SZS_TRY_CUDA(launch_utf8_decode(*tapes[t], end[t], reinterpret_cast<std::uint64_t *>(area + layout[t][0]), set,
+                                            reinterpret_cast<std::uint16_t *>(area + layout[t][1]), context->sm_count,
+                                            stream));
     SZS_TRY_CUDA(launch_utf8_codes(set, stream));
-    std::uint32_t seen[2] = {0, 0}; // symbols, overflow
-    SZS_TRY_CUDA(cudaMemcpyAsync(seen, &set->symbols, sizeof(seen), cudaMemcpyDeviceToHost, stream));
+    auto *seen = reinterpret_cast<std::uint32_t *>(context->spare_host()); // symbols, beyond
+    SZS_TRY_CUDA(cudaMemcpyAsync(seen, &set->symbols, 2 * sizeof(std::uint32_t), cudaMemcpyDeviceToHost, stream));
     SZS_TRY_CUDA(cudaStreamSynchronize(stream));
-    if (seen[1] || seen[0] > 65536)
+    std::uint32_t const symbols = seen[0];
+    bool const beyond = seen[1] != 0;
+    if (symbols > 65536)
         return {sz_unexpected_dimensions_k, "A UTF-8 call may use at most 65,536 distinct code points"};
-    wide = seen[0] > 256; // 16-bit codes beyond 256 code points
+    wide = symbols > 256; // 16-bit codes beyond 256 code points
     for (int t = 0; t < 2; ++t) {
         if (!tapes[t]) continue;
         auto const *counts = reinterpret_cast<std::uint64_t const *>(area + layout[t][0]);
-        auto *offsets = reinterpret_cast<std::uint64_t *>(area + layout[t][1]);
-        auto *data = reinterpret_cast<std::uint8_t *>(area + layout[t][2]);
-        SZS_TRY_CUDA(launch_utf8_scan(counts, offsets, tapes[t]->count, area + scan_at, scan_bytes, stream));
-        SZS_TRY_CUDA(launch_utf8_write(*tapes[t], end[t], offsets, set, data, wide, context->sm_count, stream));
-        tapes[t]->base = data;
-        tapes[t]->offsets = offsets;
-        tapes[t]->offset_bits = 64;
+        auto *values = reinterpret_cast<std::uint16_t *>(area + layout[t][1]);
+        auto *bytes = reinterpret_cast<std::uint8_t *>(area + layout[t][2]);
+        if (beyond)
+            SZS_TRY_CUDA(launch_utf8_write(*tapes[t], end[t], counts, set, wide ? static_cast<void *>(values) : bytes, wide,
+                                           context->sm_count, stream));
+        else if (!wide)
+            SZS_TRY_CUDA(launch_utf8_recode(*tapes[t], counts, set, values, bytes, context->sm_count, stream));
+        // Kernels address `base + offsets[i]` (twice the offset for 16-bit codes); the codes start at offsets[0].
+        tapes[t]->base = wide ? reinterpret_cast<std::uint8_t const *>(values) - 2 * first[t] : bytes - first[t];
+        tapes[t]->lengths = counts;
     }
     if (!has_candidates) candidates = queries;
     return {};
@@ -2193,7 +2190,7 @@ sz_status_t fingerprint_call(void *engine_handle, void *scope_handle, tape_view_
     if (!status.ok()) return report(status, error_message);
     status = context->inputs.reserve(align_up(plan.offsets_bytes, 256) + align_up(plan.data_bytes, 256) + 512, stream);
     if (!status.ok()) return report(status, error_message);
-    tape_t staged;
+    tape_t staged {};
     status = stage_tape(texts, plan, static_cast<unsigned char *>(context->inputs.data), staged, stream);
     if (!status.ok()) return report(status, error_message);
     // Parameters, once per device.

@@ -28,8 +28,8 @@ constexpr std::uint64_t direct_max_rows_k = 1024; // longest pattern of the dire
  *  about 0.33 ms for a pair of 1,000 bytes however few there are, where the warp-per-pair kernel spreads few pairs over
  *  more SMs (256 pairs 0.28 ms, 2,560 0.45 ms, 3,600 0.54 ms). */
 constexpr std::uint64_t direct_min_pairs_k = 1536;
-/** The longest string of both tapes and the bytes of their data into `extents` (4 values in page-locked host memory:
- *  longest query, query bytes, longest candidate, candidate bytes). */
+/** The longest string of both tapes and the sums of their lengths into `extents` (4 values in page-locked host memory:
+ *  longest query, all queries, longest candidate, all candidates). */
 cudaError_t launch_direct_extents(tape_t const &queries, tape_t const &candidates, std::uint64_t *extents,
                                   cudaStream_t stream);
 /** Whether the direct kernels take a unit-cost cross product with these longest strings; `swapped`: with the
@@ -89,22 +89,25 @@ struct rune_set_t {
     std::uint32_t present[rune_words_k]; // bit (r & 31) of word r >> 5: code point r occurs in the batch
     std::uint32_t rank[rune_words_k];    // distinct code points below word w's first
     std::uint32_t symbols;               // distinct code points
-    std::uint32_t overflow;              // always 0: every decodable value has its bit
+    std::uint32_t beyond;                // a code point beyond the Basic Multilingual Plane occurs
 };
-/** Counts each string's code points into `counts[i]` and marks them in `set` (both zeroed by the caller);
- *  `end` is the tape's last offset: a sequence cut off there reads zeros beyond it. */
-cudaError_t launch_utf8_count(tape_t const &tape, std::uint64_t end, std::uint64_t *counts, rune_set_t *set,
-                              int sm_count, cudaStream_t stream);
+/** The first and last offsets of both tapes into `extents` (4 values in page-locked host memory). */
+cudaError_t launch_utf8_extents(tape_t const &queries, tape_t const &candidates, std::uint64_t *extents,
+                                cudaStream_t stream);
+/** Counts each string's code points into `counts[i]`, marks them in `set` (its bitmap, `symbols` and `beyond` zeroed by
+ *  the caller) and writes them as 16-bit values at `values` + the string's offset from the tape's first; `end` is the
+ *  tape's last offset: a sequence cut off there reads zeros beyond it. */
+cudaError_t launch_utf8_decode(tape_t const &tape, std::uint64_t end, std::uint64_t *counts, rune_set_t *set,
+                               std::uint16_t *values, int sm_count, cudaStream_t stream);
 /** Ranks the set's bitmap words and counts the distinct code points (one CTA). */
 cudaError_t launch_utf8_codes(rune_set_t *set, cudaStream_t stream);
-/** Device scratch the exclusive scan of `count + 1` counts needs. */
-std::size_t utf8_scan_scratch_bytes(std::uint64_t count);
-/** `offsets[0..count]` = exclusive scan of `counts[0..count]` (counts[count] must be 0). */
-cudaError_t launch_utf8_scan(std::uint64_t const *counts, std::uint64_t *offsets, std::uint64_t count, void *scratch,
-                             std::size_t scratch_bytes, cudaStream_t stream);
-/** Writes each string's codes at `out + offsets[i]` (in codes): one byte each, or 16 bits each when `wide`. */
-cudaError_t launch_utf8_write(tape_t const &tape, std::uint64_t end, std::uint64_t const *offsets,
-                              rune_set_t const *set, void *out, bool wide, int sm_count, cudaStream_t stream);
+/** The values of a call over at most 256 code points, none beyond the plane, as one-byte ranks at the same positions. */
+cudaError_t launch_utf8_recode(tape_t const &tape, std::uint64_t const *counts, rune_set_t const *set,
+                               std::uint16_t const *values, std::uint8_t *out, int sm_count, cudaStream_t stream);
+/** Walks the strings again and writes each one's ranks at `out` + its offset from the tape's first (in codes): one byte
+ *  each, or 16 bits each when `wide`. */
+cudaError_t launch_utf8_write(tape_t const &tape, std::uint64_t end, std::uint64_t const *counts, rune_set_t const *set,
+                              void *out, bool wide, int sm_count, cudaStream_t stream);
 
 /** Shape of a wavefront-DP launch for one engine configuration. */
 struct dp_launch_shape_t {

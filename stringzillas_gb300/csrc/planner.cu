@@ -23,7 +23,7 @@ __device__ __forceinline__ void tape_string(tape_t const &tape, std::uint64_t in
         begin = offsets[index], end = offsets[index + 1];
     }
     start = tape.base + (wide ? 2 * begin : begin); // 16-bit codes: lengths stay in codes
-    length = end - begin;
+    length = tape.lengths ? tape.lengths[index] : end - begin;
 }
 
 /** Maps a flat pair index onto (query, candidate); the symmetric form walks the lower triangle row by row, the

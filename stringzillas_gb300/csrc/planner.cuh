@@ -78,12 +78,14 @@ enum pair_mode_t : int {
     mode_symmetric_k = 2, // (q, c) for c <= q, mirrored on output
 };
 
-/** A tape as the kernels see it: `base + offsets[i]` is the start of string i. */
+/** A tape as the kernels see it: `base + offsets[i]` is the start of string i, which ends where string i + 1 starts, or
+ *  after `lengths[i]` symbols where there are lengths (transcoded UTF-8: codes at the positions of the bytes). */
 struct tape_t {
     std::uint8_t const *base;
     void const *offsets;
     std::uint64_t count;
     int offset_bits; // 32 or 64
+    std::uint64_t const *lengths;
 };
 
 /** Everything the planning kernels need. */

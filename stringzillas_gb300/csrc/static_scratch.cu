@@ -202,7 +202,7 @@ sz_status_t static_scratch_pairwise(static_call_t const &call, sz_sequence_u64ta
     if (status == cudaSuccess) status = cudaMemsetAsync(scratch, 0, static_scratch_control_bytes_k, call.stream);
     if (status != cudaSuccess) return fail(sz_status_unknown_k, cudaGetErrorName(status));
 
-    tape_t a, b;
+    tape_t a {}, b {};
     a.base = reinterpret_cast<std::uint8_t const *>(first->data), a.offsets = first->offsets;
     a.count = first->count, a.offset_bits = 64;
     b.base = reinterpret_cast<std::uint8_t const *>(second->data), b.offsets = second->offsets;

@@ -11,16 +11,16 @@
  *  bytes are not checked, so a sequence cut off by the end of a string reads on into the next string of the tape.
  *  The same rule is applied here; bytes past the end of the tape read as 0.
  *
- *  Passes: (1) one warp per string walks its runes, counts them and marks each in a bitmap of code points (a CTA
- *  marks the Basic Multilingual Plane in shared memory, 8 KB, and merges it into the global bitmap once at its end;
- *  rarer code points are marked in the global bitmap directly); (2) one CTA ranks the bitmap's words, so a code
- *  point's code is the number of distinct code points below it; (3) after an exclusive scan of the counts, one warp
- *  per string writes its codes, each the word's rank plus a population count (the Basic Multilingual Plane's ranks and
- *  bits staged in shared memory, 16 KB). A warp decodes 128 bytes at once when the string is well formed
- *  (`warp_walk`), else its first lane walks the string with the sequential rule above.
+ *  Passes: (1) one warp per string walks its code points, counts them, marks each in a bitmap (a CTA marks the Basic
+ *  Multilingual Plane in shared memory, 8 KB, and merges what the global bitmap lacks at its end; rarer code points are
+ *  marked in the global bitmap directly) and writes them as 16-bit values, from the code unit of the string's first byte
+ *  on, so no scan of the counts is needed and the tapes keep their offsets beside the counts as lengths. (2) One CTA
+ *  ranks the bitmap's words, so a code point's rank is the number of distinct code points below it. A call over more
+ *  than 256 code points, all inside that plane, is then done: its codes are the code points. (3) Calls over at most 256
+ *  are recoded from the 16-bit values to one-byte ranks, and calls with code points beyond the plane walk their strings
+ *  again and write ranks. 65,536 pairs of 100-300 CJK ideographs (79.7 MB): 0.72 ms with a counting and a writing walk,
+ *  a scan and byte loads, 0.20 ms now.
  */
-#include <cub/device/device_scan.cuh>
-
 #include "launchers.h"
 
 namespace szs_gb300 {
@@ -50,114 +50,138 @@ __device__ __forceinline__ std::uint64_t tape_offset(tape_t const &tape, std::ui
 constexpr std::uint32_t plane_words_k = 65536 / 32; // the Basic Multilingual Plane's 2,048 bitmap words
 constexpr int utf8_threads_k = 128;
 
-/** Bit k (k < 4) set where byte k of `x` is a continuation byte (10xxxxxx). */
-__device__ __forceinline__ std::uint32_t continuation_bits(std::uint32_t x) {
-    std::uint32_t const tops = x & ~(x << 1) & 0x80808080u; // bit 7 of a byte: its bit 7 set and bit 6 clear
-    return ((tops >> 7) * 0x01020408u) >> 24;                // gather bits 0, 8, 16, 24 into bits 0..3
-}
-
 /**
- *  One warp walks the string [begin, stop) 128 bytes at a time, lane L on bytes 4L..4L+3 of each window (coalesced
- *  loads), and calls `visit(rune, index)` once per code point, on the lane holding its lead byte, `index` counting
- *  code points from the string's start. This holds only when the string is well formed in the decoder's sense: its
- *  first byte is a lead byte and every lead byte's length covers exactly the continuation bytes (10xxxxxx) that follow
- *  it, ending at `stop`; then the code points start exactly at the lead bytes, as a sequential walk would find them,
- *  and no byte past `stop` is needed. Returns false, warp-uniformly, as soon as a window breaks that (code points
- *  visited before stay visited: both passes then walk the whole string again sequentially), or for strings of 2^31
- *  bytes or more. Sets `count` to the string's code points on success. Offsets inside the string are 32-bit and the
- *  checks are mask arithmetic, without branches.
+ *  One warp walks the string [begin, stop) 128 bytes at a time, lane L on bytes 4L..4L+3 of each window (from aligned
+ *  words, shifted to the string's own alignment), and calls `visit(rune, index)` once per code point, `index` counting
+ *  code points from the string's start: consecutive lanes hold consecutive code points. This holds only when the string
+ *  is well formed in the decoder's sense: its continuation bytes (10xxxxxx) are exactly those that its lead bytes ask
+ *  for, the byte after every lead of 0xC0 or more, the second after 0xE0 or more and the third after 0xF0 or more, none
+ *  past `stop`; then the code points start exactly at the other bytes, as a sequential walk would find them. Returns
+ *  false, warp-uniformly, as soon as a window breaks that (code points visited before stay visited: both passes then
+ *  walk the whole string again sequentially), or for strings of 2^31 bytes or more. Sets `count` to the string's code
+ *  points on success. `positions`: 128 bytes of shared memory of the warp's own.
  */
 template <typename visit_>
 __device__ __forceinline__ bool warp_walk(tape_t const &tape, std::uint64_t begin, std::uint64_t stop,
-                                          std::uint64_t &count, visit_ &&visit) {
+                                          std::uint8_t *positions, std::uint64_t &count, visit_ &&visit) {
     if (stop - begin >= (1ull << 31)) return false;
     std::uint32_t const n = (std::uint32_t)(stop - begin);
-    std::uint8_t const *string = tape.base + begin;
+    count = 0;
+    if (!n) return true;
+    std::uintptr_t const address = reinterpret_cast<std::uintptr_t>(tape.base + begin);
+    std::uint32_t const *aligned = reinterpret_cast<std::uint32_t const *>(address & ~std::uintptr_t(3));
+    std::uint32_t const skew = (std::uint32_t)(address & 3), last = (skew + n - 1) >> 2;
     int const lane = threadIdx.x & 31;
     std::uint32_t const lower = (1u << lane) - 1u;
-    std::uint64_t runes = 0;
+    std::uint32_t runes = 0;
+    std::uint32_t asked = 0; // lane 0: continuation bytes that the last window's leads ask of this window's first bytes
     for (std::uint32_t window = 0; window < n; window += 128) {
-        std::uint32_t const rel = window + 4u * (std::uint32_t)lane;
-        // This lane's four bytes, and the four after them (the next lane's, or the next window's for lane 31);
-        // bytes past the string read as 0 and never decide a well-formed string.
-        std::uint32_t own = 0, ahead = 0;
-#pragma unroll
-        for (std::uint32_t k = 0; k < 4; ++k) {
-            own |= (rel + k < n ? (std::uint32_t)string[rel + k] : 0u) << (8 * k);
-            if (lane == 0) ahead |= (window + 128 + k < n ? (std::uint32_t)string[window + 128 + k] : 0u) << (8 * k);
+        std::uint32_t const at = window / 4 + lane;
+        std::uint32_t const a = __ldg(aligned + min(at, last)), b = __ldg(aligned + min(at + 1, last)),
+                            c = __ldg(aligned + min(at + 2, last));
+        std::uint32_t own = __funnelshift_r(a, b, 8 * skew);
+        std::uint32_t const high = __funnelshift_r(b, c, 8 * skew); // read only where a sequence goes on
+        std::uint32_t valid = 0x80808080u;
+        if (window + 128 > n) {
+            int const keep = (int)n - (int)(window + 4 * lane); // this lane's bytes inside the string
+            std::uint32_t const mask = keep >= 4 ? 0xFFFFFFFFu : (keep <= 0 ? 0u : 0xFFFFFFFFu >> (32 - 8 * keep));
+            own &= mask, valid &= mask;
         }
-        std::uint32_t const next_lane = __shfl_sync(0xFFFFFFFFu, own, (lane + 1) & 31);
-        std::uint32_t const next_window = __shfl_sync(0xFFFFFFFFu, ahead, 0);
-        std::uint32_t const high = lane == 31 ? next_window : next_lane;
-        std::uint32_t const continuation = continuation_bits(own) | continuation_bits(high) << 4;
-
-        bool ok = !(rel == 0 && (continuation & 1u)); // the string starts on a lead byte
-        std::uint32_t leads = 0, lengths = 0;          // lengths: 4 bits per byte slot
+        if (!__any_sync(0xFFFFFFFFu, (own & 0x80808080u) | asked)) { // ASCII
+            std::uint32_t const total = min(128u, n - window);
 #pragma unroll
-        for (std::uint32_t j = 0; j < 4; ++j) {
-            std::uint32_t const position = rel + j;
-            std::uint32_t const byte = (own >> (8 * j)) & 0xFFu;
-            bool const lead = position < n && !((continuation >> j) & 1u);
-            // Lead bytes' lengths from their leading ones: 0 -> 1, 2 -> 2, 3 -> 3, 4 or more -> 4.
-            std::uint32_t const length = min(max((std::uint32_t)__clz(~(byte << 24)), 1u), 4u);
-            std::uint32_t const needed = ((1u << (length - 1)) - 1u) << (j + 1);
-            bool const covered = position + length <= n && (continuation & needed) == needed &&
-                                 (position + length == n || !((continuation >> (j + length)) & 1u));
-            ok = ok && (!lead || covered);
-            leads |= (lead ? 1u : 0u) << j;
-            lengths |= length << (4 * j);
+            for (std::uint32_t k = 0; k < 128; k += 32) {
+                std::uint32_t const p = k + lane;
+                std::uint32_t const word = __shfl_sync(0xFFFFFFFFu, own, p >> 2);
+                if (p < total) visit(__byte_perm(word, 0u, 0x4440u + (p & 3u)), (std::uint64_t)(runes + p));
+            }
+            runes += total;
+            continue;
         }
-        if (!__all_sync(0xFFFFFFFFu, ok)) return false;
-        std::uint32_t before = 0, total = 0; // code points of lower lanes in this window, and of the whole window
+        // Per byte, in its top bit: continuation bytes, and leads of two, three and four bytes.
+        std::uint32_t const continuation = own & ~(own << 1) & 0x80808080u;
+        std::uint32_t const two = own & (own << 1) & 0x80808080u, three = two & (own << 2), four = three & (own << 3);
+        std::uint32_t const here = two << 8 | three << 16 | four << 24, beyond = two >> 24 | three >> 16 | four >> 8;
+        std::uint32_t const above = __shfl_up_sync(0xFFFFFFFFu, beyond, 1);
+        bool const broken = (here | (lane ? above : asked)) != continuation;
+        std::uint32_t const carried = __shfl_sync(0xFFFFFFFFu, beyond, 31);
+        asked = lane ? 0u : carried;
+        if (__any_sync(0xFFFFFFFFu, broken)) return false;
+        std::uint32_t const leads = (((valid & ~continuation) >> 7) * 0x01020408u) >> 24; // four bits
+        // The window's code points in order: their positions, so that lane k takes the k-th.
+        std::uint32_t const found = __popc(leads);
+        std::uint32_t const ones = __ballot_sync(0xFFFFFFFFu, found & 1u), twos = __ballot_sync(0xFFFFFFFFu, found & 2u),
+                            fours = __ballot_sync(0xFFFFFFFFu, found & 4u);
+        std::uint32_t const before = __popc(ones & lower) + 2u * __popc(twos & lower) + 4u * __popc(fours & lower);
+        std::uint32_t const total = __popc(ones) + 2u * __popc(twos) + 4u * __popc(fours);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            std::uint32_t const slot = __ballot_sync(0xFFFFFFFFu, (leads >> j) & 1u);
-            before += __popc(slot & lower), total += __popc(slot);
+        for (std::uint32_t j = 0; j < 4; ++j)
+            if ((leads >> j) & 1u) positions[before + __popc(leads & ((1u << j) - 1u))] = (std::uint8_t)(4 * lane + j);
+        __syncwarp();
+        for (std::uint32_t k = 0; k < total; k += 32) {
+            bool const live = k + lane < total;
+            std::uint32_t const p = live ? positions[k + lane] : 0u;
+            std::uint32_t const low_word = __shfl_sync(0xFFFFFFFFu, own, p >> 2);
+            std::uint32_t const high_word = __shfl_sync(0xFFFFFFFFu, high, p >> 2);
+            // The lead byte on top, then the three bytes after it; a sequence's bits are the top ones of 6 + 18.
+            std::uint32_t const bytes = __byte_perm(low_word, high_word, 0x0123u + 0x1111u * (p & 3u));
+            std::uint32_t const lead = bytes >> 24;
+            std::uint32_t const more = (lead >= 0xC0u) + (lead >= 0xE0u) + (lead >= 0xF0u);
+            std::uint32_t const sixes = bytes & 0x3F3F3F3Fu;
+            std::uint32_t const twelves = ((sixes >> 2) & 0x0FC00FC0u) | (sixes & 0x003F003Fu);
+            std::uint32_t const all = (twelves >> 16) << 12 | (twelves & 0xFFFu);
+            std::uint32_t const rune = more ? (all >> (18 - 6 * more)) & ((1u << (5 * more + 6)) - 1u) : lead;
+            if (live) visit(rune, (std::uint64_t)(runes + k + lane));
         }
-#pragma unroll
-        for (std::uint32_t j = 0; j < 4; ++j) {
-            if (!((leads >> j) & 1u)) continue;
-            std::uint32_t const word = __funnelshift_r(own, high, 8 * j); // bytes j..j+3
-            std::uint32_t const length = (lengths >> (4 * j)) & 0xFu;
-            std::uint32_t const b0 = word & 0xFFu, c1 = (word >> 8) & 0x3Fu, c2 = (word >> 16) & 0x3Fu,
-                                c3 = (word >> 24) & 0x3Fu;
-            std::uint32_t const rune = length == 1   ? b0
-                                       : length == 2 ? (b0 & 0x1Fu) << 6 | c1
-                                       : length == 3 ? (b0 & 0x0Fu) << 12 | c1 << 6 | c2
-                                                     : (b0 & 0x07u) << 18 | c1 << 12 | c2 << 6 | c3;
-            visit(rune, runes + before + (std::uint64_t)__popc(leads & ((1u << j) - 1u)));
-        }
+        __syncwarp();
         runes += total;
     }
     count = runes;
-    return true;
+    return !__any_sync(0xFFFFFFFFu, asked); // a sequence cut off by the string's end
 }
 
-/** Pass 1: rune counts per string, and the bitmap of code points: one warp per string. */
-__global__ void __launch_bounds__(utf8_threads_k) utf8_count_kernel(tape_t const tape, std::uint64_t const end,
+/** Pass 1: code points per string, the bitmap, and the code points as 16-bit values (truncated beyond the Basic
+ *  Multilingual Plane, which sets `set->beyond`): one warp per string, written at `out` + its offset from the tape's
+ *  first. */
+__global__ void __launch_bounds__(utf8_threads_k) utf8_decode_kernel(tape_t const tape, std::uint64_t const end,
                                                                      std::uint64_t *__restrict__ counts,
-                                                                     rune_set_t *__restrict__ set) {
+                                                                     rune_set_t *__restrict__ set,
+                                                                     std::uint16_t *__restrict__ out) {
     __shared__ std::uint32_t plane_s[plane_words_k];
+    __shared__ std::uint8_t positions_s[utf8_threads_k / 32][128];
     for (std::uint32_t k = threadIdx.x; k < plane_words_k; k += blockDim.x) plane_s[k] = 0u;
     __syncthreads();
     auto mark = [&](std::uint32_t rune) {
         std::uint32_t const bit = 1u << (rune & 31u);
-        if (rune < 65536u) atomicOr(&plane_s[rune >> 5], bit);
-        else atomicOr(&set->present[rune >> 5], bit);
+        if (rune < 65536u) {
+            if (!(plane_s[rune >> 5] & bit)) atomicOr(&plane_s[rune >> 5], bit);
+        }
+        else {
+            atomicOr(&set->present[rune >> 5], bit);
+            set->beyond = 1u;
+        }
     };
     int const lane = threadIdx.x & 31;
+    std::uint64_t const first = tape_offset(tape, 0);
     std::uint64_t const warps = (std::uint64_t)gridDim.x * (blockDim.x >> 5);
     for (std::uint64_t i = (std::uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < tape.count;
          i += warps) {
         std::uint64_t const begin = tape_offset(tape, i), stop = tape_offset(tape, i + 1);
+        std::uint16_t *target = out + (begin - first);
         std::uint64_t runes = 0;
-        bool const walked = warp_walk(tape, begin, stop, runes,
-                                      [&](std::uint32_t rune, std::uint64_t) { mark(rune); });
+        bool const walked = warp_walk(tape, begin, stop, positions_s[threadIdx.x >> 5], runes,
+                                      [&](std::uint32_t rune, std::uint64_t index) {
+                                          mark(rune);
+                                          target[index] = (std::uint16_t)rune;
+                                      });
+        __syncwarp();
         if (!walked && lane == 0) { // the decoder's sequential rule, as the reference applies it
             runes = 0;
             for (std::uint64_t position = begin; position < stop; ++runes) {
                 std::uint32_t length;
-                mark(rune_at(tape.base, position, end, length));
+                std::uint32_t const rune = rune_at(tape.base, position, end, length);
+                mark(rune);
+                target[runes] = (std::uint16_t)rune;
                 position += length;
             }
         }
@@ -165,14 +189,15 @@ __global__ void __launch_bounds__(utf8_threads_k) utf8_count_kernel(tape_t const
     }
     __syncthreads();
     for (std::uint32_t k = threadIdx.x; k < plane_words_k; k += blockDim.x)
-        if (plane_s[k]) atomicOr(&set->present[k], plane_s[k]);
+        if (plane_s[k] & ~__ldcg(&set->present[k])) atomicOr(&set->present[k], plane_s[k]);
 }
 
 /** Pass 2: the rank of every bitmap word and the number of distinct code points (one CTA of 32 warps, each over a
- *  contiguous block of 2,048 words read 32 consecutive words at a time). */
+ *  contiguous block of words read 32 at a time): the Basic Multilingual Plane's words, and all 65,536 only when a code
+ *  point beyond it was marked. */
 __global__ void __launch_bounds__(1024) utf8_codes_kernel(rune_set_t *__restrict__ set) {
     constexpr int warps = 32;
-    constexpr std::uint32_t per_warp = rune_words_k / warps;
+    std::uint32_t const per_warp = (set->beyond ? rune_words_k : plane_words_k) / warps;
     __shared__ std::uint32_t warp_totals[warps];
     int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     std::uint32_t const *present = set->present + warp * per_warp;
@@ -202,13 +227,44 @@ __global__ void __launch_bounds__(1024) utf8_codes_kernel(rune_set_t *__restrict
     }
 }
 
-/** Pass 3: each string's codes at its scanned offset (one byte each, or two for more than 256 code points): one warp
- *  per string. */
+/** A string's room past its codes, filled with code 0 (one of the batch's, so that an alphabet pass over the tape's whole
+ *  range sees no other symbols). */
+__device__ __forceinline__ void fill_room(std::uint8_t *target, std::uint64_t codes, std::uint64_t room, int lane) {
+    for (std::uint64_t k = codes + lane; k < room; k += 32) target[k] = 0;
+}
+
+/** Pass 3, at most 256 code points, none beyond the plane: each string's 16-bit values as one-byte ranks. */
+__global__ void __launch_bounds__(utf8_threads_k)
+    utf8_recode_kernel(tape_t const tape, std::uint64_t const *__restrict__ counts, rune_set_t const *__restrict__ set,
+                       std::uint16_t const *__restrict__ values, std::uint8_t *__restrict__ out) {
+    __shared__ std::uint32_t present_s[plane_words_k], rank_s[plane_words_k];
+    for (std::uint32_t k = threadIdx.x; k < plane_words_k; k += blockDim.x)
+        present_s[k] = set->present[k], rank_s[k] = set->rank[k];
+    __syncthreads();
+    int const lane = threadIdx.x & 31;
+    std::uint64_t const first = tape_offset(tape, 0);
+    std::uint64_t const warps = (std::uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (std::uint64_t i = (std::uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < tape.count;
+         i += warps) {
+        std::uint64_t const begin = tape_offset(tape, i), room = tape_offset(tape, i + 1) - begin, codes = counts[i];
+        std::uint16_t const *source = values + (begin - first);
+        std::uint8_t *target = out + (begin - first);
+        for (std::uint64_t k = lane; k < codes; k += 32) {
+            std::uint32_t const rune = source[k];
+            target[k] = (std::uint8_t)(rank_s[rune >> 5] + __popc(present_s[rune >> 5] & ((1u << (rune & 31u)) - 1u)));
+        }
+        fill_room(target, codes, room, lane);
+    }
+}
+
+/** Pass 3, calls with code points beyond the plane: each string's ranks (one byte each, or two for more than 256 code
+ *  points), one warp per string. */
 template <typename code_type_>
 __global__ void __launch_bounds__(utf8_threads_k)
-    utf8_write_kernel(tape_t const tape, std::uint64_t const end, std::uint64_t const *__restrict__ offsets,
+    utf8_write_kernel(tape_t const tape, std::uint64_t const end, std::uint64_t const *__restrict__ counts,
                       rune_set_t const *__restrict__ set, code_type_ *__restrict__ out) {
     __shared__ std::uint32_t present_s[plane_words_k], rank_s[plane_words_k];
+    __shared__ std::uint8_t positions_s[utf8_threads_k / 32][128];
     for (std::uint32_t k = threadIdx.x; k < plane_words_k; k += blockDim.x)
         present_s[k] = set->present[k], rank_s[k] = set->rank[k];
     __syncthreads();
@@ -218,39 +274,53 @@ __global__ void __launch_bounds__(utf8_threads_k)
                              : __ldg(set->rank + word) + __popc(__ldg(set->present + word) & below);
     };
     int const lane = threadIdx.x & 31;
+    std::uint64_t const first = tape_offset(tape, 0);
     std::uint64_t const warps = (std::uint64_t)gridDim.x * (blockDim.x >> 5);
     for (std::uint64_t i = (std::uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < tape.count;
          i += warps) {
         std::uint64_t const begin = tape_offset(tape, i), stop = tape_offset(tape, i + 1);
-        code_type_ *target = out + offsets[i];
+        code_type_ *const target = out + (begin - first);
         std::uint64_t runes = 0;
-        bool const walked = warp_walk(tape, begin, stop, runes, [&](std::uint32_t rune, std::uint64_t index) {
-            target[index] = (code_type_)code_of(rune);
-        });
-        if (!walked && lane == 0) // the decoder's sequential rule, as the reference applies it
+        bool const walked = warp_walk(tape, begin, stop, positions_s[threadIdx.x >> 5], runes,
+                                      [&](std::uint32_t rune, std::uint64_t index) {
+                                          target[index] = (code_type_)code_of(rune);
+                                      });
+        __syncwarp();
+        if (!walked && lane == 0) { // the decoder's sequential rule, as the reference applies it
+            code_type_ *next = target;
             for (std::uint64_t position = begin; position < stop;) {
                 std::uint32_t length;
-                *target++ = (code_type_)code_of(rune_at(tape.base, position, end, length));
+                *next++ = (code_type_)code_of(rune_at(tape.base, position, end, length));
                 position += length;
             }
+        }
+        if constexpr (sizeof(code_type_) == 1) fill_room(target, counts[i], stop - begin, lane);
     }
+}
+
+/** Both tapes' first and last offsets, into page-locked host memory. */
+__global__ void utf8_extents_kernel(tape_t const queries, tape_t const candidates, std::uint64_t *__restrict__ extents) {
+    tape_t const &tape = threadIdx.x < 2 ? queries : candidates;
+    if (threadIdx.x < 4) extents[threadIdx.x] = tape_offset(tape, threadIdx.x & 1 ? tape.count : 0);
 }
 
 } // namespace
 
-std::size_t utf8_scan_scratch_bytes(std::uint64_t count) {
-    std::size_t bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, bytes, static_cast<std::uint64_t *>(nullptr),
-                                  static_cast<std::uint64_t *>(nullptr), (int)(count + 1));
-    return bytes;
+static int utf8_grid(std::uint64_t strings, int sm_count) {
+    std::uint64_t const blocks = (strings + utf8_threads_k / 32 - 1) / (utf8_threads_k / 32); // a warp per string
+    return (int)(blocks < (std::uint64_t)sm_count * 16 ? blocks : (std::uint64_t)sm_count * 16);
 }
 
-cudaError_t launch_utf8_count(tape_t const &tape, std::uint64_t end, std::uint64_t *counts, rune_set_t *set,
-                              int sm_count, cudaStream_t stream) {
+cudaError_t launch_utf8_extents(tape_t const &queries, tape_t const &candidates, std::uint64_t *extents,
+                                cudaStream_t stream) {
+    utf8_extents_kernel<<<1, 32, 0, stream>>>(queries, candidates, extents);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_utf8_decode(tape_t const &tape, std::uint64_t end, std::uint64_t *counts, rune_set_t *set,
+                               std::uint16_t *values, int sm_count, cudaStream_t stream) {
     if (!tape.count) return cudaSuccess;
-    std::uint64_t const blocks = (tape.count + utf8_threads_k / 32 - 1) / (utf8_threads_k / 32); // a warp per string
-    int const grid = (int)(blocks < (std::uint64_t)sm_count * 16 ? blocks : (std::uint64_t)sm_count * 16);
-    utf8_count_kernel<<<grid, utf8_threads_k, 0, stream>>>(tape, end, counts, set);
+    utf8_decode_kernel<<<utf8_grid(tape.count, sm_count), utf8_threads_k, 0, stream>>>(tape, end, counts, set, values);
     return cudaGetLastError();
 }
 
@@ -259,22 +329,21 @@ cudaError_t launch_utf8_codes(rune_set_t *set, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_utf8_scan(std::uint64_t const *counts, std::uint64_t *offsets, std::uint64_t count, void *scratch,
-                             std::size_t scratch_bytes, cudaStream_t stream) {
-    return cub::DeviceScan::ExclusiveSum(scratch, scratch_bytes, counts, offsets, (int)(count + 1), stream);
+cudaError_t launch_utf8_recode(tape_t const &tape, std::uint64_t const *counts, rune_set_t const *set,
+                               std::uint16_t const *values, std::uint8_t *out, int sm_count, cudaStream_t stream) {
+    if (!tape.count) return cudaSuccess;
+    utf8_recode_kernel<<<utf8_grid(tape.count, sm_count), utf8_threads_k, 0, stream>>>(tape, counts, set, values, out);
+    return cudaGetLastError();
 }
 
-cudaError_t launch_utf8_write(tape_t const &tape, std::uint64_t end, std::uint64_t const *offsets,
-                              rune_set_t const *set, void *out, bool wide, int sm_count, cudaStream_t stream) {
+cudaError_t launch_utf8_write(tape_t const &tape, std::uint64_t end, std::uint64_t const *counts, rune_set_t const *set,
+                              void *out, bool wide, int sm_count, cudaStream_t stream) {
     if (!tape.count) return cudaSuccess;
-    std::uint64_t const blocks = (tape.count + utf8_threads_k / 32 - 1) / (utf8_threads_k / 32); // a warp per string
-    int const grid = (int)(blocks < (std::uint64_t)sm_count * 16 ? blocks : (std::uint64_t)sm_count * 16);
+    int const grid = utf8_grid(tape.count, sm_count);
     if (wide)
-        utf8_write_kernel<<<grid, utf8_threads_k, 0, stream>>>(tape, end, offsets, set,
-                                                               static_cast<std::uint16_t *>(out));
+        utf8_write_kernel<<<grid, utf8_threads_k, 0, stream>>>(tape, end, counts, set, static_cast<std::uint16_t *>(out));
     else
-        utf8_write_kernel<<<grid, utf8_threads_k, 0, stream>>>(tape, end, offsets, set,
-                                                               static_cast<std::uint8_t *>(out));
+        utf8_write_kernel<<<grid, utf8_threads_k, 0, stream>>>(tape, end, counts, set, static_cast<std::uint8_t *>(out));
     return cudaGetLastError();
 }
 

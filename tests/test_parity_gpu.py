@@ -1211,3 +1211,44 @@ def test_near_diagonal_code_points(szs, port, points):
     engine = szs.LevenshteinDistancesUTF8()
     got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
     np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_utf8_costs(), tape(first), tape(second)))
+
+
+@pytest.mark.parametrize("alphabet", ["latin", "greek-cjk", "emoji-few", "emoji-many", "ascii"])
+def test_utf8_transcoding_windows(szs, port, alphabet):
+    """Strings around the transcoder's 128-byte windows: sequences of every length across their borders, windows of ASCII
+    between others, strings at every alignment, empty ones, malformed ones (a lone continuation byte, a sequence cut off
+    at the string's end or by a lead byte) among well-formed ones, few and many code points within and beyond the Basic
+    Multilingual Plane; pairwise and cross products, sliced tapes."""
+    rng = np.random.default_rng(zlib_seed(alphabet))
+    points = {"latin": list(range(32, 127)) + list(range(0xC0, 0x150)),
+              "greek-cjk": list(range(32, 60)) + list(range(0x391, 0x3C9)) + list(range(0x4E00, 0x4E00 + 700)),
+              "emoji-few": list(range(48, 100)) + list(range(0x1F600, 0x1F640)),
+              "emoji-many": list(range(48, 100)) + list(range(0x1F300, 0x1F500)) + list(range(0xFF00, 0xFFF0)),
+              "ascii": list(range(0, 128))}[alphabet]
+    points = np.array(points)
+
+    def make(count):
+        strings = []
+        for i in range(count):
+            text = rng.choice(points, size=int(rng.integers(0, 200)))
+            if i % 3 == 0:
+                text[: len(text) // 2] = 65
+            raw = "".join(map(chr, text)).encode()
+            if i % 10 == 7:
+                raw = raw[: int(rng.integers(0, len(raw) + 1))]
+            if i % 10 == 8:
+                at = int(rng.integers(0, len(raw) + 1))
+                raw = raw[:at] + bytes([int(rng.choice([0x80, 0xC3, 0xE4, 0xF0, 0xFF]))]) + raw[at:]
+            strings.append(raw)
+        return strings + [b"", "é".encode() * 64, b"a" * 127 + "é".encode(), b"a" * 126 + "中".encode(), b"a" * 128]
+    first, second = make(400), make(400)
+    engine = szs.LevenshteinDistancesUTF8()
+    costs = oracle.levenshtein_utf8_costs()
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    np.testing.assert_array_equal(got, port.pairs(costs, tape(first), tape(second)))
+    got = engine.pairwise(szs.Strs(first)[3:301], szs.Strs(second)[5:303]).astype(np.int64)
+    (a, a_offsets), (b, b_offsets) = tape(first), tape(second)
+    want = port.pairs(costs, (a, a_offsets[3:302].copy()), (b, b_offsets[5:304].copy()))
+    np.testing.assert_array_equal(got, want)
+    got = engine(szs.Strs(first[:60]), szs.Strs(second[:50])).astype(np.int64)
+    np.testing.assert_array_equal(got, port.cross(costs, tape(first[:60]), tape(second[:50])))
