@@ -34,7 +34,10 @@
 
 namespace szs_gb300 {
 
-constexpr int band_warps_k = 8;
+#ifndef SZS_BAND_WARPS
+#define SZS_BAND_WARPS 8
+#endif
+constexpr int band_warps_k = SZS_BAND_WARPS; // warps per CTA
 constexpr int band_chunk_k = 32;                      // columns staged and published at a time
 
 template <int kind_, bool affine_, int rows_per_lane_, int columns_per_step_ = 1>
@@ -145,7 +148,8 @@ __device__ __forceinline__ void band_publish(band_ring_t const &ring, int slot, 
 /** Most CTAs one long pair can share (enough for every 128-row strip of a 250,000-row pair to have its own warp, so
  *  no warp sweeps a second strip after its first), and the ring words of a group. */
 constexpr int band_group_max_ctas_k = 256;
-constexpr int band_group_max_members_k = band_group_max_ctas_k * band_warps_k;
+constexpr int band_group_max_members_k = band_group_max_ctas_k * 8; // whatever the build's warps per CTA, up to 8
+static_assert(band_warps_k <= 8, "a group's ring words hold eight warps per CTA");
 
 /** One pass over a pair (16-bit or 32-bit cells): ring progress and the combined result. */
 struct band_pass_state_t {

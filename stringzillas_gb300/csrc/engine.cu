@@ -1073,7 +1073,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         std::uint64_t const slots = (std::uint64_t)context->sm_count * shape.group_ctas_per_sm;
         if (pairs_here * 2 > slots) return;
         std::uint64_t const strips = ((std::uint64_t)plan.max_cols + strip_rows - 1) / strip_rows;
-        std::uint64_t const useful = (strips + band_warps_per_cta() - 1) / band_warps_per_cta();
+        std::uint64_t const useful = (strips + shape.warps_per_cta - 1) / shape.warps_per_cta;
         std::uint64_t const size = std::min<std::uint64_t>({slots / pairs_here, (std::uint64_t)band_group_max_ctas(),
                                                             useful});
         if (size < 2) return;
@@ -1081,8 +1081,8 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         ctas = (int)(std::min<std::uint64_t>(pairs_here, slots / group_ctas) * group_ctas);
     };
     auto band_job = [&](job_kind_t kind, int key_begin, int key_end, std::uint64_t pairs_here, int ctas, int group_ctas,
-                        dp_launch_shape_t const &shape, std::size_t bytes_per_cta) {
-        std::size_t const bytes = align_up(bytes_per_cta * (std::size_t)ctas, 256);
+                        dp_launch_shape_t const &shape, std::size_t bytes_per_warp) {
+        std::size_t const bytes = align_up(bytes_per_warp * (std::size_t)shape.warps_per_cta * (std::size_t)ctas, 256);
         job_t job {kind, kind == job_band16_k ? 16 : 32, 0, key_begin, key_end, pairs_here, ctas, scratch_total, bytes};
         job.fills = group_ctas > 1 || ctas >= context->sm_count * shape.ctas_per_sm;
         job.rows = shape.rows_per_lane;
@@ -1104,11 +1104,12 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
     // 1,100-6,000: 5.1 ms single, 7.5 ms grouped). Returns the first bin left to single CTAs; calls with few pairs are
     // left to `band_groups`.
     auto band_largest = [&](std::uint64_t pairs_here, dp_launch_shape_t const &shape, std::uint64_t strip_rows,
-                            std::size_t bytes_per_cta) -> int {
+                            std::size_t bytes_per_warp) -> int {
         int const key_begin = bin_band16_begin_k, key_end = key_begin + bin_dp_classes_k;
         if (schedule == szs_gb300_schedule_plain_k || shape.group_ctas_per_sm <= 0) return key_begin;
         std::uint64_t const slots = (std::uint64_t)context->sm_count * shape.group_ctas_per_sm;
-        if (pairs_here * 2 <= slots || bytes_per_cta * slots > band_largest_scratch_k) return key_begin;
+        if (pairs_here * 2 <= slots || bytes_per_warp * shape.warps_per_cta * slots > band_largest_scratch_k)
+            return key_begin;
         auto smallest = [&](int key) { return std::ldexp(1.0, 10 + bin_dp_classes_k - 1 - (key - key_begin)); };
         double total = 0, grouped = 0;
         for (int key = key_begin; key < key_end; ++key) total += 1.5 * smallest(key) * plan.count[key];
@@ -1124,12 +1125,12 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             double const strips = smallest(key) / (double)plan.max_cols / (double)strip_rows;
             std::uint64_t const size = std::min<std::uint64_t>(
                 {(std::uint64_t)(1.5 * smallest(key) / (band_largest_share_k * share)),
-                 (std::uint64_t)std::ceil(strips / band_warps_per_cta()), (std::uint64_t)band_group_max_ctas(), left});
+                 (std::uint64_t)std::ceil(strips / shape.warps_per_cta), (std::uint64_t)band_group_max_ctas(), left});
             if (size < least || grouped * 2 > total ||
                 smallest(key) < band_largest_mean_k * total / (double)pairs_here)
                 break;
             std::uint64_t const groups = std::min<std::uint64_t>(plan.count[key], left / size);
-            band_job(job_band16_k, key, key + 1, plan.count[key], (int)(groups * size), (int)size, shape, bytes_per_cta);
+            band_job(job_band16_k, key, key + 1, plan.count[key], (int)(groups * size), (int)size, shape, bytes_per_warp);
             jobs[job_count - 1].first = true;
             left -= groups * size;
         }
@@ -1143,9 +1144,8 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             if (shape.ctas_per_sm <= 0) return {sz_status_unknown_k, "16-bit band kernel cannot be resident"};
             // Local scores keep room for a 32-bit ring: a pair that reaches the 16-bit limit is scored again.
             std::size_t const ring_scale = engine.kind == kind_smith_waterman_k ? 2 : 1;
-            std::size_t const bytes_per_cta =
-                band16_words_per_slot * 4 * ring_scale * (std::size_t)band_warps_per_cta();
-            int const rest = band_largest(all_pairs, shape, 2u * 32u * (std::uint64_t)shape.rows_per_lane, bytes_per_cta);
+            std::size_t const bytes_per_warp = band16_words_per_slot * 4 * ring_scale;
+            int const rest = band_largest(all_pairs, shape, 2u * 32u * (std::uint64_t)shape.rows_per_lane, bytes_per_warp);
             int const end = bin_band16_begin_k + bin_dp_classes_k;
             std::uint64_t const pairs_here = pairs_in(rest, end);
             int ctas = 0, group_ctas = 1;
@@ -1162,7 +1162,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
                     band_groups(pairs_here, narrow, 2u * 32u * 4u, narrow_ctas, narrow_group);
                 if (narrow_group > group_ctas) shape = narrow, ctas = narrow_ctas, group_ctas = narrow_group;
             }
-            if (pairs_here) band_job(job_band16_k, rest, end, pairs_here, ctas, group_ctas, shape, bytes_per_cta);
+            if (pairs_here) band_job(job_band16_k, rest, end, pairs_here, ctas, group_ctas, shape, bytes_per_warp);
         }
     }
     {
@@ -1182,7 +1182,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
                 if (narrow_group > group_ctas) shape = narrow, ctas = narrow_ctas, group_ctas = narrow_group;
             }
             band_job(job_band_k, bin_band_begin_k, bin_band_begin_k + bin_dp_classes_k, pairs_here, ctas, group_ctas,
-                     shape, cells_per_warp * 4 * (std::size_t)band_warps_per_cta());
+                     shape, cells_per_warp * 4);
         }
     }
     for (int cell_bits : {64, 32}) {

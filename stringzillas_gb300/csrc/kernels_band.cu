@@ -2,7 +2,10 @@
  *  @file kernels_band.cu
  *  @brief Instantiations and launcher of the band kernel (dp_band.cuh). Compiled twice, with `SZS_BAND_ROWS` 8 (one
  *         CTA per pair, and groups for a few long pairs) or 4 (groups of CTAs per pair: strips of 128 rows, so a
- *         single long pair spreads over twice the warps, each step half as long).
+ *         single long pair spreads over twice the warps, each step half as long). The 4-row build has four warps per CTA
+ *         (`SZS_BAND_WARPS`), one per scheduler of an SM: its strips are bound by their own step latency, which a second
+ *         warp on the scheduler only adds to (NW, one pair of 30,000: 7.33 ms with eight, 7.16 with four, 7.27 with two;
+ *         16 of 10,000: 3.16, 2.80 and 2.83; SW, 4 of 8,000 on 16-bit cells: 1.79, 1.53 and 1.51).
  */
 #include "dp_band.cuh"
 #include "launchers.h"
@@ -157,7 +160,6 @@ cudaError_t launch_band_rows4(int kind, bool affine, int key_begin, int key_end,
                               std::size_t ring_cells_per_slot, int ctas, cudaStream_t stream, void *group_states,
                               int group_ctas, bool wide);
 
-int band_warps_per_cta() { return band_warps_k; }
 
 dp_launch_shape_t band_shape(int kind, bool affine, int classes, bool direct, bool wide, int rows_per_lane) {
     return rows_per_lane == 4 ? band_shape_rows4(kind, affine, classes, direct, wide)

@@ -155,10 +155,7 @@ cudaError_t launch_dp16_compare(bool affine, int rows, int key_begin, int key_en
  *  direct-table instance; `rows_per_lane` 8 (strips of 256 rows) or 4 (128 rows: for groups of CTAs per pair). */
 dp_launch_shape_t band_shape(int kind, bool affine, int classes, bool direct = false, bool wide = false,
                              int rows_per_lane = 8);
-/** Warps per band CTA (ring slots per CTA). */
-int band_warps_per_cta();
-
-/** Runs the band kernel over bins [key_begin, key_end). `scratch` holds `ctas * band_warps_per_cta()` ring slots of
+/** Runs the band kernel over bins [key_begin, key_end). `scratch` holds `ctas * warps_per_cta` ring slots of
  *  `ring_cells_per_slot` 32-bit cells. Bounded waits that give up set bit 0 of `bins->error_flags`. With
  *  `group_states` (one zeroed `band_group_state_bytes()` record per group) the grouped kernel runs instead: a
  *  cooperative launch of `ctas` CTAs in groups of `group_ctas`, each group sharing one pair at a time. */
@@ -177,7 +174,7 @@ int band_group_max_ctas();
 dp_launch_shape_t band16_shape(int kind, bool affine, int classes, int compare = 0, bool wide = false,
                                int rows_per_lane = 8);
 
-/** Runs the 16-bit band kernel over bins [key_begin, key_end). `scratch` holds `ctas * band_warps_per_cta()` ring
+/** Runs the 16-bit band kernel over bins [key_begin, key_end). `scratch` holds `ctas * warps_per_cta` ring
  *  slots of `ring_words_per_slot` 32-bit words (twice that for local scores, which may rescore a pair on 32-bit
  *  cells). Bounded waits that give up set bit 0 of `bins->error_flags`. */
 cudaError_t launch_band16(int kind, bool affine, int key_begin, int key_end, pair_task_t const *tasks,
