@@ -36,6 +36,7 @@ UNITS = [
     ("kernels_band16", "kernels_band16.cu", ["-DSZS_BAND16_ROWS=8"]),
     ("kernels_band16_4", "kernels_band16.cu", ["-DSZS_BAND16_ROWS=4", "-DSZS_BAND_WARPS=4"]),
     ("direct", "direct.cu", []),
+    ("small", "small.cu", []),
     ("kernels_short8", "kernels_short.cu", ["-DSZS_SHORT_ROWS=8"]),
     ("kernels_short12", "kernels_short.cu", ["-DSZS_SHORT_ROWS=12"]),
     ("kernels_short16", "kernels_short.cu", ["-DSZS_SHORT_ROWS=16"]),

@@ -23,6 +23,16 @@ cudaError_t launch_plan(plan_args_t const &args, plan_bins_t *bins, pair_task_t 
 cudaError_t launch_alphabet(tape_t const &queries, tape_t const &candidates, bool has_candidates,
                             batch_alphabet_t *alphabet, int sm_count, cudaStream_t stream,
                             std::uint64_t sample_bytes = 0);
+/** One pair of a small call: its strings' places in the packed bytes, the shorter one as rows (at most 1,024 bytes). */
+struct small_pair_t {
+    std::uint32_t rows, cols, rows_length, cols_length;
+};
+constexpr std::uint64_t small_max_pairs_k = 2048;      // pairs of a call packed and scored by one kernel
+constexpr std::uint64_t small_max_bytes_k = 1u << 20;  // bytes of their strings
+constexpr std::uint64_t small_max_rows_k = 1024;       // shorter sides: one word per lane
+/** Unit-cost Levenshtein of `count` packed pairs, one warp each, into `results` (device or page-locked host memory). */
+cudaError_t launch_myers_small(small_pair_t const *pairs, std::uint32_t count, std::uint8_t const *bytes,
+                               std::int64_t *results, cudaStream_t stream);
 constexpr std::uint64_t direct_max_rows_k = 1024; // longest pattern of the direct cross-product kernels
 /** Fewest cells of a cross product for the direct kernels with patterns of 513 to 1,024 rows: one thread per cell takes
  *  about 0.33 ms for a pair of 1,000 bytes however few there are, where the warp-per-pair kernel spreads few pairs over

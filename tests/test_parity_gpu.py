@@ -1252,3 +1252,31 @@ def test_utf8_transcoding_windows(szs, port, alphabet):
     np.testing.assert_array_equal(got, want)
     got = engine(szs.Strs(first[:60]), szs.Strs(second[:50])).astype(np.int64)
     np.testing.assert_array_equal(got, port.cross(costs, tape(first[:60]), tape(second[:50])))
+
+
+@pytest.mark.parametrize("longest", [1, 31, 32, 33, 255, 700, 1023, 1024, 1025])
+def test_small_host_calls(szs, port, longest):
+    """Few pairs from host memory take one packed copy and one kernel, a warp per pair (patterns of up to 1,024 bytes, one
+    more row sends the call to the planned routes): every edge of a word, empty strings on either side, texts longer than
+    their chunk of 32 bytes, every byte value, slices, 32- and 64-bit offsets, one pair, and 2,049 of them."""
+    rng = np.random.default_rng(longest)
+    letters = np.arange(256, dtype=np.uint8)
+    lengths = [(longest, longest), (0, longest), (longest, 0), (0, 0), (longest, 3 * longest + 5), (2 * longest, longest)]
+    lengths += [tuple(rng.integers(0, longest + 1, 2)) for _ in range(90)]
+    first = [bytes(rng.choice(letters if i % 2 else DNA, size=n)) for i, (n, _) in enumerate(lengths)]
+    second = [bytes(rng.choice(letters if i % 2 else DNA, size=m)) for i, (_, m) in enumerate(lengths)]
+    second += [a[: len(a) // 2] + b"x" + a[len(a) // 2:] for a in first[:8]]
+    first += first[:8]
+    engine = szs.LevenshteinDistances()
+    want = port.pairs(oracle.levenshtein_costs(), tape(first), tape(second))
+    for kind in (np.uint32, np.uint64):
+        def strs(items):
+            data, offsets = tape(items)
+            return szs.Strs.from_buffers(data.copy(), offsets.astype(kind))
+        np.testing.assert_array_equal(engine.pairwise(strs(first), strs(second)).astype(np.int64), want)
+        np.testing.assert_array_equal(engine.pairwise(strs(first)[5:50], strs(second)[5:50]).astype(np.int64), want[5:50])
+    np.testing.assert_array_equal(engine.pairwise(first[:1], second[:1]).astype(np.int64), want[:1])
+    if longest == 33:
+        many = (first * 22)[:2049], (second * 22)[:2049]
+        got = engine.pairwise(szs.Strs(many[0]), szs.Strs(many[1])).astype(np.int64)
+        np.testing.assert_array_equal(got, np.tile(want, 22)[:2049])
