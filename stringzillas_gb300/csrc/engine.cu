@@ -355,6 +355,7 @@ struct engine_t {
     score_costs_t costs {};
     int magnitude = 1;
     bool unit_levenshtein = false;
+    bool tilted = false;              // global affine costs that the 16x2 wavefront may tilt (`packed_tilt_fits`)
     bool packed_profile_fits = false; // every substitution cost (minus `open` for affine gaps) fits a signed byte
     szs_gb300_tuning_t tuning {};     // zeros: built-in choices
     int local_gain = -1;              // local scores with non-positive gaps: largest substitution gain (>= 0)
@@ -476,6 +477,25 @@ static bool packed_profile_fits(score_costs_t const &costs) {
                 (!fits(costs.profile_table[cc * 32 + row_class]) || !fits(costs.profile_table_t[cc * 32 + row_class])))
                 return false;
     return true;
+}
+
+/**
+ *  Whether the 16x2 wavefront may tilt an engine's tracks (dp_packed.cuh): values are kept minus `extend` per row and
+ *  column, costs minus twice `extend`, which have to fit the int8 profile as they are, and wherever the planner's bound
+ *  `(span + 4) * magnitude < 32767` holds the tilted values have to fit 16 bits too. Alignments (gaps <= 0): tilted
+ *  values lie between a few gap costs below 0 and `gain * min(n, m) - extend * (n + m)`, at most `(gain / 2 - extend) *
+ *  (n + m)`. Levenshtein (costs >= 0): between `-extend * (n + m)`, at least `-2 extend * max(n, m)`, and a few gap costs.
+ */
+static bool packed_tilt_fits(score_costs_t const &costs, int magnitude, int least_cost, int gain) {
+    if (!costs.affine || costs.kind == kind_smith_waterman_k) return false;
+    int const extend = costs.extend;
+    if (costs.kind == kind_levenshtein_k) {
+        int const low = std::min(costs.match, costs.mismatch) - 2 * extend;
+        int const high = std::max(costs.match, costs.mismatch) - 2 * extend;
+        return 2 * extend <= magnitude && low >= -128 && high <= 127;
+    }
+    return costs.open <= 0 && extend <= 0 && gain - 2 * extend <= 2 * magnitude && least_cost - 2 * extend >= -128 &&
+           gain - 2 * extend <= 127;
 }
 
 /* ---- inputs ----------------------------------------------------------------------------------------------------- */
@@ -1036,6 +1056,8 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             }
     }
 
+    bool const tilted = engine.tilted && compare_mode == compare_none_k;
+
     // The launch list, longest pairs first (64- and 32-bit wavefront, packed with the most rows per lane, then the
     // bit-parallel kernels by word count), so the routes' tails overlap each other instead of adding up.
     enum job_kind_t { job_dp_k, job_dp16_k, job_myers_k, job_band_k, job_band16_k, job_myers_warp_k, job_short_k,
@@ -1208,7 +1230,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         int const rows = 4 * (choice + 1);
         int const warps = engine.tuning.packed_warps[choice] ? (int)engine.tuning.packed_warps[choice] : 4;
         dp_launch_shape_t const shape =
-            dp16_shape(engine.kind, costs.affine != 0, rows, packed_costs.classes, warps, compare_mode, wide);
+            dp16_shape(engine.kind, costs.affine != 0, rows, packed_costs.classes, warps, compare_mode, wide, tilted);
         if (shape.ctas_per_sm <= 0) return {sz_status_unknown_k, "Packed wavefront kernel cannot be resident"};
         std::uint64_t const warps_needed = (pairs_here + 1) / 2;
         std::uint64_t const needed = (warps_needed + shape.warps_per_cta - 1) / shape.warps_per_cta;
@@ -1366,7 +1388,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         key_append(launch_key, cells_per_warp), key_append(launch_key, myers_planes), key_append(launch_key, wide);
         key_append(launch_key, near_list_at);
         key_append(launch_key, schedule), key_append(launch_key, lanes_used);
-        key_append(launch_key, engine.kind), key_append(launch_key, compare_mode);
+        key_append(launch_key, engine.kind), key_append(launch_key, compare_mode), key_append(launch_key, tilted);
     }
     auto issue_jobs = [&](cudaStream_t s) -> status_t {
         SZS_TRY_CUDA(cudaEventRecord(context->fork, s));
@@ -1405,7 +1427,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             else if (job.kind == job_dp16_k)
                 SZS_TRY_CUDA(launch_dp16(engine.kind, costs.affine != 0, job.variant, job.key_begin, job.key_end, tasks,
                                          bins, packed_costs, results, scratch, cells_per_warp, job.ctas, job.warps,
-                                         lane_stream, compare_mode, wide));
+                                         lane_stream, compare_mode, wide, tilted));
             else if (job.kind == job_myers_chain_k) {
                 // One cooperative launch per wave of pairs, one after another on this lane (they share the scratch).
                 for (std::uint64_t first = 0; first < job.pairs; first += chain_wave)
@@ -2109,6 +2131,11 @@ sz_status_t create_engine(int kind, int match, int mismatch, int open, int exten
     }
     engine->magnitude = std::max(magnitude, 1);
     engine->packed_profile_fits = packed_profile_fits(costs);
+    int least_cost = 0, gain = 0;
+    if (kind != kind_levenshtein_k)
+        for (int i = 0; i < 1024; ++i)
+            least_cost = std::min(least_cost, (int)table[i]), gain = std::max(gain, (int)table[i]);
+    engine->tilted = packed_tilt_fits(costs, engine->magnitude, least_cost, gain);
     if (kind == kind_smith_waterman_k && open <= 0 && extend <= 0) {
         // The bound of a local score: every used substitution cost, at most, per diagonal step.
         bool used[32] = {};
@@ -2144,16 +2171,17 @@ sz_status_t create_dense_engine(int kind, int open, int extend, std::int8_t cons
     costs.affine = open != extend;
     costs.classes = 1; // replaced per call by the batch's own codes
     int magnitude = std::max(cost_abs(open), cost_abs(extend));
-    int shift = costs.affine ? open : 0, gain = 0;
+    int shift = costs.affine ? open : 0, gain = 0, least_cost = 0;
     bool fits = true;
     for (int i = 0; i < 256 * 256; ++i) {
         int const cost = table[i];
         magnitude = std::max(magnitude, cost_abs(cost));
-        gain = std::max(gain, cost);
+        gain = std::max(gain, cost), least_cost = std::min(least_cost, cost);
         fits = fits && cost - shift >= -128 && cost - shift <= 127;
     }
     engine->magnitude = std::max(magnitude, 1);
     engine->packed_profile_fits = fits;
+    engine->tilted = packed_tilt_fits(costs, engine->magnitude, least_cost, gain);
     if (kind == kind_smith_waterman_k && open <= 0 && extend <= 0) {
         engine->local_gain = gain;
         costs.local_limit16 = 32767 - gain;

@@ -16,12 +16,12 @@ namespace {
 // 8 rows per lane (the planner's choice for longer pairs) take two columns per step. 4 rows (short pairs) keep one:
 // with two, the 31 steps by which lane 31 trails lane 0 would idle twice the columns of a short sweep (a cross
 // product of 100-byte strings ran 6 % slower). 12 and 16 rows have no registers to spare.
-template <int kind_, bool affine_, int rows_, int compare_, bool wide_>
-using dp16_instance_t = dp16_policy_t<kind_, affine_, rows_, compare_, wide_, rows_ == 8 ? 2 : 1>;
+template <int kind_, bool affine_, int rows_, int compare_, bool wide_, bool tilted_>
+using dp16_instance_t = dp16_policy_t<kind_, affine_, rows_, compare_, wide_, rows_ == 8 ? 2 : 1, tilted_>;
 
-template <int kind_, bool affine_, int rows_, int compare_, bool wide_>
+template <int kind_, bool affine_, int rows_, int compare_, bool wide_, bool tilted_>
 dp_launch_shape_t dp16_shape_rows(int classes, int warps) {
-    using policy_t = dp16_instance_t<kind_, affine_, rows_, compare_, wide_>;
+    using policy_t = dp16_instance_t<kind_, affine_, rows_, compare_, wide_, tilted_>;
     dp_launch_shape_t shape;
     shape.threads_per_cta = warps * 32;
     shape.warps_per_cta = warps;
@@ -37,22 +37,22 @@ dp_launch_shape_t dp16_shape_rows(int classes, int warps) {
     return shape;
 }
 
-template <int kind_, bool affine_, int compare_ = compare_none_k, bool wide_ = false>
+template <int kind_, bool affine_, int compare_ = compare_none_k, bool wide_ = false, bool tilted_ = false>
 dp_launch_shape_t dp16_shape_of(int rows, int classes, int warps) {
     switch (rows) {
-    case 4: return dp16_shape_rows<kind_, affine_, 4, compare_, wide_>(classes, warps);
-    case 8: return dp16_shape_rows<kind_, affine_, 8, compare_, wide_>(classes, warps);
-    case 12: return dp16_shape_rows<kind_, affine_, 12, compare_, wide_>(classes, warps);
-    case 16: return dp16_shape_rows<kind_, affine_, 16, compare_, wide_>(classes, warps);
+    case 4: return dp16_shape_rows<kind_, affine_, 4, compare_, wide_, tilted_>(classes, warps);
+    case 8: return dp16_shape_rows<kind_, affine_, 8, compare_, wide_, tilted_>(classes, warps);
+    case 12: return dp16_shape_rows<kind_, affine_, 12, compare_, wide_, tilted_>(classes, warps);
+    case 16: return dp16_shape_rows<kind_, affine_, 16, compare_, wide_, tilted_>(classes, warps);
     default: return dp_launch_shape_t {0, 0, 0, 0, 0};
     }
 }
 
-template <int kind_, bool affine_, int rows_, int compare_, bool wide_>
+template <int kind_, bool affine_, int rows_, int compare_, bool wide_, bool tilted_>
 cudaError_t dp16_launch_rows(int key_begin, int key_end, pair_task_t const *tasks, plan_bins_t *bins,
                              score_costs_t const &costs, std::int64_t *results, void *scratch,
                              std::size_t scratch_cells_per_warp, int ctas, int warps, cudaStream_t stream) {
-    using policy_t = dp16_instance_t<kind_, affine_, rows_, compare_, wide_>;
+    using policy_t = dp16_instance_t<kind_, affine_, rows_, compare_, wide_, tilted_>;
     int const shared = dp16_shared_bytes<policy_t>(warps, costs.classes);
     auto kernel = dp16_wavefront_kernel<policy_t>;
     cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
@@ -62,13 +62,14 @@ cudaError_t dp16_launch_rows(int key_begin, int key_end, pair_task_t const *task
     return cudaGetLastError();
 }
 
-template <int kind_, bool affine_, int compare_ = compare_none_k, bool wide_ = false>
+template <int kind_, bool affine_, int compare_ = compare_none_k, bool wide_ = false, bool tilted_ = false>
 cudaError_t dp16_launch_of(int rows, int key_begin, int key_end, pair_task_t const *tasks, plan_bins_t *bins,
                            score_costs_t const &costs, std::int64_t *results, void *scratch,
                            std::size_t scratch_cells_per_warp, int ctas, int warps, cudaStream_t stream) {
 #define SZS_DP16_ROWS(rows_)                                                                                         \
-    dp16_launch_rows<kind_, affine_, rows_, compare_, wide_>(key_begin, key_end, tasks, bins, costs, results, scratch, \
-                                                             scratch_cells_per_warp, ctas, warps, stream)
+    dp16_launch_rows<kind_, affine_, rows_, compare_, wide_, tilted_>(key_begin, key_end, tasks, bins, costs, results, \
+                                                                       scratch, scratch_cells_per_warp, ctas, warps,  \
+                                                                       stream)
     switch (rows) {
     case 4: return SZS_DP16_ROWS(4);
     case 8: return SZS_DP16_ROWS(8);
@@ -110,8 +111,15 @@ cudaError_t launch_dp16_compare(bool affine, int rows, int key_begin, int key_en
 
 #else
 
+// `tilted`: the four-operation form of global affine cells, for engines whose costs allow it.
 #define SZS_DP16_DISPATCH(call_, ...)                                                                                \
-    switch (kind * 2 + (affine ? 1 : 0)) {                                                                           \
+    if (tilted) {                                                                                                    \
+        if (kind == kind_levenshtein_k && affine)                                                                    \
+            return call_<kind_levenshtein_k, true, compare_none_k, false, true>(__VA_ARGS__);                        \
+        if (kind == kind_needleman_wunsch_k && affine)                                                               \
+            return call_<kind_needleman_wunsch_k, true, compare_none_k, false, true>(__VA_ARGS__);                   \
+    }                                                                                                                \
+    else switch (kind * 2 + (affine ? 1 : 0)) {                                                                      \
     case 0: return call_<kind_levenshtein_k, false>(__VA_ARGS__);                                                    \
     case 1: return call_<kind_levenshtein_k, true>(__VA_ARGS__);                                                     \
     case 2: return call_<kind_needleman_wunsch_k, false>(__VA_ARGS__);                                               \
@@ -121,7 +129,8 @@ cudaError_t launch_dp16_compare(bool affine, int rows, int key_begin, int key_en
     default: break;                                                                                                  \
     }
 
-dp_launch_shape_t dp16_shape(int kind, bool affine, int rows, int classes, int warps, int compare, bool wide) {
+dp_launch_shape_t dp16_shape(int kind, bool affine, int rows, int classes, int warps, int compare, bool wide,
+                             bool tilted) {
     if (warps < 1 || warps > 8) return dp_launch_shape_t {0, 0, 0, 0, 0};
     if (compare != compare_none_k || wide) {
         if (kind != kind_levenshtein_k || compare == compare_none_k) return dp_launch_shape_t {0, 0, 0, 0, 0};
@@ -134,7 +143,7 @@ dp_launch_shape_t dp16_shape(int kind, bool affine, int rows, int classes, int w
 cudaError_t launch_dp16(int kind, bool affine, int rows, int key_begin, int key_end, pair_task_t const *tasks,
                         plan_bins_t *bins, score_costs_t const &costs, std::int64_t *results, void *scratch,
                         std::size_t scratch_cells_per_warp, int ctas, int warps, cudaStream_t stream, int compare,
-                        bool wide) {
+                        bool wide, bool tilted) {
     if (warps < 1 || warps > 8) return cudaErrorInvalidValue;
     if (compare != compare_none_k || wide) {
         if (kind != kind_levenshtein_k || compare == compare_none_k) return cudaErrorInvalidValue;

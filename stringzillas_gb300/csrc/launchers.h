@@ -144,14 +144,14 @@ cudaError_t launch_dp(int kind, bool affine, int cell_bits, int key_begin, int k
  *  warps per CTA; ctas_per_sm = 0 if unsupported. `compare` (a `compare_mode_t`, dp_packed.cuh): the Levenshtein
  *  instances that compare codes instead of reading a profile (batches over more than 32 byte values). */
 dp_launch_shape_t dp16_shape(int kind, bool affine, int rows, int classes, int warps, int compare = 0,
-                             bool wide = false);
+                             bool wide = false, bool tilted = false);
 
 /** Runs the 16x2 packed wavefront kernel over bins [key_begin, key_end): two scheduled pairs per warp. `scratch`
  *  holds `ctas * warps_per_cta` rows of `scratch_cells_per_warp` 32-bit words. */
 cudaError_t launch_dp16(int kind, bool affine, int rows, int key_begin, int key_end, pair_task_t const *tasks,
                         plan_bins_t *bins, score_costs_t const &costs, std::int64_t *results, void *scratch,
                         std::size_t scratch_cells_per_warp, int ctas, int warps, cudaStream_t stream,
-                        int compare = 0, bool wide = false);
+                        int compare = 0, bool wide = false, bool tilted = false);
 
 /** The compare-mode halves of `dp16_shape` and `launch_dp16` (Levenshtein only; `wide`: strings of 16-bit codes),
  *  built in their own translation unit. */

@@ -1280,3 +1280,30 @@ def test_small_host_calls(szs, port, longest):
         many = (first * 22)[:2049], (second * 22)[:2049]
         got = engine.pairwise(szs.Strs(many[0]), szs.Strs(many[1])).astype(np.int64)
         np.testing.assert_array_equal(got, np.tile(want, 22)[:2049])
+
+
+@pytest.mark.parametrize("rows", [4, 8, 12, 16])
+@pytest.mark.parametrize("family,costs,gain", [("nw", (-6, -3), 6), ("nw", (-11, -1), 11), ("nw", (-4, -3), 5),
+                                               ("lev", (0, 4, 4, 2), 0), ("lev", (0, 2, 3, 1), 0), ("lev", (1, 3, 4, 3), 0)])
+def test_tilted_tracks_at_the_16bit_bound(szs, port, family, costs, gain, rows):
+    """Global affine costs that the 16x2 wavefront may tilt, at the edge of what may be tilted and past it (the third and
+    the last keep the plain form): identical, unrelated and very unequal strings up to the longest pairs that 16-bit cells
+    take, where the tilted values come within a few of 32,767 (or -32,768)."""
+    rng = np.random.default_rng(zlib_seed(family, costs, rows))
+    b2c, table = dna_tables()
+    table[1:5, 1:5] = -gain
+    np.fill_diagonal(table[1:5, 1:5], gain)
+    engine, oracle_costs = make_engine(szs, family, costs, b2c, table)
+    magnitude = max(abs(c) for c in costs + (gain,))
+    most = 32766 // magnitude - 4  # span of the longest pair on 16-bit cells: n + m, or max(n, m) for distances
+    longest = most // 2 if family == "nw" else min(most, 8000)
+    first, second = [], []
+    for n in (longest, longest - 1, longest, 129, 400, 700):
+        same = bytes(rng.choice(DNA, size=n))
+        first += [same, same, bytes(rng.choice(DNA, size=n)), b"A" * n, bytes(rng.choice(DNA, size=130))]
+        second += [same, same[: n // 2] + same[n // 2 + 3:], bytes(rng.choice(DNA, size=n)), b"C" * n,
+                   bytes(rng.choice(DNA, size=(most - 130 if family == "nw" else longest)))]
+    engine.set_tuning({"packed_rows": [rows] * 16, "band_min_rows_packed": 1 << 20, "band_min_rows": 1 << 20,
+                       "band_min_rows_few": 1 << 20, "short_max_rows": 1})
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    np.testing.assert_array_equal(got, port.pairs(oracle_costs, tape(first), tape(second)))
