@@ -362,8 +362,8 @@ class _Engine:
         values), ``cell_bits`` (16 values), ``band_min_rows``, ``packed_warps`` (4 values),
         ``band_min_rows_packed``, ``pipeline_chunk_kb``, ``packed_step_cost`` (4 values), ``band_min_rows_few``,
         ``band_min_rows_compare``, ``band_wait_polls`` (the band kernels' wait bound, clamped to the built-in
-        one) and ``short_max_rows`` (shorter sides up to this take the short-pair kernel; at most 128); None restores
-        the built-in choices."""
+        one) and ``short_max_rows`` (longer shorter sides never take the short-pair kernel; at most 448); None
+        restores the built-in choices."""
         err = ctypes.c_char_p()
         if tuning is None:
             status = lib.szs_gb300_engine_set_tuning(self.handle, None, ctypes.byref(err))

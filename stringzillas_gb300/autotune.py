@@ -113,9 +113,10 @@ def tune_family(szs, make_engine, family, rng, target_cells=4e9, log=print):
     from . import workloads as w
     alphabet = w.DNA if family.startswith("lev") else w.AMINO_ACIDS
     engine = make_engine()
-    # While the warp routes are measured, keep every measured class off the band.
+    # While the warp routes are measured, keep every measured class off the band, and off the short route where it is
+    # an alternative to them.
     table = {"packed_rows": [0] * 16, "cell_bits": [0] * 16, "band_min_rows": 1 << (max(CLASSES) + 1),
-             "packed_warps": [0] * 4, "band_min_rows_packed": 1 << (max(CLASSES) + 1)}
+             "packed_warps": [0] * 4, "band_min_rows_packed": 1 << (max(CLASSES) + 1), "short_max_rows": 128}
     measurements = {}
     rows_votes = {}
     batches, fits = {}, []
@@ -210,6 +211,7 @@ def tune_family(szs, make_engine, family, rng, target_cells=4e9, log=print):
         measurements[field] = {str(t): cells / (ms * 1e6) for t, ms in timings.items()}
         log(f"  {family:10s} {field} {best} " + " ".join(f"{t}={cells / (ms * 1e6):7.0f}"
                                                         for t, ms in timings.items()))
+    del table["short_max_rows"]
     return table, measurements
 
 

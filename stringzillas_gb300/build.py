@@ -40,6 +40,9 @@ UNITS = [
     ("kernels_short8", "kernels_short.cu", ["-DSZS_SHORT_ROWS=8"]),
     ("kernels_short12", "kernels_short.cu", ["-DSZS_SHORT_ROWS=12"]),
     ("kernels_short16", "kernels_short.cu", ["-DSZS_SHORT_ROWS=16"]),
+    ("kernels_short20", "kernels_short.cu", ["-DSZS_SHORT_ROWS=20"]),
+    ("kernels_short24", "kernels_short.cu", ["-DSZS_SHORT_ROWS=24"]),
+    ("kernels_short28", "kernels_short.cu", ["-DSZS_SHORT_ROWS=28"]),
     ("probe", "probe.cu", []),
     ("static_scratch", "static_scratch.cu", []),
     ("server", "server.cu", []),

@@ -1,6 +1,6 @@
 /**
  *  @file dp_short.cuh
- *  @brief Short pairs (shorter side at most 128): a warp cut into segments of 1 to 16 lanes, each segment scoring
+ *  @brief Short pairs (shorter side at most 448): a warp cut into segments of 1 to 16 lanes, each segment scoring
  *         two pairs at once on 16x2 packed cells, so a warp holds up to 64 pairs.
  *
  *  The 16x2 wavefront (dp_packed.cuh) gives a pair a whole warp: lane L owns rows L*R..L*R+R-1 of a strip of
@@ -24,6 +24,15 @@
  *  and the column codes from a register the segment's lanes load L columns at a time. A segment runs
  *  max(m_A, m_B) + L - 1 steps; the warp runs its slowest segment's steps, so the planner bins these pairs by the
  *  length of their longer side.
+ *
+ *  Bound: the ALU pipe (82 % busy), so what is left to save is rows past a pair's end, fill steps and operations. Large
+ *  batches therefore cut every octave of rows into quarters (a pair pads its rows by 9 % on average, by 17 % in halves),
+ *  with 16 to 28 rows per lane, and take pairs up to 448 rows from the whole-warp wavefront, whose strips of 128 to 512
+ *  rows and 31 fill steps of two columns cost a pair of 130-300 rows as much again as its cells: 65,536 pairs of text of
+ *  100-300 characters, affine distances, 1,030 -> 790 us per call (of 260-310: 1,730 -> 1,330); 1,048,576 DNA pairs of
+ *  16-128, affine local scores, 2,140 -> 2,000 us, part of it from the running maxima below. Batches that leave warp
+ *  slots free keep halves of octaves with at most 16 rows per lane: each shape is a launch, and a warp's own chain of
+ *  steps is their time (16,384 pairs of 16-128: 134 us, 166 in quarters; 206 in halves with 24 rows per lane).
  *
  *  Counterpart of the reference's register tier for short pairs (include/stringzillas/similarities/cuda.cuh:
  *  4837-5031, one thread per pair with 16-bit rows), and the same recurrences as its serial walkers
@@ -51,8 +60,11 @@ struct short_policy_t {
     static constexpr int segments_k = warp_size_k / lanes_;
     static constexpr bool compare_k = compare_ != compare_none_k;
     static constexpr bool multiply_k = compare_ == compare_multiply_k;
+    // Four warps per scheduler in 128 registers; three tracks of 24 or 28 rows (H, E and the codes) take 168 instead.
+    static constexpr int ctas_per_sm_k = compare_k && affine_ && rows_per_lane_ >= 24 ? 3 : 4;
     static_assert(lanes_ == 1 || lanes_ == 2 || lanes_ == 4 || lanes_ == 8 || lanes_ == 16, "segments of 1 to 16 lanes");
     static_assert(rows_per_lane_ % 4 == 0, "profile rows are read in 4-byte words");
+    static_assert(segment_rows_k <= short_max_rows_k, "a pair's whole column fits one strip");
     static_assert(!compare_k || kind_ == kind_levenshtein_k, "only Levenshtein costs are a function of equality");
 };
 
@@ -62,10 +74,14 @@ __host__ __device__ constexpr int short_profile_bytes_per_warp(int classes) {
     return policy_::compare_k ? 0 : policy_::segments_k * 2 * classes * policy_::segment_rows_k;
 }
 
+/** Row classes of one orientation of the row-class-major table: the engine's 32 and the filler row. */
+constexpr int short_row_classes_k = 33;
+constexpr int short_filler_class_k = 32;
+
 /** Costs, both orientations of the row-class-major table (`row_costs`), then the warps' profiles. */
 template <typename policy_>
 __host__ __device__ constexpr int short_shared_bytes(int warps_per_cta, int classes) {
-    return int((sizeof(score_costs_t) + 15) / 16 * 16) + 2 * 32 * 32 +
+    return int((sizeof(score_costs_t) + 15) / 16 * 16) + 2 * short_row_classes_k * 32 +
            warps_per_cta * short_profile_bytes_per_warp<policy_>(classes);
 }
 
@@ -163,20 +179,30 @@ __device__ __forceinline__ void short_score_segment(pair_task_t const &a, bool a
         std::uint32_t const class_mask = compare ? 0xFFu : 31u;
         class_a[r] = costs.byte_to_class[i <= (std::int64_t)n_a ? a.rows[i - 1] : 0u] & class_mask;
         class_b[r] = costs.byte_to_class[i <= (std::int64_t)n_b ? b.rows[i - 1] : 0u] & class_mask;
+        if (local && i > (std::int64_t)n_a) class_a[r] = short_filler_class_k;
+        if (local && i > (std::int64_t)n_b) class_b[r] = short_filler_class_k;
         if constexpr (compare) row_codes[r] = class_a[r] | (class_b[r] << 16);
     }
     if constexpr (!compare) {
-        short_write_profile<R, S>(row_costs + (a.transposed ? 1024 : 0), class_a, classes, profile_a, segment_lane * R);
-        short_write_profile<R, S>(row_costs + (b.transposed ? 1024 : 0), class_b, classes, profile_b, segment_lane * R);
+        constexpr int orientation = short_row_classes_k * 32;
+        short_write_profile<R, S>(row_costs + (a.transposed ? orientation : 0), class_a, classes, profile_a,
+                                  segment_lane * R);
+        short_write_profile<R, S>(row_costs + (b.transposed ? orientation : 0), class_b, classes, profile_b,
+                                  segment_lane * R);
     }
-    std::uint32_t h_col[R], e_col[R], best_row[R];
+    std::uint32_t h_col[R], e_col[R];
+    // Local scores: running maxima over every cell, filler rows included. A filler row (past its pair's last) costs
+    // -128 against every column: its cells take their values from gaps out of the rows above and from diagonals that
+    // lose `-open` at least, never above the cells they come from, as long as gap costs are not positive (the planner
+    // keeps local calls with positive ones off this kernel). So no row needs a maximum of its own: one three-way
+    // maximum takes two cells.
+    std::uint32_t best[2] = {0u, 0u};
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         std::int32_t const h = edge.score(row0 + r) + h_shift;
         h_col[r] = pack16(h, h);
         std::int32_t const e = gap_seed(row0 + r);
         e_col[r] = pack16(e, e);
-        best_row[r] = 0;
     }
     std::int32_t const diag_seed = edge.score(row0 - 1) + h_shift;
     std::uint32_t diag_up = pack16(diag_seed, diag_seed);
@@ -279,7 +305,8 @@ __device__ __forceinline__ void short_score_segment(pair_task_t const &a, bool a
             if constexpr (local) {
                 if constexpr (steady) {
 #pragma unroll
-                    for (int r = 0; r < R; ++r) best_row[r] = __vimax3_s16x2(best_row[r], cell_h[r], 0u);
+                    for (int r = 0; r < R; r += 2)
+                        best[r / 2 % 2] = __vimax3_s16x2(best[r / 2 % 2], cell_h[r], cell_h[r + 1]);
                 }
                 else {
                     // Columns past one pair's end carry filler in that half: masked out of the maxima (H >= 0).
@@ -287,19 +314,20 @@ __device__ __forceinline__ void short_score_segment(pair_task_t const &a, bool a
                                                                : ((j <= (int)m_a ? 0x0000FFFFu : 0u) |
                                                                   (j <= (int)m_b ? 0xFFFF0000u : 0u));
 #pragma unroll
-                    for (int r = 0; r < R; ++r) best_row[r] = __vimax3_s16x2(best_row[r], cell_h[r] & mask, 0u);
+                    for (int r = 0; r < R; r += 2)
+                        best[r / 2 % 2] = __vimax3_s16x2(best[r / 2 % 2], cell_h[r] & mask, cell_h[r + 1] & mask);
                 }
             }
             else if constexpr (!steady) {
                 if (segment_lane == a_lane && j == (int)m_a) {
 #pragma unroll
                     for (int r = 0; r < R; ++r)
-                        if (r == a_row) result_a = low16(cell_h[r]);
+                        if (r == a_row) result_a = low16(h_col[r]) - h_shift;
                 }
                 if (segment_lane == b_lane && j == (int)m_b) {
 #pragma unroll
                     for (int r = 0; r < R; ++r)
-                        if (r == b_row) result_b = high16(cell_h[r]);
+                        if (r == b_row) result_b = high16(h_col[r]) - h_shift;
                 }
             }
             out_h = h_up, out_f = f_up;
@@ -316,13 +344,7 @@ __device__ __forceinline__ void short_score_segment(pair_task_t const &a, bool a
     for (; t < warp_steps; ++t) step(t, std::false_type {});
 
     if constexpr (local) {
-        std::uint32_t lane_best = 0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            std::uint32_t const keep = ((row0 + r <= (std::int64_t)n_a) ? 0x0000FFFFu : 0u) |
-                                       ((row0 + r <= (std::int64_t)n_b) ? 0xFFFF0000u : 0u);
-            lane_best = __vimax3_s16x2(lane_best, best_row[r] & keep, 0u);
-        }
+        std::uint32_t lane_best = __vimax3_s16x2(best[0], best[1], 0u);
 #pragma unroll
         for (int offset = L / 2; offset > 0; offset >>= 1)
             lane_best = __vimax3_s16x2(lane_best, __shfl_xor_sync(0xFFFFFFFFu, lane_best, offset), 0u);
@@ -339,7 +361,7 @@ __device__ __forceinline__ void short_score_segment(pair_task_t const &a, bool a
 /** Persistent kernel over the short bins [key_begin, key_end): each warp takes 2 x (32 / L) consecutive scheduled
  *  pairs at a time, two per segment. */
 template <typename policy_>
-__global__ void __launch_bounds__(256) dp16_short_kernel(pair_task_t const *__restrict__ tasks,
+__global__ void __launch_bounds__(128, policy_::ctas_per_sm_k) dp16_short_kernel(pair_task_t const *__restrict__ tasks,
                                                          plan_bins_t *__restrict__ bins, int key_begin, int key_end,
                                                          score_costs_t const costs,
                                                          std::int64_t *__restrict__ results) {
@@ -347,18 +369,20 @@ __global__ void __launch_bounds__(256) dp16_short_kernel(pair_task_t const *__re
     extern __shared__ __align__(16) unsigned char shared_bytes[];
     score_costs_t &costs_s = *reinterpret_cast<score_costs_t *>(shared_bytes);
     std::uint8_t *row_costs = shared_bytes + ((sizeof(score_costs_t) + 15) / 16) * 16;
-    std::int8_t *profiles = reinterpret_cast<std::int8_t *>(row_costs + 2 * 32 * 32);
+    std::int8_t *profiles = reinterpret_cast<std::int8_t *>(row_costs + 2 * short_row_classes_k * 32);
     {
         auto const *src = reinterpret_cast<std::uint32_t const *>(&costs);
         auto *dst = reinterpret_cast<std::uint32_t *>(&costs_s);
         for (unsigned i = threadIdx.x; i < sizeof(score_costs_t) / 4; i += blockDim.x) dst[i] = src[i];
         // Row-class-major copies of both orientations: row_costs[o][row class][column class] = table - shift (the
-        // affine tracks' s - open, which the planner checked fits a byte).
+        // affine tracks' s - open, which the planner checked fits a byte); the filler row after each.
         std::int32_t const shift = policy_::affine_k ? costs.open : 0;
-        for (unsigned i = threadIdx.x; i < 2 * 32 * 32; i += blockDim.x) {
-            unsigned const o = i >> 10, row = (i >> 5) & 31u, column = i & 31u;
+        for (unsigned i = threadIdx.x; i < 2 * short_row_classes_k * 32; i += blockDim.x) {
+            unsigned const o = i / (short_row_classes_k * 32), row = i / 32 % short_row_classes_k, column = i & 31u;
             std::int8_t const *table = o ? costs.profile_table_t : costs.profile_table;
-            row_costs[i] = (std::uint8_t)(std::int8_t)(table[column * 32 + row] - shift);
+            row_costs[i] = row == short_filler_class_k
+                               ? std::uint8_t(0x80)
+                               : (std::uint8_t)(std::int8_t)(table[column * 32 + row] - shift);
         }
     }
     __syncthreads();

@@ -215,7 +215,7 @@ struct device_context_t {
     pinned_buffer_t results_host;
     cudaEvent_t start = nullptr, stop = nullptr;
     cudaEvent_t compute_start = nullptr, compute_stop = nullptr;
-    static constexpr int lanes_k = 8; // auxiliary streams the routes of one call run on concurrently
+    static constexpr int lanes_k = 16; // auxiliary streams the routes of one call run on concurrently
     cudaStream_t lanes[lanes_k] = {nullptr};
     cudaEvent_t fork = nullptr;
     cudaEvent_t joins[lanes_k] = {nullptr};
@@ -864,6 +864,10 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
     args.short_max_rows = engine.tuning.short_max_rows
                               ? std::min<std::uint32_t>(engine.tuning.short_max_rows, (std::uint32_t)short_max_rows_k)
                               : (std::uint32_t)short_max_rows_k;
+    // The short kernel's running maxima count on gaps that cost something (dp_short.cuh).
+    if (engine.kind == kind_smith_waterman_k && engine.local_gain < 0) args.short_max_rows = 0;
+    args.short_fine = args.pairs >= short_fine_pairs_k && args.packed_allowed && !args.unit_levenshtein ? 1 : 0;
+    args.classes = costs.classes;
     // A batched call with fewer pairs than one wave of the 16x2 route (two pairs per warp, about 16 resident warps
     // per SM) would leave SMs idle on the wavefront: its longer pairs spread over a band CTA's warps instead.
     if (schedule != szs_gb300_schedule_plain_k && args.pairs < 32ull * (std::uint64_t)context->sm_count) {
@@ -1071,7 +1075,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         int ctas;
         std::size_t scratch_offset, scratch_bytes;
         int group_ctas = 1;            // band jobs: CTAs sharing one pair (1 = one CTA per pair)
-        int rows = 8;                  // band jobs: rows per lane (4 for groups of CTAs per pair)
+        int rows = 8;                  // rows per lane of band jobs (4 for groups of CTAs per pair) and short-pair jobs
         std::size_t state_offset = 0;  // grouped band jobs: the groups' state records in the scratch buffer
         std::size_t state_bytes = 0;
         bool fills = true;             // the grid takes every resident CTA slot of its kernel on the device
@@ -1241,22 +1245,23 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         scratch_total += bytes;
     }
     // Short pairs: one job per segment shape, most rows first.
-    for (int shape_index : {3, 6, 2, 5, 1, 4, 0}) {
+    for (int shape_index = short_shapes_k - 1; shape_index >= 0; --shape_index) {
         int const key_begin = bin_short_begin_k + shape_index * short_m_classes_k;
         int const key_end = key_begin + short_m_classes_k;
         std::uint64_t const pairs_here = pairs_in(key_begin, key_end);
         if (!pairs_here) continue;
         int const warps = 4;
+        int const rows = short_rows_for(packed_costs.classes, compare_mode, shape_index, pairs_here, context->sm_count);
         dp_launch_shape_t const shape =
-            short_shape(engine.kind, costs.affine != 0, shape_index, packed_costs.classes, warps, compare_mode);
+            short_shape(engine.kind, costs.affine != 0, shape_index, rows, packed_costs.classes, warps, compare_mode);
         if (shape.ctas_per_sm <= 0) return {sz_status_unknown_k, "Short-pair kernel cannot be resident"};
-        int const rows = short_rows_for(packed_costs.classes, compare_mode, shape_index);
         std::uint64_t const lanes = (std::uint64_t)(short_segment_rows(shape_index) / rows);
         std::uint64_t const per_warp = 2u * (32u / lanes); // pairs per warp
         std::uint64_t const warps_needed = (pairs_here + per_warp - 1) / per_warp;
         std::uint64_t const needed = (warps_needed + warps - 1) / warps;
         int const ctas = (int)std::min<std::uint64_t>(needed, (std::uint64_t)context->sm_count * shape.ctas_per_sm);
         jobs[job_count++] = {job_short_k, shape_index, warps, key_begin, key_end, pairs_here, ctas, 0, 0};
+        jobs[job_count - 1].rows = rows;
         jobs[job_count - 1].fills = needed >= (std::uint64_t)context->sm_count * shape.ctas_per_sm;
     }
     int myers_planes = 0;
@@ -1438,9 +1443,9 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
                                                     costs.wait_polls, lane_stream));
             }
             else if (job.kind == job_short_k)
-                SZS_TRY_CUDA(launch_short(engine.kind, costs.affine != 0, job.variant, job.key_begin, job.key_end,
-                                          tasks, bins, packed_costs, results, job.ctas, job.warps, lane_stream,
-                                          compare_mode));
+                SZS_TRY_CUDA(launch_short(engine.kind, costs.affine != 0, job.variant, job.rows, job.key_begin,
+                                          job.key_end, tasks, bins, packed_costs, results, job.ctas, job.warps,
+                                          lane_stream, compare_mode));
             else if (job.kind == job_near_k) {
                 SZS_TRY_CUDA(launch_myers_near(job.variant, myers_planes, tasks, bins, job.key_begin, job.key_end, alphabet,
                                                results, near_list, job.ctas, lane_stream));

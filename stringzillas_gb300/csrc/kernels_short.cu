@@ -1,19 +1,19 @@
 /**
  *  @file kernels_short.cu
  *  @brief Instantiations and launcher of the segmented 16x2 kernel for short pairs (dp_short.cuh) for every cost
- *         family, profile and compare modes. Segment shapes 0-3 for shorter sides up to 16, 32, 64 and 128:
- *         either 2, 4, 8, 16 lanes x 8 rows (profiles over many classes: a warp's profiles stay at 32 x 8 rows per
- *         pair) or 1, 2, 4, 8 lanes x 16 rows (few classes or compare mode: fewer lanes and steps per pair); shapes
- *         4-6 for shorter sides up to 24, 48 and 96: 2, 4, 8 lanes x 12 rows, so that a pair pads its rows to at
- *         most 1.5x instead of 2x and the middle of each octave runs fewer fill steps.
+ *         family, profile and compare modes. Segment shape 0 holds 16 rows; the octave above 16 << k has four shapes,
+ *         1 + 4 k + q, of 5/4, 6/4, 7/4 and 8/4 times its start. With few classes or in compare mode they are 2^k lanes
+ *         x 20, 24 and 28 rows and 2^(k + 1) lanes x 16 rows; profiles over many classes, whose segments together stay
+ *         near 32 x 8 rows per pair and warp in shared memory, have the 6/4 and 8/4 shapes with 2^(k + 1) lanes x 12
+ *         and 2^(k + 2) lanes x 8 rows.
  *
- *  Compiled three times, with `SZS_SHORT_ROWS` 8, 12 or 16, so the families build in parallel.
+ *  Compiled six times, with `SZS_SHORT_ROWS` 8, 12, 16, 20, 24 or 28, so the families build in parallel.
  */
 #include "dp_short.cuh"
 #include "launchers.h"
 
 #ifndef SZS_SHORT_ROWS
-#error "compile with -DSZS_SHORT_ROWS=<8|12|16>"
+#error "compile with -DSZS_SHORT_ROWS=<8|12|16|20|24|28>"
 #endif
 
 namespace szs_gb300 {
@@ -51,45 +51,48 @@ cudaError_t short_launch_of(int key_begin, int key_end, pair_task_t const *tasks
     return cudaGetLastError();
 }
 
-#if SZS_SHORT_ROWS == 12
-// Segment shapes of this family: 4, 5, 6 for shorter sides up to 24, 48, 96 (2, 4, 8 lanes x 12 rows).
-#define SZS_SHORT_SHAPES(call_, kind_, affine_, compare_, ...)                                                       \
-    switch (shape) {                                                                                                 \
-    case 4: return call_<kind_, affine_, 2, 12, compare_>(__VA_ARGS__);                                              \
-    case 5: return call_<kind_, affine_, 4, 12, compare_>(__VA_ARGS__);                                              \
-    case 6: return call_<kind_, affine_, 8, 12, compare_>(__VA_ARGS__);                                              \
-    default: break;                                                                                                  \
-    }
+// Lanes per segment: 1 to 16, but not one lane of 8 or 12 rows.
+#if SZS_SHORT_ROWS < 16
+#define SZS_SHORT_LANES_1(call_, kind_, affine_, compare_, ...)
 #else
-// Segment shapes of this family: 0, 1, 2, 3 for shorter sides up to 16, 32, 64, 128 (lanes x rows).
-#define SZS_SHORT_SHAPES(call_, kind_, affine_, compare_, ...)                                                       \
-    switch (shape) {                                                                                                 \
-    case 0: return call_<kind_, affine_, 16 / SZS_SHORT_ROWS, SZS_SHORT_ROWS, compare_>(__VA_ARGS__);                \
-    case 1: return call_<kind_, affine_, 32 / SZS_SHORT_ROWS, SZS_SHORT_ROWS, compare_>(__VA_ARGS__);                \
-    case 2: return call_<kind_, affine_, 64 / SZS_SHORT_ROWS, SZS_SHORT_ROWS, compare_>(__VA_ARGS__);                \
-    case 3: return call_<kind_, affine_, 128 / SZS_SHORT_ROWS, SZS_SHORT_ROWS, compare_>(__VA_ARGS__);               \
+#define SZS_SHORT_LANES_1(call_, kind_, affine_, compare_, ...)                                                      \
+    case 1: return call_<kind_, affine_, 1, SZS_SHORT_ROWS, compare_>(__VA_ARGS__);
+#endif
+#define SZS_SHORT_LANES(call_, kind_, affine_, compare_, ...)                                                        \
+    switch (lanes) {                                                                                                 \
+    SZS_SHORT_LANES_1(call_, kind_, affine_, compare_, __VA_ARGS__)                                                  \
+    case 2: return call_<kind_, affine_, 2, SZS_SHORT_ROWS, compare_>(__VA_ARGS__);                                  \
+    case 4: return call_<kind_, affine_, 4, SZS_SHORT_ROWS, compare_>(__VA_ARGS__);                                  \
+    case 8: return call_<kind_, affine_, 8, SZS_SHORT_ROWS, compare_>(__VA_ARGS__);                                  \
+    case 16: return call_<kind_, affine_, 16, SZS_SHORT_ROWS, compare_>(__VA_ARGS__);                                \
     default: break;                                                                                                  \
     }
+
+#if SZS_SHORT_ROWS == 8
+#define SZS_SHORT_COMPARE(call_, ...) break; // profiles over many classes only
+#else
+#define SZS_SHORT_COMPARE(call_, ...)                                                                                \
+    if (kind != kind_levenshtein_k) break;                                                                           \
+    switch ((affine ? 2 : 0) + (compare == compare_multiply_k ? 1 : 0)) {                                            \
+    case 0: SZS_SHORT_LANES(call_, kind_levenshtein_k, false, compare_select_k, __VA_ARGS__) break;                  \
+    case 1: SZS_SHORT_LANES(call_, kind_levenshtein_k, false, compare_multiply_k, __VA_ARGS__) break;                \
+    case 2: SZS_SHORT_LANES(call_, kind_levenshtein_k, true, compare_select_k, __VA_ARGS__) break;                   \
+    default: SZS_SHORT_LANES(call_, kind_levenshtein_k, true, compare_multiply_k, __VA_ARGS__) break;                \
+    }                                                                                                                \
+    break;
 #endif
 
 #define SZS_SHORT_DISPATCH(call_, ...)                                                                               \
     if (compare != compare_none_k) {                                                                                 \
-        if (kind != kind_levenshtein_k) break;                                                                       \
-        switch ((affine ? 2 : 0) + (compare == compare_multiply_k ? 1 : 0)) {                                        \
-        case 0: SZS_SHORT_SHAPES(call_, kind_levenshtein_k, false, compare_select_k, __VA_ARGS__) break;             \
-        case 1: SZS_SHORT_SHAPES(call_, kind_levenshtein_k, false, compare_multiply_k, __VA_ARGS__) break;           \
-        case 2: SZS_SHORT_SHAPES(call_, kind_levenshtein_k, true, compare_select_k, __VA_ARGS__) break;              \
-        default: SZS_SHORT_SHAPES(call_, kind_levenshtein_k, true, compare_multiply_k, __VA_ARGS__) break;           \
-        }                                                                                                            \
-        break;                                                                                                       \
+        SZS_SHORT_COMPARE(call_, __VA_ARGS__)                                                                        \
     }                                                                                                                \
     switch (kind * 2 + (affine ? 1 : 0)) {                                                                           \
-    case 0: SZS_SHORT_SHAPES(call_, kind_levenshtein_k, false, compare_none_k, __VA_ARGS__) break;                   \
-    case 1: SZS_SHORT_SHAPES(call_, kind_levenshtein_k, true, compare_none_k, __VA_ARGS__) break;                    \
-    case 2: SZS_SHORT_SHAPES(call_, kind_needleman_wunsch_k, false, compare_none_k, __VA_ARGS__) break;              \
-    case 3: SZS_SHORT_SHAPES(call_, kind_needleman_wunsch_k, true, compare_none_k, __VA_ARGS__) break;               \
-    case 4: SZS_SHORT_SHAPES(call_, kind_smith_waterman_k, false, compare_none_k, __VA_ARGS__) break;                \
-    case 5: SZS_SHORT_SHAPES(call_, kind_smith_waterman_k, true, compare_none_k, __VA_ARGS__) break;                 \
+    case 0: SZS_SHORT_LANES(call_, kind_levenshtein_k, false, compare_none_k, __VA_ARGS__) break;                    \
+    case 1: SZS_SHORT_LANES(call_, kind_levenshtein_k, true, compare_none_k, __VA_ARGS__) break;                     \
+    case 2: SZS_SHORT_LANES(call_, kind_needleman_wunsch_k, false, compare_none_k, __VA_ARGS__) break;               \
+    case 3: SZS_SHORT_LANES(call_, kind_needleman_wunsch_k, true, compare_none_k, __VA_ARGS__) break;                \
+    case 4: SZS_SHORT_LANES(call_, kind_smith_waterman_k, false, compare_none_k, __VA_ARGS__) break;                 \
+    case 5: SZS_SHORT_LANES(call_, kind_smith_waterman_k, true, compare_none_k, __VA_ARGS__) break;                  \
     default: break;                                                                                                  \
     }
 
@@ -98,19 +101,19 @@ cudaError_t short_launch_of(int key_begin, int key_end, pair_task_t const *tasks
 #define SZS_CONCAT_(a, b) a##b
 #define SZS_CONCAT(a, b) SZS_CONCAT_(a, b)
 
-dp_launch_shape_t SZS_CONCAT(short_shape_rows, SZS_SHORT_ROWS)(int kind, bool affine, int shape, int classes,
+dp_launch_shape_t SZS_CONCAT(short_shape_rows, SZS_SHORT_ROWS)(int kind, bool affine, int lanes, int classes,
                                                                int warps, int compare) {
-    if (warps >= 1 && warps <= 8) do {
+    if (warps >= 1 && warps <= 4) do {
             SZS_SHORT_DISPATCH(short_shape_of, classes, warps)
         } while (false);
     return dp_launch_shape_t {0, 0, 0, 0, 0};
 }
 
-cudaError_t SZS_CONCAT(launch_short_rows, SZS_SHORT_ROWS)(int kind, bool affine, int shape, int key_begin,
+cudaError_t SZS_CONCAT(launch_short_rows, SZS_SHORT_ROWS)(int kind, bool affine, int lanes, int key_begin,
                                                            int key_end, pair_task_t const *tasks, plan_bins_t *bins,
                                                            score_costs_t const &costs, std::int64_t *results,
                                                            int ctas, int warps, cudaStream_t stream, int compare) {
-    if (warps >= 1 && warps <= 8) do {
+    if (warps >= 1 && warps <= 4) do {
             SZS_SHORT_DISPATCH(short_launch_of, key_begin, key_end, tasks, bins, costs, results, ctas, warps, stream)
         } while (false);
     return cudaErrorInvalidValue;
@@ -118,47 +121,53 @@ cudaError_t SZS_CONCAT(launch_short_rows, SZS_SHORT_ROWS)(int kind, bool affine,
 
 #if SZS_SHORT_ROWS == 16
 
-dp_launch_shape_t short_shape_rows8(int kind, bool affine, int shape, int classes, int warps, int compare);
-cudaError_t launch_short_rows8(int kind, bool affine, int shape, int key_begin, int key_end, pair_task_t const *tasks,
-                               plan_bins_t *bins, score_costs_t const &costs, std::int64_t *results, int ctas,
-                               int warps, cudaStream_t stream, int compare);
-dp_launch_shape_t short_shape_rows12(int kind, bool affine, int shape, int classes, int warps, int compare);
-cudaError_t launch_short_rows12(int kind, bool affine, int shape, int key_begin, int key_end, pair_task_t const *tasks,
-                                plan_bins_t *bins, score_costs_t const &costs, std::int64_t *results, int ctas,
-                                int warps, cudaStream_t stream, int compare);
+#define SZS_SHORT_DECLARE(rows_)                                                                                     \
+    dp_launch_shape_t short_shape_rows##rows_(int kind, bool affine, int lanes, int classes, int warps, int compare); \
+    cudaError_t launch_short_rows##rows_(int kind, bool affine, int lanes, int key_begin, int key_end,               \
+                                         pair_task_t const *tasks, plan_bins_t *bins, score_costs_t const &costs,    \
+                                         std::int64_t *results, int ctas, int warps, cudaStream_t stream,            \
+                                         int compare);
+SZS_SHORT_DECLARE(8)
+SZS_SHORT_DECLARE(12)
+SZS_SHORT_DECLARE(20)
+SZS_SHORT_DECLARE(24)
+SZS_SHORT_DECLARE(28)
 
-int short_rows_for(int classes, int compare, int shape) {
-    if (shape >= 4) return 12;
-    return compare != compare_none_k || classes <= 8 ? 16 : 8;
+int short_rows_for(int classes, int compare, int shape, std::uint64_t pairs, int sm_count) {
+    bool const few = compare != compare_none_k || classes <= short_few_classes_k;
+    int const quarter = shape == 0 ? 3 : (shape - 1) % 4;
+    if (quarter == 3) return few ? 16 : 8;
+    if (!few) return 12;
+    // The 6/4 shapes up to 16 lanes have a second form of half the rows in twice the lanes, whose steps are half as
+    // long: where the pairs leave warp slots free, a warp's own chain of steps is what takes the time.
+    int const lanes = short_segment_rows(shape) / 24;
+    std::uint64_t const warps = pairs / (64u / lanes);
+    return quarter == 1 && lanes <= 8 && warps < 64u * (std::uint64_t)sm_count ? 12 : 20 + 4 * quarter;
 }
 
-int short_segment_rows(int shape) {
-    constexpr int rows[short_shapes_k] = {16, 32, 64, 128, 24, 48, 96};
-    return shape >= 0 && shape < short_shapes_k ? rows[shape] : 0;
-}
-
-dp_launch_shape_t short_shape(int kind, bool affine, int shape, int classes, int warps, int compare) {
-    switch (short_rows_for(classes, compare, shape)) {
-    case 12: return short_shape_rows12(kind, affine, shape, classes, warps, compare);
-    case 16: return short_shape_rows16(kind, affine, shape, classes, warps, compare);
-    default: return short_shape_rows8(kind, affine, shape, classes, warps, compare);
+dp_launch_shape_t short_shape(int kind, bool affine, int shape, int rows, int classes, int warps, int compare) {
+    int const lanes = short_segment_rows(shape) / rows;
+    switch (rows) {
+    case 8: return short_shape_rows8(kind, affine, lanes, classes, warps, compare);
+    case 12: return short_shape_rows12(kind, affine, lanes, classes, warps, compare);
+    case 16: return short_shape_rows16(kind, affine, lanes, classes, warps, compare);
+    case 20: return short_shape_rows20(kind, affine, lanes, classes, warps, compare);
+    case 24: return short_shape_rows24(kind, affine, lanes, classes, warps, compare);
+    default: return short_shape_rows28(kind, affine, lanes, classes, warps, compare);
     }
 }
 
-cudaError_t launch_short(int kind, bool affine, int shape, int key_begin, int key_end, pair_task_t const *tasks,
-                         plan_bins_t *bins, score_costs_t const &costs, std::int64_t *results, int ctas, int warps,
-                         cudaStream_t stream, int compare) {
-    switch (short_rows_for(costs.classes, compare, shape)) {
-    case 12:
-        return launch_short_rows12(kind, affine, shape, key_begin, key_end, tasks, bins, costs, results, ctas, warps,
-                                   stream, compare);
-    case 16:
-        return launch_short_rows16(kind, affine, shape, key_begin, key_end, tasks, bins, costs, results, ctas, warps,
-                                   stream, compare);
-    default:
-        return launch_short_rows8(kind, affine, shape, key_begin, key_end, tasks, bins, costs, results, ctas, warps,
-                                  stream, compare);
-    }
+cudaError_t launch_short(int kind, bool affine, int shape, int rows, int key_begin, int key_end,
+                         pair_task_t const *tasks, plan_bins_t *bins, score_costs_t const &costs,
+                         std::int64_t *results, int ctas, int warps, cudaStream_t stream, int compare) {
+    int const lanes = short_segment_rows(shape) / rows;
+    auto const launch = rows == 8    ? launch_short_rows8
+                        : rows == 12 ? launch_short_rows12
+                        : rows == 16 ? launch_short_rows16
+                        : rows == 20 ? launch_short_rows20
+                        : rows == 24 ? launch_short_rows24
+                                     : launch_short_rows28;
+    return launch(kind, affine, lanes, key_begin, key_end, tasks, bins, costs, results, ctas, warps, stream, compare);
 }
 
 #endif

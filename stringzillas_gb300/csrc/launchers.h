@@ -192,15 +192,15 @@ cudaError_t launch_band16(int kind, bool affine, int key_begin, int key_end, pai
                           std::size_t ring_words_per_slot, int ctas, cudaStream_t stream, void *group_states = nullptr,
                           int group_ctas = 1, int compare = 0, bool wide = false, int rows_per_lane = 8);
 
-/** Short pairs (shorter side at most 128) on the segmented 16x2 kernel: `shape` 0-6 for shorter sides up to 16, 32,
- *  64, 128, 24, 48, 96 (`short_segment_rows`); shapes 4-6 have 12 rows per lane, shapes 0-3 16 when compare mode or
- *  at most 8 classes, else 8 (`short_rows_for`); `compare` as for the 16x2 wavefront (Levenshtein only). */
-int short_rows_for(int classes, int compare, int shape);
-int short_segment_rows(int shape);
-dp_launch_shape_t short_shape(int kind, bool affine, int shape, int classes, int warps, int compare = 0);
-cudaError_t launch_short(int kind, bool affine, int shape, int key_begin, int key_end, pair_task_t const *tasks,
-                         plan_bins_t *bins, score_costs_t const &costs, std::int64_t *results, int ctas, int warps,
-                         cudaStream_t stream, int compare = 0);
+/** Short pairs (shorter side at most 256) on the segmented 16x2 kernel: `shape` 0-16 by the rows a segment holds
+ *  (`short_segment_rows`) with `rows` per lane as `short_rows_for` gives them for so many pairs (profiles over more
+ *  than `short_few_classes_k` classes: shapes of 16, 24, 32, 48, 64, 96 and 128 rows only); `compare` as for the 16x2
+ *  wavefront (Levenshtein only). */
+int short_rows_for(int classes, int compare, int shape, std::uint64_t pairs, int sm_count);
+dp_launch_shape_t short_shape(int kind, bool affine, int shape, int rows, int classes, int warps, int compare = 0);
+cudaError_t launch_short(int kind, bool affine, int shape, int rows, int key_begin, int key_end,
+                         pair_task_t const *tasks, plan_bins_t *bins, score_costs_t const &costs,
+                         std::int64_t *results, int ctas, int warps, cudaStream_t stream, int compare = 0);
 
 /** Very long unit-cost pairs on chains of warps (myers_chain.cuh): one cooperative launch scores pairs
  *  [first, first + pairs) of bin `key` with `words` (1, 2, 4) words per lane and `planes` code planes, each pair on

@@ -50,6 +50,26 @@ __device__ __forceinline__ std::int64_t trivial_score(plan_args_t const &args, s
 
 __device__ __forceinline__ int floor_log2_u64(std::uint64_t x) { return x ? 63 - __clzll((long long)x) : 0; }
 
+/** Symbols of a whole tape (bytes, where strings are transcoded in place). */
+__device__ __forceinline__ std::uint64_t tape_symbols(tape_t const &tape) {
+    if (tape.offset_bits == 32) {
+        auto const *offsets = static_cast<std::uint32_t const *>(tape.offsets);
+        return offsets[tape.count] - offsets[0];
+    }
+    auto const *offsets = static_cast<std::uint64_t const *>(tape.offsets);
+    return offsets[tape.count] - offsets[0];
+}
+
+/** Whether a call's pairs are many and long enough, by the means of their lengths, to fill the device in each of the
+ *  short route's twenty shapes. */
+__device__ __forceinline__ bool short_fine_batch(plan_args_t const &args) {
+    if (!args.short_fine) return false;
+    tape_t const &second = args.mode == mode_symmetric_k ? args.queries : args.candidates;
+    float const cells = (float)args.pairs * ((float)tape_symbols(args.queries) / (float)args.queries.count) *
+                        ((float)tape_symbols(second) / (float)second.count);
+    return cells >= short_fine_cells_k;
+}
+
 struct pair_route_info_t {
     int key; // -1 for trivial
     std::uint8_t const *rows, *cols;
@@ -61,7 +81,7 @@ struct pair_route_info_t {
  *  with one extra step of headroom for the E/F intermediates. */
 __device__ __forceinline__ pair_route_info_t route_pair(plan_args_t const &args, std::uint8_t const *first,
                                                         std::uint64_t first_length, std::uint8_t const *second,
-                                                        std::uint64_t second_length) {
+                                                        std::uint64_t second_length, bool short_fine) {
     pair_route_info_t info;
     info.key = -1;
     // Rows take the shorter string; equal lengths keep the first string on rows.
@@ -133,21 +153,25 @@ __device__ __forceinline__ pair_route_info_t route_pair(plan_args_t const &args,
         args.local_gain >= 0 && args.packed_allowed && profile_fits && args.cell_bits[length_class] == 0;
     // Short pairs: a few lanes per pair instead of a warp (dp_short.cuh).
     if (packed && !args.wide && n <= args.short_max_rows) {
-        if (args.force_route >= 0) {
-            info.key = bin_short_begin_k + 3 * short_m_classes_k; // plain form: one bin (128-row segments), input order
+        bool const plain = args.force_route >= 0;
+        int const classes = args.alphabet ? (int)args.alphabet->symbols : args.classes;
+        bool const few = !profile_fits || classes <= short_few_classes_k, large = !plain && short_fine;
+        bool const fine = few && large;
+        if (plain && n <= short_few_rows_k) {
+            info.key = bin_short_begin_k + 12 * short_m_classes_k; // plain form: one bin (128-row segments), input order
             return info;
         }
-        int const shape = n <= 16   ? 0
-                          : n <= 24 ? 4
-                          : n <= 32 ? 1
-                          : n <= 48 ? 5
-                          : n <= 64 ? 2
-                          : n <= 96 ? 6
-                                    : 3;
-        int m_class = m < 512 ? int(m / 16) : 32 + floor_log2_u64(m) - 9;
-        m_class = m_class > short_m_classes_k - 1 ? short_m_classes_k - 1 : m_class;
-        info.key = bin_short_begin_k + shape * short_m_classes_k + (short_m_classes_k - 1 - m_class);
-        return info;
+        if (n <= (fine ? short_max_rows_k : large ? short_profile_rows_k : short_few_rows_k)) {
+            int const octave = n <= 16 ? 0 : floor_log2_u64(n - 1) - 4;
+            int quarter = n <= 16 ? -1 : int((n - 1) >> (octave + 2)) - 4;
+            if (!fine) quarter |= 1;
+            int const shape = 1 + 4 * octave + quarter;
+            // Classes of 16 columns over the rows of the next smaller shape, then octaves of that excess.
+            int const excess = int(m) - (n <= 16 ? 0 : (4 << octave) * (fine ? 4 + quarter : 3 + quarter));
+            int m_class = excess < 320 ? excess / 16 : 20 + min(6, floor_log2_u64(excess) - 8);
+            info.key = bin_short_begin_k + shape * short_m_classes_k + (short_m_classes_k - 1 - m_class);
+            return info;
+        }
     }
     if (n > band_rows && fits32_early && !force64) {
         // Long pairs take a band in both forms (16-bit cells when they fit); the plain form keeps them in one bin,
@@ -202,14 +226,15 @@ __device__ __forceinline__ pair_route_info_t route_pair(plan_args_t const &args,
     return info;
 }
 
-__device__ __forceinline__ pair_route_info_t route_of_pair(plan_args_t const &args, std::uint64_t p) {
+__device__ __forceinline__ pair_route_info_t route_of_pair(plan_args_t const &args, std::uint64_t p,
+                                                           bool short_fine) {
     std::uint64_t q, c;
     pair_indices(args, p, q, c);
     std::uint8_t const *first, *second;
     std::uint64_t first_length, second_length;
     tape_string(args.queries, q, first, first_length, args.wide);
     tape_string(args.mode == mode_symmetric_k ? args.queries : args.candidates, c, second, second_length, args.wide);
-    return route_pair(args, first, first_length, second, second_length);
+    return route_pair(args, first, first_length, second, second_length, short_fine);
 }
 
 /** Whether two strings of `n` <= `m` symbols look so alike that their distance should be at most `distance`: by the
@@ -234,9 +259,11 @@ __global__ void plan_count_kernel(plan_args_t const args, plan_bins_t *__restric
     __shared__ std::uint32_t histogram[bin_keys_k];
     __shared__ unsigned long long block_cells;
     __shared__ std::uint32_t block_max_cols, block_max_myers, block_max_myers_warp, block_max_chain;
+    __shared__ bool short_fine;
     for (int i = threadIdx.x; i < bin_keys_k; i += blockDim.x) histogram[i] = 0;
     if (threadIdx.x == 0)
-        block_cells = 0, block_max_cols = 0, block_max_myers = 0, block_max_myers_warp = 0, block_max_chain = 0;
+        block_cells = 0, block_max_cols = 0, block_max_myers = 0, block_max_myers_warp = 0, block_max_chain = 0,
+        short_fine = short_fine_batch(args);
     __syncthreads();
     std::uint64_t thread_cells = 0;
     std::uint32_t thread_max_cols = 0, thread_max_myers = 0, thread_max_myers_warp = 0, thread_max_chain = 0;
@@ -249,7 +276,7 @@ __global__ void plan_count_kernel(plan_args_t const args, plan_bins_t *__restric
         std::uint64_t const p = base + lane;
         pair_route_info_t info;
         info.key = -1, info.n = info.m = 0;
-        if (p < args.pairs) info = route_of_pair(args, p);
+        if (p < args.pairs) info = route_of_pair(args, p, short_fine);
         unsigned const key = info.key < 0 ? 0xFFFFFFFFu : (unsigned)info.key;
         unsigned const peers = __match_any_sync(0xFFFFFFFFu, key);
         if (key != 0xFFFFFFFFu && lane == __ffs(peers) - 1) atomicAdd(&histogram[key], (unsigned)__popc(peers));
@@ -365,11 +392,13 @@ __global__ void plan_scatter_kernel(plan_args_t const args, plan_bins_t *__restr
                                     pair_task_t *__restrict__ tasks) {
     __shared__ std::uint32_t counts[bin_keys_k];
     __shared__ std::uint32_t bases[bin_keys_k];
+    __shared__ bool short_fine;
     int const lane = threadIdx.x & 31;
     std::uint64_t const per_block = (args.pairs + gridDim.x - 1) / gridDim.x;
     std::uint64_t const begin = min(args.pairs, (std::uint64_t)blockIdx.x * per_block);
     std::uint64_t const end = min(args.pairs, begin + per_block);
     for (int i = threadIdx.x; i < bin_keys_k; i += blockDim.x) counts[i] = 0;
+    if (threadIdx.x == 0) short_fine = short_fine_batch(args);
     __syncthreads();
     // A warp's lanes that share a bin: one shared-memory atomic for all of them; returns this lane's rank.
     auto claim = [&](unsigned key) -> std::uint32_t {
@@ -386,7 +415,7 @@ __global__ void plan_scatter_kernel(plan_args_t const args, plan_bins_t *__restr
         std::uint64_t const p = base + lane;
         pair_route_info_t info;
         info.key = -1;
-        if (p < end) info = route_of_pair(args, p);
+        if (p < end) info = route_of_pair(args, p, short_fine);
         claim(info.key < 0 ? 0xFFFFFFFFu : (unsigned)info.key);
     }
     __syncthreads();
@@ -400,7 +429,7 @@ __global__ void plan_scatter_kernel(plan_args_t const args, plan_bins_t *__restr
         std::uint64_t const p = base + lane;
         pair_route_info_t info;
         info.key = -1;
-        if (p < end) info = route_of_pair(args, p);
+        if (p < end) info = route_of_pair(args, p, short_fine);
         unsigned const key = info.key < 0 ? 0xFFFFFFFFu : (unsigned)info.key;
         std::uint32_t const rank = claim(key);
         if (key != 0xFFFFFFFFu) {

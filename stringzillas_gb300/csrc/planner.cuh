@@ -60,11 +60,24 @@ constexpr int bin_myers_warp_begin_k = bin_band16_begin_k + bin_dp_classes_k; //
 static_assert(bin_myers_warp_begin_k + myers_warp_max_words_k * myers_warp_classes_k <= bin_keys_k,
               "bin layout exceeds the key space");
 constexpr int bin_short_begin_k = bin_myers_warp_begin_k + myers_warp_max_words_k * myers_warp_classes_k; // 1488
-constexpr int short_shapes_k = 7;      // segments holding 16, 32, 64, 128, then 24, 48 and 96 rows
-constexpr int short_m_classes_k = 48;  // text-length classes per shape
-constexpr int short_max_rows_k = 128;  // default: shorter sides up to this take the short route
+constexpr int short_shapes_k = 20;     // segments holding 16 rows, then four shapes per octave up to 448
+constexpr int short_m_classes_k = 27;  // text-length classes per shape
+constexpr int short_max_rows_k = 448;  // default: shorter sides up to this take the short route (large batches)
+constexpr int short_few_rows_k = 128;  // the same for smaller batches and the plain form
+constexpr int short_profile_rows_k = 192; // the same for large batches whose profile has many classes
+constexpr int short_few_classes_k = 8; // profiles over at most this many classes fit segments of 16-28 rows per lane
+/** Pairs, and cells by the mean lengths, from which a call cuts its short pairs' rows in quarter octaves instead of
+ *  halves and takes longer ones: 655e6 cells of text pairs of 100-300 took 334 us either way (340 here), 800e6 384 -> 370
+ *  and 1.3e9 573 -> 515; 340e6 cells of DNA pairs of 16-128 226 -> 263. */
+constexpr std::uint64_t short_fine_pairs_k = 1 << 14;
+constexpr float short_fine_cells_k = 800e6f;
 static_assert(bin_short_begin_k + short_shapes_k * short_m_classes_k <= bin_keys_k, "bin layout exceeds the key space");
-constexpr int bin_myers_chain_k = bin_short_begin_k + short_shapes_k * short_m_classes_k; // 1824
+constexpr int bin_myers_chain_k = bin_short_begin_k + short_shapes_k * short_m_classes_k; // 2028
+/** Rows of a segment of one shape, on the host and on the device. */
+__host__ __device__ constexpr int short_segment_rows(int shape) {
+    return shape == 0 ? 16 : (16 << ((shape - 1) / 4)) / 4 * (5 + (shape - 1) % 4);
+}
+static_assert(short_segment_rows(short_shapes_k - 1) == short_max_rows_k, "the last shape holds the longest short pairs");
 static_assert(bin_myers_chain_k < bin_keys_k, "bin layout exceeds the key space");
 constexpr int near_min_words_k = 5; // patterns of the thread route that the near-diagonal kernel tries
 constexpr std::uint32_t near_samples_k = 128; // pairs sampled per call
@@ -113,6 +126,8 @@ struct plan_args_t {
     std::uint16_t packed_step_cost[4];  // relative cost of one lane step with 4, 8, 12, 16 rows per lane
     std::uint32_t band_min_rows_compare; // the same for compare-mode Levenshtein pairs (no profile)
     std::uint32_t short_max_rows;        // 16x2 pairs whose shorter side is at most this take the short route
+    int short_fine;                      // 1: quarter octaves of rows, where the profile has few classes
+    int classes;                         // profile classes of the engine's table (not read for Levenshtein or dense)
     std::uint32_t near_sample_stride;    // unit-cost calls: every so many pairs one is sampled for likeness (0: none)
 };
 

@@ -1307,3 +1307,38 @@ def test_tilted_tracks_at_the_16bit_bound(szs, port, family, costs, gain, rows):
                        "band_min_rows_few": 1 << 20, "short_max_rows": 1})
     got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
     np.testing.assert_array_equal(got, port.pairs(oracle_costs, tape(first), tape(second)))
+
+
+@pytest.mark.parametrize("name,family,costs,letters", [
+    ("lev-linear", "lev", (0, 3, 2, 2), 4), ("lev-affine", "lev", (0, 4, 5, 2), 8), ("lev-nine", "lev", (0, 4, 5, 2), 9),
+    ("multiply", "lev", (0, 2, 3, 1), 256), ("select", "lev", (0, 5, 3, 1), 256), ("compare-linear", "lev", (3, 1, 5, 5), 256),
+    ("nw-linear", "nw", (-5, -5), 4), ("nw-affine", "nw", (-11, -1), 4), ("nw-protein", "nw", (-11, -1), 20),
+    ("sw-linear", "sw", (-5, -5), 4), ("sw-affine", "sw", (-5, -2), 4), ("sw-free-gaps", "sw", (0, 0), 4),
+    ("sw-positive-gaps", "sw", (1, 2), 4), ("sw-protein", "sw", (-11, -1), 20)])
+def test_short_pairs_of_large_batches(szs, port, name, family, costs, letters):
+    """Large batches cut short pairs into quarter octaves of rows up to 448 (over few symbols, or comparing codes; up to
+    192 in halves over many): both sides of every shape's limit and lengths in between, texts from one character to
+    thousands, empty strings, partners of one segment with uneven rows and columns."""
+    rng = np.random.default_rng(zlib_seed(name))
+    alphabet = {4: DNA, 20: PROTEIN}.get(letters, np.arange(letters, dtype=np.uint8))
+    b2c, table = protein_tables(rng, symmetric=False) if letters == 20 else dna_tables()
+    edges = [16] + [(16 << k) * q // 4 for k in range(5) for q in (5, 6, 7, 8)][:19]
+    lengths = [(n, m) for e in edges for n in (e - 1, e, e + 1) for m in (1, e, e + 17, 2 * e + 5)]
+    lengths += [(0, 300), (300, 0), (0, 0), (20, 3000), (200, 2500), (448, 1500)]
+    count = 17000
+    drawn = rng.integers(1, 470, size=(count - len(lengths), 2))
+    lengths += [tuple(pair) for pair in drawn]
+    pool = rng.choice(alphabet, size=1 << 20).astype(np.uint8)
+    starts = rng.integers(0, pool.size - 4000, size=(count, 2))
+    def cut(side):
+        return [bytes(pool[starts[i, side]:starts[i, side] + lengths[i][side]]) for i in range(count)]
+    first, second = cut(0), cut(1)
+    for k in range(0, count, 5):  # alike, too: the second string within the first one's
+        second[k] = first[k][: len(first[k]) // 2] + first[k][len(first[k]) // 2 + 2:]
+    mean = np.mean([len(s) for s in first]) * np.mean([len(s) for s in second])
+    assert count * mean > 800e6
+    engine, oracle_costs = make_engine(szs, family, costs, b2c, table)
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    want = port.pairs(oracle_costs, tape(first), tape(second))
+    bad = np.flatnonzero(got != want)
+    assert bad.size == 0, f"{bad.size} mismatches, first {[(lengths[b], got[b], want[b]) for b in bad[:5]]}"
