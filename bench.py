@@ -52,7 +52,9 @@ METRIC = "GCUPS batched Levenshtein/NW/SW, 1 GB300, vs plain launch; serving p50
 #  - 16x2 compare mode (Levenshtein over more than 32 byte values): per register of two cells, affine 5 DPX + 1 DPX
 #    add-min (0 where the codes are equal, else 1) + 1 multiply-add giving both pairs' costs -> 3.5 per cell.
 #  - bit-parallel over at most four symbols (the shared-table kernel, DNA): the match masks come from shared memory,
-#    so per word and column only the 10 ops of the Myers step remain -> 10 / 32 per cell.
+#    so per word and column only the 10 ops of the Myers step remain -> 10 / 32 per cell. Pairs that are alike (these
+#    workloads' partners) are scored in a window of words along the diagonal, so only its cells count (`scored_share`).
+#  - global affine 16x2 cells may be tilted (4 DPX instead of 5: 2.5 per cell); the fraction still counts 3.0.
 OPS_PER_CELL = {"myers_dna": 13.0 / 32.0, "myers_dna_table": 10.0 / 32.0, "dp_linear": 4.0, "dp_affine": 7.0,
                 "packed_affine": 3.0, "packed_affine_local": 3.5, "packed_compare_affine": 3.5}
 
@@ -87,15 +89,14 @@ WORKLOADS = {
 }
 
 
-# DRAM bytes per step of the dominant kernels, from one ncu capture of the same command
-# (profiles/myers_table_c2_dram_traffic.txt: dram__bytes_read.sum + dram__bytes_write.sum over one step's launches).
-DRAM_TRAFFIC_PER_STEP = {"c2": 702.2e6 + 1.1e6}
+# DRAM bytes per step of the dominant kernels, from an ncu capture of the same command, where one was taken of the
+# kernels that run now.
+DRAM_TRAFFIC_PER_STEP = {}
 
 # What ncu shows about the dominant kernel's integer pipe, beside the algorithmic fraction above
-# (profiles/myers_table_c2_batched_levenshtein.txt).
-PIPE_EVIDENCE = {"c2": "ncu, shared-table bit-parallel kernel (W = 8 and 7): ALU pipe 84 % busy, 12.4 ALU instructions "
-                       "executed per pattern word and text column against the step's 10 (byte extraction, table "
-                       "address, alphabet check, pattern setup)"}
+# (profiles/myers_near_dna_reads.txt).
+PIPE_EVIDENCE = {"c2": "ncu, window of three words along the diagonal: ALU pipe 85 % busy, 2.4 instructions per cycle and SM, "
+                       "DRAM 15 %"}
 
 
 def parse_args():
@@ -244,6 +245,18 @@ def ops_per_cell(kind_and_tables):
     if kind == "levp":
         return OPS_PER_CELL["packed_affine"]
     return OPS_PER_CELL["packed_affine_local"] if kind == "sw" else OPS_PER_CELL["packed_affine"]
+
+
+def scored_share(first, second, kind_and_tables):
+    """Share of the matrices' cells that the kernels score: alike pairs of unit-cost workloads take a window of three words
+    along the diagonal from five words of pattern on, nine beyond sixteen words in batches of 16 pairs per SM."""
+    if kind_and_tables[0] != "lev":
+        return 1.0
+    a, b = np.diff(first[1]).astype(np.int64), np.diff(second[1]).astype(np.int64)
+    n, m = np.minimum(a, b), np.maximum(a, b)
+    words = (n + 31) // 32
+    window = np.where(words < 5, n, np.where(words <= 16, 96, n if len(n) < 16 * 152 else 288))
+    return float((np.minimum(window, n) * m).sum() / max(1, (n * m).sum()))
 
 
 class Clocks:
@@ -669,9 +682,8 @@ FINGERPRINT_WORKLOAD = ("Min-Hash fingerprints: 16,384 documents, len U[1,000, 3
 # Integer operations per byte and dimension, counted from the rolling step: x = state*a + D*out + (D + 1 + in) (two
 # 32x64-bit products as multiply-adds and two 64-bit adds: 6), the reduction to [0, 2m) (shift, multiply-high,
 # shift, 32x64-bit product, 64-bit subtract: 7) and the high-word test against the running minimum (3). The
-# executed count (ncu, profiles/fingerprints_minhash_1024d.txt) is 28.8 instructions per byte-dimension.
+# rolling kernel executes 28.8 instructions per byte-dimension (ncu, profiles/fingerprints_minhash_1024d.txt).
 FINGERPRINT_OPS_PER_BYTE_DIM = 16.0
-FINGERPRINT_EXECUTED_INST_PER_BYTE_DIM = 28.8
 
 
 def fingerprint_texts(count=16384, low=1000, high=3000, seed=7):
@@ -744,8 +756,8 @@ def fingerprints_leg(szs, torch, scope, peaks, steps=3, warmup=3, cpu_seconds=10
                          "peak": None if int_peak is None else int_peak / 1e12, "unit": "Tops/s",
                          "frac": None if int_peak is None else ops / (device_ms * 1e-3) / int_peak,
                          "ops_per_byte_dimension": FINGERPRINT_OPS_PER_BYTE_DIM,
-                         "executed_instructions_per_byte_dimension": FINGERPRINT_EXECUTED_INST_PER_BYTE_DIM,
-                         "note": "bound by the integer multiply-add pipe (68.9% busy in ncu), not by memory"},
+                         "note": "the operations of the rolling form; windows of up to 32 bytes are dot products on "
+                                 "tensor cores, which the integer pipe never sees: the fraction exceeds 1"},
         "cpu_baseline": {"value": done_bytes * dims / cpu_s / 1e9, "unit": "G byte-dimensions/s", "cores": 1,
                          "kind": "port", "sample": f"{done_bytes} bytes of the documents, oracle C restatement"},
         "sample_parity_exact": exact,
@@ -839,7 +851,8 @@ def run_ours(args):
         step_compute_s = compute_ms / args.steps * 1e-3
         algorithmic_bytes = input_bytes + 8 * pairs
         achieved_gbs = algorithmic_bytes / step_compute_s / 1e9
-        int_ops = cells_per_step * ops_per_cell(kind_and_tables)
+        share = scored_share(first, second, kind_and_tables)
+        int_ops = cells_per_step * share * ops_per_cell(kind_and_tables)
         int_peak = None
         if peaks:
             int_peak = {"lev": peaks["lop3"], "nw32": peaks["dpx_viaddmax_s32"], "nwd": peaks["dpx_viaddmax_s32"]}.get(
@@ -858,7 +871,7 @@ def run_ours(args):
             "roofline_int": {"bound": "int_pipe", "achieved": int_ops / step_compute_s / 1e12,
                              "peak": None if int_peak is None else int_peak / 1e12, "unit": "Tops/s",
                              "frac": None if int_peak is None else int_ops / step_compute_s / int_peak,
-                             "ops_per_cell": ops_per_cell(kind_and_tables), "measured_peaks_tops":
+                             "ops_per_cell": ops_per_cell(kind_and_tables), "scored_share": share, "measured_peaks_tops":
                                  None if peaks is None else {k: v / 1e12 for k, v in peaks.items()},
                              "pipe_evidence": PIPE_EVIDENCE.get(args.workload)},
             "plain": {"value": plain_cells / (plain_ms * 1e-3) / 1e9, "unit": "GCUPS",
