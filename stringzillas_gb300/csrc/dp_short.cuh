@@ -60,8 +60,11 @@ struct short_policy_t {
     static constexpr int segments_k = warp_size_k / lanes_;
     static constexpr bool compare_k = compare_ != compare_none_k;
     static constexpr bool multiply_k = compare_ == compare_multiply_k;
-    // Four warps per scheduler in 128 registers; three tracks of 24 or 28 rows (H, E and the codes) take 168 instead.
-    static constexpr int ctas_per_sm_k = compare_k && affine_ && rows_per_lane_ >= 24 ? 3 : 4;
+    // Four warps per scheduler in 128 registers; 8 rows, and 12 of local scores, leave room for five in 96; three tracks of
+    // 24 or 28 rows (H, E and the codes) take three in 168.
+    static constexpr int ctas_per_sm_k = rows_per_lane_ == 8 || (rows_per_lane_ == 12 && local_k) ? 5
+                                         : compare_k && affine_ && rows_per_lane_ >= 24           ? 3
+                                                                                                  : 4;
     static_assert(lanes_ == 1 || lanes_ == 2 || lanes_ == 4 || lanes_ == 8 || lanes_ == 16, "segments of 1 to 16 lanes");
     static_assert(rows_per_lane_ % 4 == 0, "profile rows are read in 4-byte words");
     static_assert(segment_rows_k <= short_max_rows_k, "a pair's whole column fits one strip");
@@ -377,13 +380,14 @@ __global__ void __launch_bounds__(128, policy_::ctas_per_sm_k) dp16_short_kernel
         // Row-class-major copies of both orientations: row_costs[o][row class][column class] = table - shift (the
         // affine tracks' s - open, which the planner checked fits a byte); the filler row after each.
         std::int32_t const shift = policy_::affine_k ? costs.open : 0;
-        for (unsigned i = threadIdx.x; i < 2 * short_row_classes_k * 32; i += blockDim.x) {
-            unsigned const o = i / (short_row_classes_k * 32), row = i / 32 % short_row_classes_k, column = i & 31u;
+        for (unsigned i = threadIdx.x; i < 2 * 32 * 32; i += blockDim.x) {
+            unsigned const o = i >> 10, row = (i >> 5) & 31u, column = i & 31u;
             std::int8_t const *table = o ? costs.profile_table_t : costs.profile_table;
-            row_costs[i] = row == short_filler_class_k
-                               ? std::uint8_t(0x80)
-                               : (std::uint8_t)(std::int8_t)(table[column * 32 + row] - shift);
+            row_costs[o * short_row_classes_k * 32 + row * 32 + column] =
+                (std::uint8_t)(std::int8_t)(table[column * 32 + row] - shift);
         }
+        for (unsigned i = threadIdx.x; i < 2 * 32; i += blockDim.x)
+            row_costs[(i >> 5) * short_row_classes_k * 32 + short_filler_class_k * 32 + (i & 31u)] = 0x80;
     }
     __syncthreads();
     int const lane = threadIdx.x & 31;
