@@ -1126,9 +1126,9 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
     // classes (octaves of cells) get groups of CTAs, as many as bring a pair to about half a share, but no more than the
     // class's smallest patterns have strips for, while they hold less than half of the call's cells and their pairs
     // nearly twice the mean (pairs of like sizes balance by themselves: 160 pairs of 5,000-12,000 take 6.0 ms single,
-    // 8.6 ms with their largest in groups; 300 of 2,000-16,000 log-uniform 13.4 ms single, 9.6 ms). Not the 32-bit band, whose single CTAs score more per step than its groups (400 pairs of
-    // 1,100-6,000: 5.1 ms single, 7.5 ms grouped). Returns the first bin left to single CTAs; calls with few pairs are
-    // left to `band_groups`.
+    // 8.6 ms with their largest in groups; 300 of 2,000-16,000 log-uniform 13.4 ms single, 9.6 ms). Not the 32-bit band,
+    // whose single CTAs score more per step than its groups (400 pairs of 1,100-6,000: 5.1 ms single, 7.5 ms grouped).
+    // Returns the first bin left to single CTAs; calls with few pairs are left to `band_groups`.
     auto band_largest = [&](std::uint64_t pairs_here, dp_launch_shape_t const &shape, std::uint64_t strip_rows,
                             std::size_t bytes_per_warp) -> int {
         int const key_begin = bin_band16_begin_k, key_end = key_begin + bin_dp_classes_k;
