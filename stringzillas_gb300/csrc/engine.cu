@@ -1386,6 +1386,11 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             key_append(launch_key, jobs[i].ctas), key_append(launch_key, jobs[i].scratch_offset);
             key_append(launch_key, jobs[i].group_ctas), key_append(launch_key, jobs[i].state_offset);
             key_append(launch_key, jobs[i].rows), key_append(launch_key, jobs[i].listed);
+            // A chained job's launches follow from its pairs and its longest pattern and text; it has no `ctas`.
+            if (jobs[i].kind == job_myers_chain_k) {
+                key_append(launch_key, jobs[i].pairs), key_append(launch_key, chain_strips);
+                key_append(launch_key, chain_wave), key_append(launch_key, chain_link_stride);
+            }
         }
         key_append(launch_key, packed_costs), key_append(launch_key, call_costs);
         key_append(launch_key, tasks), key_append(launch_key, bins), key_append(launch_key, results);

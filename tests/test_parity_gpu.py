@@ -1342,3 +1342,42 @@ def test_short_pairs_of_large_batches(szs, port, name, family, costs, letters):
     want = port.pairs(oracle_costs, tape(first), tape(second))
     bad = np.flatnonzero(got != want)
     assert bad.size == 0, f"{bad.size} mismatches, first {[(lengths[b], got[b], want[b]) for b in bad[:5]]}"
+
+
+def test_chained_graphs_follow_their_pairs(szs, port):
+    """Chains of warps (patterns past 8,192 bytes) in device buffers rewritten in place, every launch shape but the
+    chain's own unchanged: a longer pattern beside the same text (20 strips of 1,024 rows after 9), then two chained
+    pairs after one. Each call scores what the buffers hold, not the chains of an earlier graph."""
+    import torch
+    rng = np.random.default_rng(2024)
+    text = [rng.choice(DNA, size=21000) for _ in range(2)]
+    room = 70000
+    data = [torch.zeros(room, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    offsets = [torch.zeros(4, dtype=torch.int64, device="cuda") for _ in range(2)]
+    out = torch.zeros(3, dtype=torch.int64, device="cuda")
+    engine = szs.LevenshteinDistances()
+
+    def mutant(symbols, size):
+        symbols = symbols[:size].copy()
+        where = rng.random(size) < 0.1
+        symbols[where] = rng.choice(DNA, size=int(where.sum()))
+        return bytes(symbols)
+
+    def score(first, second):
+        for side, strings in enumerate((first, second)):
+            string_data, string_offsets = tape(strings)
+            data[side][:len(string_data)] = torch.from_numpy(string_data.copy()).cuda()
+            offsets[side].copy_(torch.from_numpy(string_offsets.astype(np.int64)))
+        out.fill_(-1)
+        torch.cuda.synchronize()
+        engine.pairwise(*(szs.Strs.from_buffers(d, o) for d, o in zip(data, offsets)), out=out)
+        want = port.pairs(oracle.levenshtein_costs(), tape(first), tape(second))
+        np.testing.assert_array_equal(out.cpu().numpy(), want)
+
+    short = bytes(rng.choice(DNA, size=70))
+    long = [bytes(t) for t in text]
+    score([mutant(text[0], 20000), mutant(text[1], 20000), short], [long[0], long[1], short[2:]])  # the scratch's size
+    for patterns in ((9000,), (20000,), (9000, 9000), (9000,), (9000, 20000)):
+        first = [mutant(text[i], size) for i, size in enumerate(patterns)] + [short] * (3 - len(patterns))
+        second = long[:len(patterns)] + [short[3:]] * (3 - len(patterns))
+        score(first, second)
