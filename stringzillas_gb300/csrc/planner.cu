@@ -48,8 +48,6 @@ __device__ __forceinline__ std::int64_t trivial_score(plan_args_t const &args, s
     return length == 0 ? 0 : (std::int64_t)args.open + (std::int64_t)args.extend * (std::int64_t)(length - 1);
 }
 
-__device__ __forceinline__ int floor_log2_u64(std::uint64_t x) { return x ? 63 - __clzll((long long)x) : 0; }
-
 /** Symbols of a whole tape (bytes, where strings are transcoded in place). */
 __device__ __forceinline__ std::uint64_t tape_symbols(tape_t const &tape) {
     if (tape.offset_bits == 32) {
@@ -162,14 +160,7 @@ __device__ __forceinline__ pair_route_info_t route_pair(plan_args_t const &args,
             return info;
         }
         if (n <= (fine ? short_max_rows_k : large ? short_profile_rows_k : short_few_rows_k)) {
-            int const octave = n <= 16 ? 0 : floor_log2_u64(n - 1) - 4;
-            int quarter = n <= 16 ? -1 : int((n - 1) >> (octave + 2)) - 4;
-            if (!fine) quarter |= 1;
-            int const shape = 1 + 4 * octave + quarter;
-            // Classes of 16 columns over the rows of the next smaller shape, then octaves of that excess.
-            int const excess = int(m) - (n <= 16 ? 0 : (4 << octave) * (fine ? 4 + quarter : 3 + quarter));
-            int m_class = excess < 320 ? excess / 16 : 20 + min(6, floor_log2_u64(excess) - 8);
-            info.key = bin_short_begin_k + shape * short_m_classes_k + (short_m_classes_k - 1 - m_class);
+            info.key = short_bin(n, m, fine);
             return info;
         }
     }

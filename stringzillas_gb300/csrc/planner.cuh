@@ -20,10 +20,10 @@
  *    [1392, 1424) 16-bit band (one CTA per pair, 16x2 cells): same layout from 1392
  *    [1424, 1488) warp-per-pair Myers (unit Levenshtein, shorter side 513..8,192): key = 1424 + 8 * (8 - W)
  *                 + (7 - text class), W = words per lane = ceil(n / 1024), text class ~ log2(m) - 9
- *    [1488, 1824) short pairs on 16x2 cells (shorter side <= 128): key = 1488 + 48 * shape + (47 - m class),
- *                 shape 0/4/1/5/2/6/3 for n <= 16/24/32/48/64/96/128, m class = m / 16 below 512, then
- *                 32 + log2(m) - 9
- *    1824         unit-cost Levenshtein beyond the warp kernel (shorter side 8,193 .. 2^20): a chain of warps per pair
+ *    [1488, 2028) short pairs on 16x2 cells (shorter side <= 448): key = 1488 + 27 * shape + (26 - m class), shape 0 for
+ *                 n <= 16, then four per octave (`short_segment_rows`), m class = excess / 16 below 320, then
+ *                 20 + log2(excess) - 8, excess = m - rows of the next smaller shape
+ *    2028         unit-cost Levenshtein beyond the warp kernel (shorter side 8,193 .. 2^20): a chain of warps per pair
  */
 #pragma once
 #include "engine_types.cuh"
@@ -78,6 +78,29 @@ __host__ __device__ constexpr int short_segment_rows(int shape) {
     return shape == 0 ? 16 : (16 << ((shape - 1) / 4)) / 4 * (5 + (shape - 1) % 4);
 }
 static_assert(short_segment_rows(short_shapes_k - 1) == short_max_rows_k, "the last shape holds the longest short pairs");
+
+__host__ __device__ inline int floor_log2_u64(std::uint64_t x) {
+#ifdef __CUDA_ARCH__
+    return x ? 63 - __clzll((long long)x) : 0;
+#else
+    return x ? 63 - __builtin_clzll(x) : 0;
+#endif
+}
+
+/** Bin of a short pair of n rows (at most 448) and m >= n columns, its rows cut in quarters of an octave when `fine`, else
+ *  in halves. Classes of 16 columns over the rows of the next smaller shape, then octaves of that excess, which has 64 bits:
+ *  a local pair's text may have 2^31 symbols and more. */
+__host__ __device__ inline int short_bin(std::uint64_t n, std::uint64_t m, bool fine) {
+    int const octave = n <= 16 ? 0 : floor_log2_u64(n - 1) - 4;
+    int quarter = n <= 16 ? -1 : int((n - 1) >> (octave + 2)) - 4;
+    if (!fine) quarter |= 1;
+    std::uint64_t const smaller = n <= 16 ? 0 : (4u << octave) * (fine ? 4u + quarter : 3u + quarter);
+    std::uint64_t const excess = m - smaller;
+    int const octaves = floor_log2_u64(excess) - 8;
+    int const m_class = excess < 320 ? int(excess / 16) : 20 + (octaves < 6 ? octaves : 6);
+    return bin_short_begin_k + (1 + 4 * octave + quarter) * short_m_classes_k + (short_m_classes_k - 1 - m_class);
+}
+
 static_assert(bin_myers_chain_k < bin_keys_k, "bin layout exceeds the key space");
 constexpr int near_min_words_k = 5; // patterns of the thread route that the near-diagonal kernel tries
 constexpr std::uint32_t near_samples_k = 128; // pairs sampled per call
