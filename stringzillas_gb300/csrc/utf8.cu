@@ -57,9 +57,11 @@ constexpr int utf8_threads_k = 128;
  *  is well formed in the decoder's sense: its continuation bytes (10xxxxxx) are exactly those that its lead bytes ask
  *  for, the byte after every lead of 0xC0 or more, the second after 0xE0 or more and the third after 0xF0 or more, none
  *  past `stop`; then the code points start exactly at the other bytes, as a sequential walk would find them. Returns
- *  false, warp-uniformly, as soon as a window breaks that (code points visited before stay visited: both passes then
- *  walk the whole string again sequentially), or for strings of 2^31 bytes or more. Sets `count` to the string's code
- *  points on success. `positions`: 128 bytes of shared memory of the warp's own.
+ *  false, warp-uniformly, as soon as a window breaks that, or for strings of 2^31 bytes or more; both passes then walk the
+ *  whole string again sequentially. Code points visited before stay visited, so each has to be one that this walk finds
+ *  too: windows before a broken one are, and a sequence that leaves its window is decoded there only if the string holds
+ *  all of its bytes (the sequential walk reads on into the next string). Sets `count` to the string's code points on
+ *  success. `positions`: 128 bytes of shared memory of the warp's own.
  */
 template <typename visit_>
 __device__ __forceinline__ bool warp_walk(tape_t const &tape, std::uint64_t begin, std::uint64_t stop,
@@ -106,7 +108,9 @@ __device__ __forceinline__ bool warp_walk(tape_t const &tape, std::uint64_t begi
         bool const broken = (here | (lane ? above : asked)) != continuation;
         std::uint32_t const carried = __shfl_sync(0xFFFFFFFFu, beyond, 31);
         asked = lane ? 0u : carried;
-        if (__any_sync(0xFFFFFFFFu, broken)) return false;
+        std::uint32_t const left = n - min(window + 128, n); // the string's bytes after this window
+        bool const cut = left < 3 && carried >> (8 * left);
+        if (__any_sync(0xFFFFFFFFu, broken || cut)) return false;
         std::uint32_t const leads = (((valid & ~continuation) >> 7) * 0x01020408u) >> 24; // four bits
         // The window's code points in order: their positions, so that lane k takes the k-th.
         std::uint32_t const found = __popc(leads);
@@ -137,7 +141,7 @@ __device__ __forceinline__ bool warp_walk(tape_t const &tape, std::uint64_t begi
         runes += total;
     }
     count = runes;
-    return !__any_sync(0xFFFFFFFFu, asked); // a sequence cut off by the string's end
+    return true;
 }
 
 /** Pass 1: code points per string, the bitmap, and the code points as 16-bit values (truncated beyond the Basic

@@ -1381,3 +1381,22 @@ def test_chained_graphs_follow_their_pairs(szs, port):
         first = [mutant(text[i], size) for i, size in enumerate(patterns)] + [short] * (3 - len(patterns))
         second = long[:len(patterns)] + [short[3:]] * (3 - len(patterns))
         score(first, second)
+
+
+@pytest.mark.parametrize("size", [128, 129, 130, 256])
+def test_utf8_cut_sequences_add_no_code_points(szs, port, size):
+    """A call over exactly 65,536 distinct code points, the most there may be, one of them spelt by sequences that their
+    strings' ends cut off at the end of a 128-byte window: the decoder reads on into the next string, whose bytes finish
+    the same code point at every alignment. Nothing else may be counted on the way."""
+    spelt = b"\xF1\xA1\xA2\xA3"  # one code point beyond the Basic Multilingual Plane
+    inside = size - 127 if size < 256 else 1  # its bytes before the string's end, the first one a window's last
+    cut = b"a" * (size - inside) + spelt[:inside]
+    first = []
+    for shift in range(4):  # at every alignment
+        first += [b"a" * (4 + (shift - len(b"".join(first))) % 4), cut, spelt[inside:] + b"b"]
+    plane = [chr(point).encode("utf-8", "surrogatepass") for point in range(0xFFFF)]
+    first += [b"".join(plane[i:i + 199]) for i in range(0, len(plane), 199)]
+    second = [text[len(text) // 2:] if i >= 12 and i % 2 else text for i, text in enumerate(first)]
+    engine = szs.LevenshteinDistancesUTF8()
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_utf8_costs(), tape(first), tape(second)))
