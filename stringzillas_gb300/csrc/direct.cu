@@ -16,7 +16,7 @@
  *  1.01 ms here; 2,048 x 2,048 tokens of 4-16 bytes 0.25 ms with the pattern's bit planes built by every thread, 0.12 ms
  *  here; 197 x 198 of 100 bytes 112 us planned, 52 us here.
  *
- *  Either side may be the pattern: the queries, unless they are longer than 1,024 bytes and the candidates are not.
+ *  Either side may be the pattern, by `direct_choice`, which also leaves calls to the planned routes (direct_rule.h).
  *  Words are chosen per pattern inside a kernel, in steps that fit its class (up to 128, 512 and 1,024 rows), which the
  *  host picks by the longest pattern; classes keep the registers of the long patterns off the short ones.
  *
@@ -171,45 +171,65 @@ __global__ void __launch_bounds__(256, most_ <= 4 ? 5 : (most_ <= 16 ? 3 : 2))
     }
 }
 
-/** The longest string of each tape (one CTA each), and the sum of their lengths, straight into page-locked host memory. */
+/** One part of a tape per CTA (queries for blockIdx.y 0, candidates for 1), straight into page-locked host memory. The
+ *  call waits for it, so its reductions are few: what a group of 32 strings shares is the same in all lanes as it is, and
+ *  the sums of words, which only choose a route, have 32 bits per warp (2,048 x 2,048 tokens: 120 us a call with seven sums
+ *  in 64 bits and atomics, 117 this way). */
 __global__ void __launch_bounds__(1024) direct_extents_kernel(tape_t const queries, tape_t const candidates,
-                                                              std::uint64_t *__restrict__ extents) {
-    __shared__ unsigned long long longest_s, sum_s;
-    if (threadIdx.x == 0) longest_s = 0, sum_s = 0;
-    __syncthreads();
-    tape_t const &tape = blockIdx.x ? candidates : queries;
-    unsigned long long longest = 0, sum = 0;
+                                                              int const query_parts, int const candidate_parts,
+                                                              direct_extents_t *__restrict__ extents) {
+    int const parts = blockIdx.y ? candidate_parts : query_parts;
+    if ((int)blockIdx.x >= parts) return;
+    constexpr int fields = sizeof(direct_extents_t) / 8;
+    __shared__ unsigned long long warps_s[fields][32];
+    int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    tape_t const &tape = blockIdx.y ? candidates : queries;
+    unsigned long long symbols = 0, padded = 0;
+    std::uint32_t longest = 0, words = 0, to_two = 0, to_four = 0, long_words = 0;
+    // A warp takes 32 strings at a time, the group that a warp of the direct kernels would.
+    std::uint64_t const threads = (std::uint64_t)parts * blockDim.x;
+    std::uint64_t const rounded = (tape.count + 31) / 32 * 32;
 #pragma unroll 8
-    for (std::uint64_t i = threadIdx.x; i < tape.count; i += blockDim.x) {
+    for (std::uint64_t i = (std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rounded; i += threads) {
         std::uint8_t const *start;
-        std::uint64_t length;
-        direct_string(tape, i, start, length);
-        longest = max(longest, (unsigned long long)length), sum += length;
+        std::uint64_t length = 0;
+        if (i < tape.count) direct_string(tape, i, start, length);
+        std::uint32_t const most = __reduce_max_sync(0xFFFFFFFFu, (std::uint32_t)min(length, (std::uint64_t)0xFFFFFFFFu));
+        std::uint32_t const here = (std::uint32_t)((length + 31) / 32);
+        longest = max(longest, most);
+        symbols += length, padded += 32ull * most;
+        words += here, to_two += here & 1u, to_four += (0u - here) & 3u;
+        long_words += length > 512 ? here : 0u;
     }
+    unsigned long long const low = __reduce_add_sync(0xFFFFFFFFu, (std::uint32_t)symbols & 0xFFFFu);
+    unsigned long long const high = __reduce_add_sync(0xFFFFFFFFu, (std::uint32_t)(symbols >> 16));
+    words = __reduce_add_sync(0xFFFFFFFFu, words), to_two = __reduce_add_sync(0xFFFFFFFFu, to_two);
+    to_four = __reduce_add_sync(0xFFFFFFFFu, to_four), long_words = __reduce_add_sync(0xFFFFFFFFu, long_words);
+    if (lane == 0) {
+        warps_s[0][warp] = longest, warps_s[1][warp] = (high << 16) + low, warps_s[2][warp] = padded;
+        warps_s[3][warp] = words, warps_s[4][warp] = (unsigned long long)words + to_two;
+        warps_s[5][warp] = (unsigned long long)words + to_four, warps_s[6][warp] = long_words;
+    }
+    __syncthreads();
+    if (warp >= fields) return;
+    unsigned long long value = warps_s[warp][lane];
 #pragma unroll
     for (int distance = 16; distance; distance >>= 1) {
-        longest = max(longest, __shfl_xor_sync(0xFFFFFFFFu, longest, distance));
-        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, distance);
+        unsigned long long const other = __shfl_xor_sync(0xFFFFFFFFu, value, distance);
+        value = warp == 0 ? max(value, other) : value + other;
     }
-    if ((threadIdx.x & 31) == 0) atomicMax(&longest_s, longest), atomicAdd(&sum_s, sum);
-    __syncthreads();
-    if (threadIdx.x == 0) extents[2 * blockIdx.x] = longest_s, extents[2 * blockIdx.x + 1] = sum_s;
+    if (lane == 0)
+        reinterpret_cast<unsigned long long *>(extents + (blockIdx.y ? query_parts : 0) + blockIdx.x)[warp] = value;
 }
 
 } // namespace
 
-cudaError_t launch_direct_extents(tape_t const &queries, tape_t const &candidates, std::uint64_t *extents,
+cudaError_t launch_direct_extents(tape_t const &queries, tape_t const &candidates, direct_extents_t *extents,
                                   cudaStream_t stream) {
-    direct_extents_kernel<<<2, 1024, 0, stream>>>(queries, candidates, extents);
+    int const query_parts = direct_extents_parts(queries.count), candidate_parts = direct_extents_parts(candidates.count);
+    dim3 const grid(std::max(query_parts, candidate_parts), 2);
+    direct_extents_kernel<<<grid, 1024, 0, stream>>>(queries, candidates, query_parts, candidate_parts, extents);
     return cudaGetLastError();
-}
-
-bool myers_direct_takes(std::uint64_t longest_query, std::uint64_t longest_candidate, std::uint64_t pairs,
-                        bool &swapped) {
-    swapped = longest_query > direct_max_rows_k && longest_candidate <= direct_max_rows_k;
-    std::uint64_t const rows = swapped ? longest_candidate : longest_query;
-    if (rows > direct_max_rows_k || longest_query >= (1ull << 31) || longest_candidate >= (1ull << 31)) return false;
-    return rows <= 512 || pairs >= direct_min_pairs_k;
 }
 
 cudaError_t launch_myers_direct(tape_t const &queries, tape_t const &candidates, bool swapped, std::uint64_t longest_rows,
@@ -218,14 +238,14 @@ cudaError_t launch_myers_direct(tape_t const &queries, tape_t const &candidates,
     // Small CTAs while there are few cells for the SMs, so that the last round is even; larger ones share a pattern's
     // table among more threads.
     unsigned threads = 256;
-    while (threads > 64 && patterns.count * ((texts.count + threads - 1) / threads) < (std::uint64_t)sm_count * 8)
+    while (threads > 64 && (threads / 2 >= texts.count ||
+                            patterns.count * ((texts.count + threads - 1) / threads) < (std::uint64_t)sm_count * 8))
         threads /= 2;
     // A CTA's table serves several rounds of texts when the patterns alone make enough CTAs (about four waves of five per
-    // SM): 2,048 x 2,048 tokens take 123 us with a table per 256 cells,
-    // 116 us with one per 1,024.
+    // SM): 2,048 x 2,048 tokens take 123 us with a table per 256 cells, 116 us with one per 1,024.
     std::uint64_t const columns = (texts.count + threads - 1) / threads;
     std::uint64_t const across = ((std::uint64_t)sm_count * 20 + patterns.count - 1) / patterns.count;
-    unsigned const grid_x = (unsigned)std::min<std::uint64_t>({columns, across, 1024});
+    unsigned const grid_x = (unsigned)std::min<std::uint64_t>(columns, across);
     std::uint64_t const wanted = ((std::uint64_t)sm_count * 32 + grid_x - 1) / grid_x;
     unsigned const grid_y = (unsigned)std::min<std::uint64_t>({patterns.count, wanted, 65535});
     dim3 const grid(grid_x, grid_y);

@@ -277,7 +277,7 @@ struct device_context_t {
         // The alphabet's mark words must start at zero (each alphabet pass clears them again).
         SZS_TRY_CUDA(cudaMemsetAsync(control.data, 0, control.bytes, own_stream));
         SZS_TRY_CUDA(cudaStreamSynchronize(own_stream));
-        status = readback.reserve(sizeof(plan_bins_t) + sizeof(batch_alphabet_t) + 256);
+        status = readback.reserve(sizeof(plan_bins_t) + sizeof(batch_alphabet_t) + spare_bytes_k);
         if (!status.ok()) return status;
         ready = true;
         return {};
@@ -290,7 +290,8 @@ struct device_context_t {
     batch_alphabet_t *alphabet_host() const noexcept {
         return reinterpret_cast<batch_alphabet_t *>(static_cast<unsigned char *>(readback.data) + sizeof(plan_bins_t));
     }
-    /** 256 spare bytes after the plan and the alphabet of the pinned readback area. */
+    /** `spare_bytes_k` after the plan and the alphabet of the pinned readback area. */
+    static constexpr std::size_t spare_bytes_k = 2 * direct_extents_parts_k * sizeof(direct_extents_t);
     std::uint64_t *spare_host() const noexcept {
         return reinterpret_cast<std::uint64_t *>(static_cast<unsigned char *>(readback.data) + sizeof(plan_bins_t) +
                                                  sizeof(batch_alphabet_t));
@@ -791,15 +792,25 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         args.wide = wide ? 1 : 0;
     }
 
-    // Cross products under unit costs: one thread per cell with the query's match masks shared by its CTA, without
-    // planning, when one side's strings are short enough. Device-resident results are written in place.
+    // Cross products under unit costs: one thread per cell with a pattern's match masks shared by its CTA, without
+    // planning, where that is the faster way (direct_rule.h). Device-resident results are written in place.
     if (engine.unit_levenshtein && !wide && call.mode == mode_cross_k && schedule != szs_gb300_schedule_plain_k && !defer) {
-        std::uint64_t *seen = context->spare_host();
+        auto *parts = reinterpret_cast<direct_extents_t *>(context->spare_host());
         SZS_TRY_CUDA(cudaEventRecord(context->start, stream));
-        SZS_TRY_CUDA(launch_direct_extents(args.queries, args.candidates, seen, stream));
+        SZS_TRY_CUDA(launch_direct_extents(args.queries, args.candidates, parts, stream));
         SZS_TRY_CUDA(cudaStreamSynchronize(stream));
-        bool swapped = false;
-        if (myers_direct_takes(seen[0], seen[2], args.pairs, swapped)) {
+        direct_extents_t seen[2] = {};
+        for (int side = 0; side < 2; ++side)
+            for (int part = 0; part < direct_extents_parts(side ? candidates_count : queries_count); ++part) {
+                direct_extents_t const &from = *parts++;
+                seen[side].longest = std::max(seen[side].longest, from.longest);
+                seen[side].symbols += from.symbols, seen[side].padded += from.padded, seen[side].words += from.words;
+                seen[side].words_two += from.words_two, seen[side].words_four += from.words_four;
+                seen[side].long_words += from.long_words;
+            }
+        direct_choice_t const choice = direct_choice(seen[0], queries_count, seen[1], candidates_count);
+        if (choice != direct_none_k) {
+            bool const swapped = choice == direct_candidates_k;
             bool const in_place = device_accessible(call.out);
             std::int64_t *target = call.out;
             if (!in_place) {
@@ -809,7 +820,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
                 target = static_cast<std::int64_t *>(context->work.data);
             }
             SZS_TRY_CUDA(cudaEventRecord(context->compute_start, stream));
-            SZS_TRY_CUDA(launch_myers_direct(args.queries, args.candidates, swapped, swapped ? seen[2] : seen[0], target,
+            SZS_TRY_CUDA(launch_myers_direct(args.queries, args.candidates, swapped, seen[swapped].longest, target,
                                              in_place ? call.stride : candidates_count, context->sm_count, stream));
             SZS_TRY_CUDA(cudaEventRecord(context->compute_stop, stream));
             auto *dense = static_cast<std::int64_t *>(context->results_host.data);
@@ -826,7 +837,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             cudaEventElapsedTime(&elapsed, context->start, context->stop);
             cudaEventElapsedTime(&compute, context->compute_start, context->compute_stop);
             stats.last_call_ms = elapsed, stats.last_compute_ms = compute;
-            stats.last_cells = seen[1] * seen[3]; // sum over cells of n x m
+            stats.last_cells = seen[0].symbols * seen[1].symbols; // sum over cells of n x m
             stats.last_launches = 2;
             stats.kernel_launches += 2;
             return {};

@@ -9,6 +9,7 @@
 
 #include <cuda_runtime.h>
 
+#include "direct_rule.h"
 #include "engine_types.cuh"
 #include "planner.cuh"
 
@@ -33,18 +34,15 @@ constexpr std::uint64_t small_max_rows_k = 1024;       // shorter sides: one wor
 /** Unit-cost Levenshtein of `count` packed pairs, one warp each, into `results` (device or page-locked host memory). */
 cudaError_t launch_myers_small(small_pair_t const *pairs, std::uint32_t count, std::uint8_t const *bytes,
                                std::int64_t *results, cudaStream_t stream);
-constexpr std::uint64_t direct_max_rows_k = 1024; // longest pattern of the direct cross-product kernels
-/** Fewest cells of a cross product for the direct kernels with patterns of 513 to 1,024 rows: one thread per cell takes
- *  about 0.33 ms for a pair of 1,000 bytes however few there are, where the warp-per-pair kernel spreads few pairs over
- *  more SMs (256 pairs 0.28 ms, 2,560 0.45 ms, 3,600 0.54 ms). */
-constexpr std::uint64_t direct_min_pairs_k = 1536;
-/** The longest string of both tapes and the sums of their lengths into `extents` (4 values in page-locked host memory:
- *  longest query, all queries, longest candidate, all candidates). */
-cudaError_t launch_direct_extents(tape_t const &queries, tape_t const &candidates, std::uint64_t *extents,
+constexpr int direct_extents_parts_k = 16; // parts of a tape that `launch_direct_extents` reads side by side, at most
+/** What `direct_choice` reads of both tapes: parts of the queries, then of the candidates, `direct_extents_parts(count)` of
+ *  each, into page-locked host memory. */
+cudaError_t launch_direct_extents(tape_t const &queries, tape_t const &candidates, direct_extents_t *extents,
                                   cudaStream_t stream);
-/** Whether the direct kernels take a unit-cost cross product with these longest strings; `swapped`: with the
- *  candidates as patterns. */
-bool myers_direct_takes(std::uint64_t longest_query, std::uint64_t longest_candidate, std::uint64_t pairs, bool &swapped);
+/** One CTA reads 8,192 strings' offsets in about the time of a launch. */
+inline int direct_extents_parts(std::uint64_t count) {
+    return (int)std::min<std::uint64_t>(count / 8192 + 1, direct_extents_parts_k);
+}
 /** Unit-cost Levenshtein over a cross product straight into `out` (row stride in elements), one thread per cell;
  *  `longest_rows` is the longest pattern (at most `direct_max_rows_k`). */
 cudaError_t launch_myers_direct(tape_t const &queries, tape_t const &candidates, bool swapped, std::uint64_t longest_rows,

@@ -1400,3 +1400,31 @@ def test_utf8_cut_sequences_add_no_code_points(szs, port, size):
     engine = szs.LevenshteinDistancesUTF8()
     got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
     np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_utf8_costs(), tape(first), tape(second)))
+
+
+@pytest.mark.parametrize("rows,columns,low,high,direct", [
+    (2000, 1, 1, 150, True), (1, 2000, 1, 150, True), (700, 7, 65, 300, True), (7, 700, 65, 300, True),
+    (33, 9000, 1, 20, True), (9000, 33, 1, 20, True), (2000, 5, 700, 1024, True), (5, 2000, 700, 1024, True),
+    (300, 31, 500, 1024, True), (70, 70, 8, 8, True), (1, 1, 1024, 1024, False), (31, 31, 1000, 1024, False),
+    (300, 300, 20, 2000, False), (40, 40, 900, 1020, False)])
+def test_cross_products_of_few_and_many_strings(szs, port, rows, columns, low, high, direct):
+    """Unit-cost cross products whose sides differ in count and length: either side as the patterns, few texts or many,
+    in both orders, into host and strided device matrices, and those that stay on the planned routes (the direct kernels
+    take two launches)."""
+    import torch
+    rng = np.random.default_rng(rows * 10007 + columns)
+    letters = np.arange(256, dtype=np.uint8) if rows % 2 else DNA
+    queries = random_strings(rng, rows, low, high, letters)
+    candidates = random_strings(rng, columns, low, high, letters)
+    candidates[0] = queries[0][:-1] + b"x"
+    want = port.cross(oracle.levenshtein_costs(), tape(queries), tape(candidates))
+    engine = szs.LevenshteinDistances()
+    np.testing.assert_array_equal(engine(szs.Strs(queries), szs.Strs(candidates)).astype(np.int64), want)
+    assert (engine.stats()["last_launches"] == 2) == direct
+    out = torch.full((rows, columns + 2), -1, dtype=torch.int64, device="cuda")
+    sides = [szs.Strs.from_buffers(*(torch.from_numpy(part.copy()).cuda() for part in (data, offsets.astype(np.int64))))
+             for data, offsets in (tape(queries), tape(candidates))]
+    engine(*sides, out=out)
+    got = out.cpu().numpy()
+    np.testing.assert_array_equal(got[:, :columns], want)
+    assert (got[:, columns:] == -1).all()

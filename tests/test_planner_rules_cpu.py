@@ -53,3 +53,81 @@ int main() {
 }
 """)
     assert not broken, broken[:5]
+
+
+def test_direct_cross_products_are_chosen_by_counts_and_lengths(tmp_path):
+    """The direct cross-product kernels: the side with more strings gives the texts, few strings on one side or the other
+    included; lengths that would leave a warp's threads waiting for its longest text, or a thread on a long chain, stay on
+    the planned routes; and no choice lies outside what the kernels take (patterns up to 1,024, 1,536 cells of patterns past
+    512)."""
+    broken = run_checks(tmp_path, r"""
+#include <cstdio>
+#include <vector>
+#include <cstdlib>
+#include "direct_rule.h"
+using namespace szs_gb300;
+using lengths_t = std::vector<std::uint64_t>;
+static direct_extents_t extents(lengths_t const &lengths) {
+    direct_extents_t e {};
+    for (std::size_t i = 0; i < lengths.size(); ++i) {
+        std::uint64_t group = 0;
+        for (std::size_t k = i / 32 * 32; k < i / 32 * 32 + 32 && k < lengths.size(); ++k) group = std::max(group, lengths[k]);
+        std::uint64_t const n = lengths[i], words = (n + 31) / 32;
+        e.longest = std::max(e.longest, n), e.symbols += n, e.padded += group, e.words += words;
+        e.words_two += (words + 1) / 2 * 2, e.words_four += (words + 3) / 4 * 4, e.long_words += n > 512 ? words : 0;
+    }
+    if (lengths.size() % 32) { // the last group's missing strings wait, too
+        std::uint64_t group = 0;
+        for (std::size_t k = lengths.size() / 32 * 32; k < lengths.size(); ++k) group = std::max(group, lengths[k]);
+        e.padded += (32 - lengths.size() % 32) * group;
+    }
+    return e;
+}
+static direct_choice_t choose(lengths_t const &q, lengths_t const &c) {
+    return direct_choice(extents(q), q.size(), extents(c), c.size());
+}
+static lengths_t same(std::size_t count, std::uint64_t length) { return lengths_t(count, length); }
+static lengths_t mixed(std::size_t count, std::uint64_t low, std::uint64_t high, int one_in) {
+    lengths_t lengths(count, low);
+    for (std::size_t i = 0; i < count; i += one_in) lengths[i] = high;
+    return lengths;
+}
+static void expect(char const *what, direct_choice_t got, direct_choice_t want) {
+    if (got != want) std::printf("%s: %d, not %d\n", what, (int)got, (int)want);
+}
+int main() {
+    expect("1,000,000 x 1 of 150", choose(same(1000000, 150), same(1, 150)), direct_candidates_k);
+    expect("1 x 1,000,000 of 150", choose(same(1, 150), same(1000000, 150)), direct_queries_k);
+    expect("100,000 x 8 of 150", choose(same(100000, 150), same(8, 150)), direct_candidates_k);
+    expect("20,000 x 16 of 800", choose(same(20000, 800), same(16, 800)), direct_candidates_k);
+    expect("16 x 20,000 of 800", choose(same(16, 800), same(20000, 800)), direct_queries_k);
+    expect("1,000,000 x 1 tokens", choose(same(1000000, 10), same(1, 10)), direct_candidates_k);
+    expect("2,048 x 2,048 tokens", choose(same(2048, 10), same(2048, 10)), direct_queries_k);
+    expect("197 x 198 of 1,000", choose(same(197, 1000), same(198, 1000)), direct_queries_k);
+    expect("2,048 of 8 x 2,048 of 512", choose(same(2048, 8), same(2048, 512)), direct_candidates_k);
+    expect("2,048 of 512 x 2,048 of 8", choose(same(2048, 512), same(2048, 8)), direct_queries_k);
+    expect("16 x 16 of 150", choose(same(16, 150), same(16, 150)), direct_queries_k);
+    expect("a few long ones", choose(mixed(1024, 20, 1000, 33), mixed(1024, 20, 1000, 33)), direct_none_k);
+    expect("20,000 of 150 x 40 of 20,000", choose(same(20000, 150), same(40, 20000)), direct_none_k);
+    expect("1 of 16 x 1 of 1,000,000", choose(same(1, 16), same(1, 1000000)), direct_none_k);
+    expect("40 x 40 of 1,000 x 5,000", choose(same(40, 1000), same(40, 5000)), direct_none_k);
+    expect("31 x 31 of 1,000", choose(same(31, 1000), same(31, 1000)), direct_none_k);
+    expect("2,000 of 1,025 x 2,000 of 1,025", choose(same(2000, 1025), same(2000, 1025)), direct_none_k);
+    expect("2,000 of 1,025 x 2,000 of 100", choose(same(2000, 1025), same(2000, 100)), direct_candidates_k);
+    std::srand(1);
+    for (int round = 0; round < 3000; ++round) {
+        lengths_t sides[2];
+        for (auto &side : sides) {
+            side.resize(1 + std::rand() % (round % 2 ? 40 : 900));
+            int const most = 1 + std::rand() % (round % 3 ? 600 : 2500);
+            for (auto &length : side) length = std::rand() % (most + 1);
+        }
+        direct_choice_t const choice = choose(sides[0], sides[1]);
+        if (choice == direct_none_k) continue;
+        std::uint64_t const rows = extents(sides[choice == direct_candidates_k]).longest;
+        if (rows > 1024 || (rows > 512 && sides[0].size() * sides[1].size() < 1536))
+            std::printf("%zu x %zu: patterns of %d\n", sides[0].size(), sides[1].size(), (int)rows);
+    }
+}
+""")
+    assert not broken, broken[:5]
