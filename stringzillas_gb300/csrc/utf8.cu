@@ -84,7 +84,10 @@ __device__ __forceinline__ bool warp_walk(tape_t const &tape, std::uint64_t begi
         std::uint32_t own = __funnelshift_r(a, b, 8 * skew);
         std::uint32_t const high = __funnelshift_r(b, c, 8 * skew); // read only where a sequence goes on
         std::uint32_t valid = 0x80808080u;
-        if (window + 128 > n) {
+        std::uint32_t outside = 0; // lane 31: which of the three bytes after this window lie past the string
+        if (window + 130 >= n) {
+            std::uint32_t const left = n - min(window + 128, n); // at most 2
+            outside = lane == 31 ? 0x00FFFFFFu << (8 * left) : 0u;
             int const keep = (int)n - (int)(window + 4 * lane); // this lane's bytes inside the string
             std::uint32_t const mask = keep >= 4 ? 0xFFFFFFFFu : (keep <= 0 ? 0u : 0xFFFFFFFFu >> (32 - 8 * keep));
             own &= mask, valid &= mask;
@@ -105,12 +108,10 @@ __device__ __forceinline__ bool warp_walk(tape_t const &tape, std::uint64_t begi
         std::uint32_t const two = own & (own << 1) & 0x80808080u, three = two & (own << 2), four = three & (own << 3);
         std::uint32_t const here = two << 8 | three << 16 | four << 24, beyond = two >> 24 | three >> 16 | four >> 8;
         std::uint32_t const above = __shfl_up_sync(0xFFFFFFFFu, beyond, 1);
-        bool const broken = (here | (lane ? above : asked)) != continuation;
+        bool const broken = (here | (lane ? above : asked)) != continuation || (beyond & outside);
         std::uint32_t const carried = __shfl_sync(0xFFFFFFFFu, beyond, 31);
         asked = lane ? 0u : carried;
-        std::uint32_t const left = n - min(window + 128, n); // the string's bytes after this window
-        bool const cut = left < 3 && carried >> (8 * left);
-        if (__any_sync(0xFFFFFFFFu, broken || cut)) return false;
+        if (__any_sync(0xFFFFFFFFu, broken)) return false;
         std::uint32_t const leads = (((valid & ~continuation) >> 7) * 0x01020408u) >> 24; // four bits
         // The window's code points in order: their positions, so that lane k takes the k-th.
         std::uint32_t const found = __popc(leads);
