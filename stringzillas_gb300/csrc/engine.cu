@@ -10,6 +10,7 @@
  */
 #include "stringzillas_gb300.h"
 #include "launchers.h"
+#include "small_rule.h"
 
 #include <cuda_runtime.h>
 
@@ -1848,21 +1849,31 @@ static status_t run_pipelined(engine_t const &engine, device_context_t *context,
 /**
  *  Small pairwise calls of unit-cost Levenshtein whose strings are in host memory: packed into one page-locked buffer (the
  *  pairs' records, then their strings), copied once and scored by one kernel that writes the results to page-locked
- *  memory. @p taken is false when a pair's shorter side is too long for it. 64 pairs of reads of 64-256 bytes take 59 us
- *  this way against 133 us planned (two planning phases, seven launches on forked streams, six copies).
+ *  memory. @p taken is false when a pair's shorter side is too long for it, or the planned routes are faster
+ *  (small_rule.h). 64 pairs of reads of 64-256 bytes take 55 us this way against 143 us planned (two planning phases,
+ *  seven launches on forked streams, six copies).
  */
 static status_t run_small(device_context_t *context, cudaStream_t stream, call_t const &call, szs_gb300_stats_t &stats,
                           bool &taken) noexcept {
     tape_view_t const &first = call.queries, &second = call.candidates;
     std::size_t const count = first.count;
     std::uint64_t cells = 0;
-    for (std::size_t i = 0; i < count; ++i) {
-        std::uint64_t const a_begin = host_offset(first, i), a_end = host_offset(first, i + 1);
-        std::uint64_t const b_begin = host_offset(second, i), b_end = host_offset(second, i + 1);
-        if (a_end < a_begin || b_end < b_begin) return {};
-        if (std::min(a_end - a_begin, b_end - b_begin) > small_max_rows_k) return {};
-        cells += (a_end - a_begin) * (b_end - b_begin);
-    }
+    small_estimate_t estimate;
+    bool fits = true;
+    auto scan = [&](auto const *a, auto const *b) {
+        for (std::size_t i = 0; i < count; ++i) {
+            std::uint64_t const a_begin = a[i], a_end = a[i + 1], b_begin = b[i], b_end = b[i + 1];
+            std::uint64_t const a_length = a_end - a_begin, b_length = b_end - b_begin;
+            std::uint64_t const shorter = std::min(a_length, b_length), longer = std::max(a_length, b_length);
+            fits &= a_end >= a_begin && b_end >= b_begin && shorter <= small_max_rows_k;
+            estimate.add(shorter, shorter ? longer : 0);
+            cells += shorter * longer;
+        }
+    };
+    if (first.offset_bits == 32)
+        scan(static_cast<std::uint32_t const *>(first.offsets), static_cast<std::uint32_t const *>(second.offsets));
+    else scan(static_cast<std::uint64_t const *>(first.offsets), static_cast<std::uint64_t const *>(second.offsets));
+    if (!fits || !estimate.pays()) return {};
     std::uint64_t const a_first = host_offset(first, 0), a_bytes = host_offset(first, count) - a_first;
     std::uint64_t const b_first = host_offset(second, 0), b_bytes = host_offset(second, count) - b_first;
     std::size_t const bytes_at = align_up(count * sizeof(small_pair_t), 256);

@@ -1428,3 +1428,19 @@ def test_cross_products_of_few_and_many_strings(szs, port, rows, columns, low, h
     got = out.cpu().numpy()
     np.testing.assert_array_equal(got[:, :columns], want)
     assert (got[:, columns:] == -1).all()
+
+
+@pytest.mark.parametrize("count,rows,cols,one_kernel", [
+    (1, 16, 60000, False), (60, 32, 9000, False), (2, 100, 50000, False), (500, 20, 1500, False),
+    (64, 200, 5000, True), (100, 60, 1000, True), (1, 1000, 20000, False), (40, 600, 900, True)])
+def test_small_host_calls_with_long_texts(szs, port, count, rows, cols, one_kernel):
+    """Few pairs from host memory whose texts are long: short patterns go to the planned routes, longer ones and short
+    texts keep the one-kernel path (one launch)."""
+    rng = np.random.default_rng(rows + cols)
+    first = [bytes(rng.choice(DNA, size=rows)) for _ in range(count)]
+    second = [bytes(rng.choice(DNA, size=cols)) for _ in range(count)]
+    first[0], second[0] = second[0], first[0]
+    engine = szs.LevenshteinDistances()
+    got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
+    np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_costs(), tape(first), tape(second)))
+    assert (engine.stats()["last_launches"] == 1) == one_kernel

@@ -131,3 +131,38 @@ int main() {
 }
 """)
     assert not broken, broken[:5]
+
+
+def test_small_host_calls_are_chosen_by_their_chains(tmp_path):
+    """Few pairs from host memory take the one-kernel path unless a long text beside a short pattern, or many warps, take
+    longer there than on the planned routes; the estimate only grows with a call's pairs and lengths."""
+    broken = run_checks(tmp_path, r"""
+#include <cstdio>
+#include "small_rule.h"
+using namespace szs_gb300;
+static bool pays(int count, std::uint64_t rows, std::uint64_t cols) {
+    small_estimate_t estimate;
+    for (int i = 0; i < count; ++i) estimate.add(rows, cols);
+    return estimate.pays();
+}
+static void expect(int count, std::uint64_t rows, std::uint64_t cols, bool want) {
+    if (pays(count, rows, cols) != want)
+        std::printf("%d x (%llu, %llu): not %d\n", count, (unsigned long long)rows, (unsigned long long)cols, (int)want);
+}
+int main() {
+    expect(64, 160, 256, true), expect(1, 1, 1, true), expect(2048, 16, 16, true);
+    expect(2048, 200, 200, true), expect(100, 60, 1200, true), expect(64, 200, 5000, true), expect(512, 1000, 1000, true);
+    expect(1, 16, 1000000, false), expect(64, 32, 10000, false), expect(4, 100, 200000, false);
+    expect(2048, 8, 500, false), expect(2048, 300, 500, false), expect(500, 20, 1500, false);
+    for (int rows : {1, 33, 100, 250})
+        for (int count : {1, 2048}) {
+            bool last = true;
+            for (std::uint64_t cols = rows; cols < (1u << 20); cols += 1 + cols / 8) {
+                bool const now = pays(count, rows, cols);
+                if (now && !last) std::printf("%d x (%d, %d): pays again\n", count, rows, (int)cols);
+                last = now;
+            }
+        }
+}
+""")
+    assert not broken, broken[:5]
