@@ -58,17 +58,19 @@ struct short_policy_t {
     static constexpr int rows_per_lane_k = rows_per_lane_;
     static constexpr int segment_rows_k = lanes_ * rows_per_lane_;
     static constexpr int segments_k = warp_size_k / lanes_;
-    static constexpr bool compare_k = compare_ != compare_none_k;
+    static constexpr bool row_maxima_k = compare_ == short_row_maxima_k; // local scores with positive gap costs
+    static constexpr bool compare_k = compare_ != compare_none_k && !row_maxima_k;
     static constexpr bool multiply_k = compare_ == compare_multiply_k;
     // Four warps per scheduler in 128 registers; 8 rows, and 12 of local scores, leave room for five in 96; three tracks of
     // 24 or 28 rows (H, E and the codes) take three in 168.
-    static constexpr int ctas_per_sm_k = rows_per_lane_ == 8 || (rows_per_lane_ == 12 && local_k) ? 5
-                                         : compare_k && affine_ && rows_per_lane_ >= 24           ? 3
-                                                                                                  : 4;
+    static constexpr int ctas_per_sm_k = rows_per_lane_ == 8 || (rows_per_lane_ == 12 && local_k && !row_maxima_k) ? 5
+                                         : compare_k && affine_ && rows_per_lane_ >= 24                            ? 3
+                                                                                                                   : 4;
     static_assert(lanes_ == 1 || lanes_ == 2 || lanes_ == 4 || lanes_ == 8 || lanes_ == 16, "segments of 1 to 16 lanes");
     static_assert(rows_per_lane_ % 4 == 0, "profile rows are read in 4-byte words");
     static_assert(segment_rows_k <= short_max_rows_k, "a pair's whole column fits one strip");
     static_assert(!compare_k || kind_ == kind_levenshtein_k, "only Levenshtein costs are a function of equality");
+    static_assert(!row_maxima_k || local_k, "only local scores are maxima over all cells");
 };
 
 /** Per-warp shared profile bytes: segments x two pairs x classes x segment rows (none in compare mode). */
@@ -196,10 +198,11 @@ __device__ __forceinline__ void short_score_segment(pair_task_t const &a, bool a
     std::uint32_t h_col[R], e_col[R];
     // Local scores: running maxima over every cell, filler rows included. A filler row (past its pair's last) costs
     // -128 against every column: its cells take their values from gaps out of the rows above and from diagonals that
-    // lose `-open` at least, never above the cells they come from, as long as gap costs are not positive (the planner
-    // keeps local calls with positive ones off this kernel). So no row needs a maximum of its own: one three-way
-    // maximum takes two cells.
-    std::uint32_t best[2] = {0u, 0u};
+    // lose `-open` at least, never above the cells they come from, as long as gap costs are not positive. So no row needs
+    // a maximum of its own: one three-way maximum takes two cells. With positive gap costs (`row_maxima_k`) a filler cell
+    // may exceed the real ones, so each row keeps its own and the filler rows' are left out at the end.
+    constexpr bool row_maxima = policy_::row_maxima_k;
+    std::uint32_t best[row_maxima ? R : 2] = {};
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         std::int32_t const h = edge.score(row0 + r) + h_shift;
@@ -308,8 +311,12 @@ __device__ __forceinline__ void short_score_segment(pair_task_t const &a, bool a
             if constexpr (local) {
                 if constexpr (steady) {
 #pragma unroll
-                    for (int r = 0; r < R; r += 2)
-                        best[r / 2 % 2] = __vimax3_s16x2(best[r / 2 % 2], cell_h[r], cell_h[r + 1]);
+                    for (int r = 0; r < R; r += 2) {
+                        if constexpr (row_maxima)
+                            best[r] = __vimax3_s16x2(best[r], cell_h[r], 0u),
+                            best[r + 1] = __vimax3_s16x2(best[r + 1], cell_h[r + 1], 0u);
+                        else best[r / 2 % 2] = __vimax3_s16x2(best[r / 2 % 2], cell_h[r], cell_h[r + 1]);
+                    }
                 }
                 else {
                     // Columns past one pair's end carry filler in that half: masked out of the maxima (H >= 0).
@@ -317,8 +324,12 @@ __device__ __forceinline__ void short_score_segment(pair_task_t const &a, bool a
                                                                : ((j <= (int)m_a ? 0x0000FFFFu : 0u) |
                                                                   (j <= (int)m_b ? 0xFFFF0000u : 0u));
 #pragma unroll
-                    for (int r = 0; r < R; r += 2)
-                        best[r / 2 % 2] = __vimax3_s16x2(best[r / 2 % 2], cell_h[r] & mask, cell_h[r + 1] & mask);
+                    for (int r = 0; r < R; r += 2) {
+                        std::uint32_t const even = cell_h[r] & mask, odd = cell_h[r + 1] & mask;
+                        if constexpr (row_maxima)
+                            best[r] = __vimax3_s16x2(best[r], even, 0u), best[r + 1] = __vimax3_s16x2(best[r + 1], odd, 0u);
+                        else best[r / 2 % 2] = __vimax3_s16x2(best[r / 2 % 2], even, odd);
+                    }
                 }
             }
             else if constexpr (!steady) {
@@ -347,7 +358,16 @@ __device__ __forceinline__ void short_score_segment(pair_task_t const &a, bool a
     for (; t < warp_steps; ++t) step(t, std::false_type {});
 
     if constexpr (local) {
-        std::uint32_t lane_best = __vimax3_s16x2(best[0], best[1], 0u);
+        std::uint32_t lane_best = 0;
+        if constexpr (row_maxima) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                std::uint32_t const keep = ((row0 + r <= (std::int64_t)n_a) ? 0x0000FFFFu : 0u) |
+                                           ((row0 + r <= (std::int64_t)n_b) ? 0xFFFF0000u : 0u);
+                lane_best = __vimax3_s16x2(lane_best, best[r] & keep, 0u);
+            }
+        }
+        else lane_best = __vimax3_s16x2(best[0], best[1], 0u);
 #pragma unroll
         for (int offset = L / 2; offset > 0; offset >>= 1)
             lane_best = __vimax3_s16x2(lane_best, __shfl_xor_sync(0xFFFFFFFFu, lane_best, offset), 0u);

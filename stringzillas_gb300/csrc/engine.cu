@@ -876,9 +876,14 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
     args.short_max_rows = engine.tuning.short_max_rows
                               ? std::min<std::uint32_t>(engine.tuning.short_max_rows, (std::uint32_t)short_max_rows_k)
                               : (std::uint32_t)short_max_rows_k;
-    // The short kernel's running maxima count on gaps that cost something (dp_short.cuh).
-    if (engine.kind == kind_smith_waterman_k && engine.local_gain < 0) args.short_max_rows = 0;
     args.short_fine = args.pairs >= short_fine_pairs_k && args.packed_allowed && !args.unit_levenshtein ? 1 : 0;
+    // Local scores with positive gap costs take the short kernel's form with a maximum per row, in halves of octaves; in
+    // small batches the wavefront's fewer launches win (DNA pairs of 16-128, short kernel / wavefront: 8,192 143 / 132 us,
+    // 16,384 146 / 170, 262,144 560 / 1,220).
+    bool const short_row_maxima = engine.kind == kind_smith_waterman_k && engine.local_gain < 0;
+    if (short_row_maxima) args.short_fine = 0;
+    if (short_row_maxima && args.pairs < short_row_maxima_pairs_k && schedule != szs_gb300_schedule_plain_k)
+        args.short_max_rows = 0;
     args.classes = costs.classes;
     // A batched call with fewer pairs than one wave of the 16x2 route (two pairs per warp, about 16 resident warps
     // per SM) would leave SMs idle on the wavefront: its longer pairs spread over a band CTA's warps instead.
@@ -1257,15 +1262,16 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         scratch_total += bytes;
     }
     // Short pairs: one job per segment shape, most rows first.
+    int const short_mode = short_row_maxima ? short_row_maxima_k : compare_mode;
     for (int shape_index = short_shapes_k - 1; shape_index >= 0; --shape_index) {
         int const key_begin = bin_short_begin_k + shape_index * short_m_classes_k;
         int const key_end = key_begin + short_m_classes_k;
         std::uint64_t const pairs_here = pairs_in(key_begin, key_end);
         if (!pairs_here) continue;
         int const warps = 4;
-        int const rows = short_rows_for(packed_costs.classes, compare_mode, shape_index, pairs_here, context->sm_count);
+        int const rows = short_rows_for(packed_costs.classes, short_mode, shape_index, pairs_here, context->sm_count);
         dp_launch_shape_t const shape =
-            short_shape(engine.kind, costs.affine != 0, shape_index, rows, packed_costs.classes, warps, compare_mode);
+            short_shape(engine.kind, costs.affine != 0, shape_index, rows, packed_costs.classes, warps, short_mode);
         if (shape.ctas_per_sm <= 0) return {sz_status_unknown_k, "Short-pair kernel cannot be resident"};
         std::uint64_t const lanes = (std::uint64_t)(short_segment_rows(shape_index) / rows);
         std::uint64_t const per_warp = 2u * (32u / lanes); // pairs per warp
@@ -1411,6 +1417,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         key_append(launch_key, near_list_at);
         key_append(launch_key, schedule), key_append(launch_key, lanes_used);
         key_append(launch_key, engine.kind), key_append(launch_key, compare_mode), key_append(launch_key, tilted);
+        key_append(launch_key, short_mode);
     }
     auto issue_jobs = [&](cudaStream_t s) -> status_t {
         SZS_TRY_CUDA(cudaEventRecord(context->fork, s));
@@ -1462,7 +1469,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             else if (job.kind == job_short_k)
                 SZS_TRY_CUDA(launch_short(engine.kind, costs.affine != 0, job.variant, job.rows, job.key_begin,
                                           job.key_end, tasks, bins, packed_costs, results, job.ctas, job.warps,
-                                          lane_stream, compare_mode));
+                                          lane_stream, short_mode));
             else if (job.kind == job_near_k) {
                 SZS_TRY_CUDA(launch_myers_near(job.variant, myers_planes, tasks, bins, job.key_begin, job.key_end, alphabet,
                                                results, near_list, job.ctas, lane_stream));

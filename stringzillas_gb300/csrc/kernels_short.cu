@@ -82,7 +82,20 @@ cudaError_t short_launch_of(int key_begin, int key_end, pair_task_t const *tasks
     break;
 #endif
 
+#if SZS_SHORT_ROWS > 16
+#define SZS_SHORT_ROW_MAXIMA(call_, ...) break; // up to 128 rows in halves of octaves only
+#else
+#define SZS_SHORT_ROW_MAXIMA(call_, ...)                                                                             \
+    if (kind != kind_smith_waterman_k) break;                                                                        \
+    if (affine) SZS_SHORT_LANES(call_, kind_smith_waterman_k, true, short_row_maxima_k, __VA_ARGS__)                 \
+    else SZS_SHORT_LANES(call_, kind_smith_waterman_k, false, short_row_maxima_k, __VA_ARGS__)                       \
+    break;
+#endif
+
 #define SZS_SHORT_DISPATCH(call_, ...)                                                                               \
+    if (compare == short_row_maxima_k) {                                                                             \
+        SZS_SHORT_ROW_MAXIMA(call_, __VA_ARGS__)                                                                     \
+    }                                                                                                                \
     if (compare != compare_none_k) {                                                                                 \
         SZS_SHORT_COMPARE(call_, __VA_ARGS__)                                                                        \
     }                                                                                                                \
@@ -134,10 +147,11 @@ SZS_SHORT_DECLARE(24)
 SZS_SHORT_DECLARE(28)
 
 int short_rows_for(int classes, int compare, int shape, std::uint64_t pairs, int sm_count) {
-    bool const few = compare != compare_none_k || classes <= short_few_classes_k;
+    bool const row_maxima = compare == short_row_maxima_k;
+    bool const few = (compare != compare_none_k && !row_maxima) || classes <= short_few_classes_k;
     int const quarter = shape == 0 ? 3 : (shape - 1) % 4;
     if (quarter == 3) return few ? 16 : 8;
-    if (!few) return 12;
+    if (!few || row_maxima) return 12;
     // The 6/4 shapes up to 16 lanes have a second form of half the rows in twice the lanes, whose steps are half as
     // long: where the pairs leave warp slots free, a warp's own chain of steps is what takes the time.
     int const lanes = short_segment_rows(shape) / 24;

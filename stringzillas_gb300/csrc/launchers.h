@@ -190,10 +190,11 @@ cudaError_t launch_band16(int kind, bool affine, int key_begin, int key_end, pai
                           std::size_t ring_words_per_slot, int ctas, cudaStream_t stream, void *group_states = nullptr,
                           int group_ctas = 1, int compare = 0, bool wide = false, int rows_per_lane = 8);
 
-/** Short pairs (shorter side at most 256) on the segmented 16x2 kernel: `shape` 0-16 by the rows a segment holds
- *  (`short_segment_rows`) with `rows` per lane as `short_rows_for` gives them for so many pairs (profiles over more
- *  than `short_few_classes_k` classes: shapes of 16, 24, 32, 48, 64, 96 and 128 rows only); `compare` as for the 16x2
- *  wavefront (Levenshtein only). */
+/** Short pairs (shorter side at most 448) on the segmented 16x2 kernel: `shape` 0-19 by the rows a segment holds
+ *  (`short_segment_rows`) with `rows` per lane as `short_rows_for` gives them for so many pairs. Profiles over more than
+ *  `short_few_classes_k` classes take the shapes in halves of octaves only, up to 128 rows or 192 in large batches.
+ *  `compare` as for the 16x2 wavefront (Levenshtein only), or `short_row_maxima_k` for local scores with positive gap
+ *  costs, in halves of octaves up to 128 rows. */
 int short_rows_for(int classes, int compare, int shape, std::uint64_t pairs, int sm_count);
 dp_launch_shape_t short_shape(int kind, bool affine, int shape, int rows, int classes, int warps, int compare = 0);
 cudaError_t launch_short(int kind, bool affine, int shape, int rows, int key_begin, int key_end,

@@ -65,6 +65,8 @@ constexpr int short_m_classes_k = 27;  // text-length classes per shape
 constexpr int short_max_rows_k = 448;  // default: shorter sides up to this take the short route (large batches)
 constexpr int short_few_rows_k = 128;  // the same for smaller batches and the plain form
 constexpr int short_profile_rows_k = 192; // the same for large batches whose profile has many classes
+constexpr int short_row_maxima_k = 3;  // beside the compare modes: local scores with positive gap costs (dp_short.cuh)
+constexpr std::uint64_t short_row_maxima_pairs_k = 12288; // pairs from which those take the short route
 constexpr int short_few_classes_k = 8; // profiles over at most this many classes fit segments of 16-28 rows per lane
 /** Pairs, and cells by the mean lengths, from which a call cuts its short pairs' rows in quarter octaves instead of
  *  halves and takes longer ones: 655e6 cells of text pairs of 100-300 took 334 us either way (340 here), 800e6 384 -> 370

@@ -1444,3 +1444,25 @@ def test_small_host_calls_with_long_texts(szs, port, count, rows, cols, one_kern
     got = engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64)
     np.testing.assert_array_equal(got, port.pairs(oracle.levenshtein_costs(), tape(first), tape(second)))
     assert (engine.stats()["last_launches"] == 1) == one_kernel
+
+
+@pytest.mark.parametrize("gaps", [(1, 2), (1, 1), (3, -1), (-2, 1)])
+@pytest.mark.parametrize("letters", [4, 20])
+def test_short_local_pairs_with_positive_gap_costs(szs, port, gaps, letters):
+    """Local scores whose gaps may gain: the short kernel keeps a maximum per row and leaves out the rows past a pair's
+    end, whose cells may exceed the real ones. Both sides of every shape's limit, uneven partners of one segment, few and
+    many classes, both schedules, and a batch small enough for the wavefront."""
+    rng = np.random.default_rng(zlib_seed(gaps, letters))
+    alphabet = DNA if letters == 4 else PROTEIN
+    b2c, table = dna_tables() if letters == 4 else protein_tables(rng, symmetric=False)
+    edges = [(n, m) for e in (16, 24, 32, 48, 64, 96, 128) for n in (e - 1, e, e + 1) for m in (1, e, 2 * e + 5)]
+    edges += [(0, 30), (30, 0), (0, 0), (20, 900), (129, 140)]
+    lengths = edges + [tuple(pair) for pair in rng.integers(1, 140, size=(13000 - len(edges), 2))]
+    first = [bytes(rng.choice(alphabet, size=n)) for n, _ in lengths]
+    second = [bytes(rng.choice(alphabet, size=m)) for _, m in lengths]
+    engine, oracle_costs = make_engine(szs, "sw", gaps, b2c, table)
+    want = port.pairs(oracle_costs, tape(first), tape(second))
+    for count, schedule in ((len(first), "batched"), (300, "batched"), (300, "plain")):
+        engine.set_schedule(schedule)
+        got = engine.pairwise(szs.Strs(first[:count]), szs.Strs(second[:count])).astype(np.int64)
+        np.testing.assert_array_equal(got, want[:count])
