@@ -48,24 +48,36 @@ __device__ __forceinline__ std::int64_t trivial_score(plan_args_t const &args, s
     return length == 0 ? 0 : (std::int64_t)args.open + (std::int64_t)args.extend * (std::int64_t)(length - 1);
 }
 
-/** Symbols of a whole tape (bytes, where strings are transcoded in place). */
-__device__ __forceinline__ std::uint64_t tape_symbols(tape_t const &tape) {
-    if (tape.offset_bits == 32) {
-        auto const *offsets = static_cast<std::uint32_t const *>(tape.offsets);
-        return offsets[tape.count] - offsets[0];
-    }
-    auto const *offsets = static_cast<std::uint64_t const *>(tape.offsets);
-    return offsets[tape.count] - offsets[0];
+/** Whether a profile over the call's symbols fits the 16x2 kernels' 32 classes, and over how many (`few`: codes are compared,
+ *  or the classes are few enough for long segments). */
+__device__ __forceinline__ bool profile_classes(plan_args_t const &args, bool &few) {
+    bool const fits = (args.kind != kind_levenshtein_k && !args.dense) || (args.alphabet && args.alphabet->symbols <= 32);
+    few = !fits || (args.alphabet ? (int)args.alphabet->symbols : args.classes) <= short_few_classes_k;
+    return fits;
 }
 
-/** Whether a call's pairs are many and long enough, by the means of their lengths, to fill the device in each of the
- *  short route's twenty shapes. */
+/** Whether a call's pairs are many and long enough to fill the device in each of the short route's twenty shapes, by 32 of
+ *  them (`short_fine_cells_k`, and over few classes `short_fine_rows`). One warp, the same in every CTA. */
 __device__ __forceinline__ bool short_fine_batch(plan_args_t const &args) {
     if (!args.short_fine) return false;
     tape_t const &second = args.mode == mode_symmetric_k ? args.queries : args.candidates;
-    float const cells = (float)args.pairs * ((float)tape_symbols(args.queries) / (float)args.queries.count) *
-                        ((float)tape_symbols(second) / (float)second.count);
-    return cells >= short_fine_cells_k;
+    std::uint64_t q, c;
+    pair_indices(args, (threadIdx.x & 31u) * (args.pairs >> 5), q, c);
+    std::uint8_t const *start;
+    std::uint64_t first_length, second_length;
+    tape_string(args.queries, q, start, first_length, args.wide);
+    tape_string(second, c, start, second_length, args.wide);
+    bool few;
+    bool const profile = profile_classes(args, few);
+    float rows = (float)min(first_length, second_length), columns = (float)max(first_length, second_length);
+#pragma unroll
+    for (int distance = 16; distance; distance >>= 1) {
+        rows += __shfl_xor_sync(0xFFFFFFFFu, rows, distance);
+        columns += __shfl_xor_sync(0xFFFFFFFFu, columns, distance);
+    }
+    rows /= 32.0f, columns /= 32.0f;
+    float const pairs = (float)args.pairs;
+    return pairs * rows * columns >= short_fine_cells_k && (!few || pairs * rows >= short_fine_rows(rows, columns, profile));
 }
 
 struct pair_route_info_t {
@@ -134,8 +146,8 @@ __device__ __forceinline__ pair_route_info_t route_pair(plan_args_t const &args,
     // The 16x2 routes hold costs in a 32-class profile: dense-table calls over more bytes than that stay on the
     // 32-bit routes. Levenshtein calls over more bytes, or over 16-bit codes, take them in compare mode (codes
     // compared, no profile).
-    bool const profile_fits = (args.kind != kind_levenshtein_k && !args.dense) ||
-                              (args.alphabet && args.alphabet->symbols <= 32);
+    bool few;
+    bool const profile_fits = profile_classes(args, few);
     bool const compare_fits = args.kind == kind_levenshtein_k && (args.alphabet != nullptr || args.wide);
     // A tuned cell width: 32 keeps the class off 16-bit cells, 64 puts it on the 64-bit wavefront (the route the
     // reach bound takes for spans near 2^31 / magnitude, reachable on any pair this way).
@@ -152,9 +164,7 @@ __device__ __forceinline__ pair_route_info_t route_pair(plan_args_t const &args,
     // Short pairs: a few lanes per pair instead of a warp (dp_short.cuh).
     if (packed && !args.wide && n <= args.short_max_rows) {
         bool const plain = args.force_route >= 0;
-        int const classes = args.alphabet ? (int)args.alphabet->symbols : args.classes;
-        bool const few = !profile_fits || classes <= short_few_classes_k, large = !plain && short_fine;
-        bool const fine = few && large;
+        bool const large = !plain && short_fine, fine = few && large;
         if (plain && n <= short_few_rows_k) {
             info.key = bin_short_begin_k + 12 * short_m_classes_k; // plain form: one bin (128-row segments), input order
             return info;
@@ -255,9 +265,10 @@ __global__ void plan_count_kernel(plan_args_t const args, plan_bins_t *__restric
     __shared__ bool short_fine;
     for (int i = threadIdx.x; i < bin_keys_k; i += blockDim.x) histogram[i] = 0;
     if (threadIdx.x == 0)
-        block_cells = 0, block_max_cols = 0, block_max_myers = 0, block_max_myers_warp = 0, block_max_chain = 0,
-        short_fine = short_fine_batch(args);
+        block_cells = 0, block_max_cols = 0, block_max_myers = 0, block_max_myers_warp = 0, block_max_chain = 0;
+    if (threadIdx.x < 32) short_fine = short_fine_batch(args);
     __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) bins->short_fine = short_fine;
     std::uint64_t thread_cells = 0;
     std::uint32_t thread_max_cols = 0, thread_max_myers = 0, thread_max_myers_warp = 0, thread_max_chain = 0;
     int const lane = threadIdx.x & 31;
@@ -385,13 +396,12 @@ __global__ void plan_scatter_kernel(plan_args_t const args, plan_bins_t *__restr
                                     pair_task_t *__restrict__ tasks) {
     __shared__ std::uint32_t counts[bin_keys_k];
     __shared__ std::uint32_t bases[bin_keys_k];
-    __shared__ bool short_fine;
+    bool const short_fine = bins->short_fine != 0; // as the first pass found
     int const lane = threadIdx.x & 31;
     std::uint64_t const per_block = (args.pairs + gridDim.x - 1) / gridDim.x;
     std::uint64_t const begin = min(args.pairs, (std::uint64_t)blockIdx.x * per_block);
     std::uint64_t const end = min(args.pairs, begin + per_block);
     for (int i = threadIdx.x; i < bin_keys_k; i += blockDim.x) counts[i] = 0;
-    if (threadIdx.x == 0) short_fine = short_fine_batch(args);
     __syncthreads();
     // A warp's lanes that share a bin: one shared-memory atomic for all of them; returns this lane's rank.
     auto claim = [&](unsigned key) -> std::uint32_t {

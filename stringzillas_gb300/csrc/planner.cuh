@@ -68,11 +68,23 @@ constexpr int short_profile_rows_k = 192; // the same for large batches whose pr
 constexpr int short_row_maxima_k = 3;  // beside the compare modes: local scores with positive gap costs (dp_short.cuh)
 constexpr std::uint64_t short_row_maxima_pairs_k = 12288; // pairs from which those take the short route
 constexpr int short_few_classes_k = 8; // profiles over at most this many classes fit segments of 16-28 rows per lane
-/** Pairs, and cells by the mean lengths, from which a call cuts its short pairs' rows in quarter octaves instead of
+/** Pairs, and cells by the mean sides of 32 of them, from which a call cuts its short pairs' rows in quarter octaves instead of
  *  halves and takes longer ones: 655e6 cells of text pairs of 100-300 took 334 us either way (340 here), 800e6 384 -> 370
  *  and 1.3e9 573 -> 515; 340e6 cells of DNA pairs of 16-128 226 -> 263. */
 constexpr std::uint64_t short_fine_pairs_k = 1 << 14;
 constexpr float short_fine_cells_k = 800e6f;
+/** Rows of all pairs together that such a call needs besides, by the means of the shorter and the longer sides: a warp
+ *  holds some 1,500 rows in quarter octaves, half as many in halves, and a call of few warps, spread over many shapes, takes
+ *  its longest chains. Fitted to calls of 5,000 to 250,000 pairs in either form (DNA profiles / compared text, halves ->
+ *  quarters): 45,000 pairs of 30 x 600 500 -> 1,170 us / 505 -> 538, 250,000 1,680 -> 1,700 / 1,750 -> 1,590; 20,000 pairs
+ *  of 100-300 on either side 407 -> 573 / 390 -> 400, 45,000 753 -> 672 / 722 -> 607; 65,536 of 40-200 476 -> 523 / 448 ->
+ *  415, 100,000 640 -> 576 / 608 -> 543; 150,000 of 16-128 374 -> 402 / 370 -> 389. */
+__host__ __device__ inline float short_fine_rows(float rows, float columns, bool profile) {
+    bool const uneven = columns > 1.3f * rows;
+    if (!profile) return 6.2e6f - 1.3e4f * rows;
+    if (uneven) return rows < 56.0f ? 1.5e7f : 1.0e7f - 2.7e4f * rows;
+    return 8.0e6f - 1.2e4f * rows;
+}
 static_assert(bin_short_begin_k + short_shapes_k * short_m_classes_k <= bin_keys_k, "bin layout exceeds the key space");
 constexpr int bin_myers_chain_k = bin_short_begin_k + short_shapes_k * short_m_classes_k; // 2028
 /** Rows of a segment of one shape, on the host and on the device. */
@@ -171,7 +183,7 @@ struct plan_bins_t {
     std::uint32_t max_chain_rows;      // longest pattern on the chained bit-parallel route
     std::uint32_t near_tried, near_failed; // pairs the near-diagonal kernel has tried, and those it had to list
     std::uint32_t near_sampled, near_alike; // pairs the planner sampled for likeness, and those found alike
-    std::uint32_t reserved;
+    std::uint32_t short_fine;              // whether short pairs are cut in quarter octaves (`short_fine_rows`)
     std::uint32_t listed[32];              // pairs it listed per class of full kernel (words; 16 + words per lane)
 };
 

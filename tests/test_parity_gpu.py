@@ -1466,3 +1466,36 @@ def test_short_local_pairs_with_positive_gap_costs(szs, port, gaps, letters):
         engine.set_schedule(schedule)
         got = engine.pairwise(szs.Strs(first[:count]), szs.Strs(second[:count])).astype(np.int64)
         np.testing.assert_array_equal(got, want[:count])
+
+
+@pytest.mark.parametrize("name,family,costs,letters", [
+    ("lev-linear", "lev", (0, 3, 2, 2), 4), ("lev-affine", "lev", (0, 4, 5, 2), 8), ("multiply", "lev", (0, 2, 3, 1), 256),
+    ("select", "lev", (0, 5, 3, 1), 256), ("compare-linear", "lev", (3, 1, 5, 5), 256), ("nw-linear", "nw", (-5, -5), 4),
+    ("nw-affine", "nw", (-11, -1), 4), ("sw-linear", "sw", (-5, -5), 4), ("sw-affine", "sw", (-5, -2), 4),
+    ("sw-free-gaps", "sw", (0, 0), 4)])
+def test_short_pairs_in_quarter_octaves(szs, port, name, family, costs, letters):
+    """Batches with rows enough for quarter octaves over few classes, or comparing codes (`short_fine_rows`): every shape up
+    to 448 rows takes a launch, both sides of every shape's limit, texts from one character to thousands, uneven partners of
+    one segment. The same pairs in a batch of a third, which stays with halves of octaves."""
+    rng = np.random.default_rng(zlib_seed(name))
+    alphabet = DNA if letters == 4 else np.arange(letters, dtype=np.uint8)
+    b2c, table = dna_tables()
+    edges = [16] + [(16 << k) * q // 4 for k in range(5) for q in (5, 6, 7, 8)][:19]
+    lengths = [(n, m) for e in edges for n in (e - 1, e, e + 1) for m in (1, e, e + 17, 2 * e + 5)]
+    lengths += [(0, 300), (300, 0), (0, 0), (20, 3000), (200, 2500), (448, 1500)]
+    count = 48000
+    lengths += [tuple(pair) for pair in rng.integers(1, 470, size=(count - len(lengths), 2))]
+    pool = rng.choice(alphabet, size=1 << 20).astype(np.uint8)
+    starts = rng.integers(0, pool.size - 4000, size=(count, 2))
+    order = rng.permutation(count)
+    first, second = ([bytes(pool[starts[i, side]:starts[i, side] + lengths[i][side]]) for i in order] for side in (0, 1))
+    for k in range(0, count, 5):  # alike, too: the second string within the first one's
+        second[k] = first[k][: len(first[k]) // 2] + first[k][len(first[k]) // 2 + 2:]
+    engine, oracle_costs = make_engine(szs, family, costs, b2c, table)
+    want = port.pairs(oracle_costs, tape(first), tape(second))
+    np.testing.assert_array_equal(engine.pairwise(szs.Strs(first), szs.Strs(second)).astype(np.int64), want)
+    assert engine.stats()["last_launches"] >= 20  # a launch per shape
+    third = count // 3
+    got = engine.pairwise(szs.Strs(first[:third]), szs.Strs(second[:third])).astype(np.int64)
+    np.testing.assert_array_equal(got, want[:third])
+    assert engine.stats()["last_launches"] < 20

@@ -166,3 +166,26 @@ int main() {
 }
 """)
     assert not broken, broken[:5]
+
+
+def test_quarter_octaves_need_rows(tmp_path):
+    """Calls measured faster in halves of octaves stay there, and those measured faster in quarters have rows enough."""
+    broken = run_checks(tmp_path, r"""
+#include <cuda_runtime.h>
+#include <cstdio>
+#include "planner.cuh"
+using namespace szs_gb300;
+static void expect(double pairs, float rows, float columns, bool profile, bool want) {
+    if ((pairs * rows >= short_fine_rows(rows, columns, profile)) != want)
+        std::printf("%.0f pairs of %.0f x %.0f, profile %d: not %d\n", pairs, rows, columns, (int)profile, (int)want);
+}
+int main() {
+    expect(150000, 30, 600, true, false), expect(45000, 30, 600, false, false), expect(250000, 30, 600, false, true);
+    expect(20000, 167, 233, true, false), expect(45000, 167, 233, true, true), expect(30000, 167, 233, false, true);
+    expect(65536, 93, 147, true, false), expect(100000, 93, 147, true, true), expect(65536, 93, 147, false, true);
+    expect(20000, 200, 200, true, false), expect(65536, 200, 200, true, true), expect(65536, 200, 200, false, true);
+    expect(65536, 120, 120, true, true), expect(1048576, 72, 72, true, true), expect(16384, 350, 350, true, true);
+    expect(150000, 53, 91, true, false), expect(150000, 53, 91, false, true), expect(16384, 450, 450, false, true);
+}
+""")
+    assert not broken, broken[:5]
