@@ -630,6 +630,7 @@ struct call_t {
     // them), scoring for `scoring_after` (the chunk's bytes); a sampled alphabet comes from `sample_*` (the first
     // chunk's tapes, on the device before the later chunks), so the plan of a chunk can run before its bytes land.
     cudaEvent_t plan_after = nullptr, scoring_after = nullptr;
+    near_sample_t near_sample {}; // how alike the pairs look, for plans made before the strings have landed
     tape_t const *sample_queries = nullptr, *sample_candidates = nullptr;
     // Two phases on one context: `plan_only` returns once the plan is read back and kept in the context; a later
     // call with `reuse_plan` (same tapes and costs) scores that plan without planning again.
@@ -898,8 +899,8 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         args.packed_step_cost[choice] = engine.tuning.packed_step_cost[choice]
                                             ? engine.tuning.packed_step_cost[choice]
                                             : (std::uint16_t)packed_step_cost_k[choice];
-    // Unit costs: whether most pairs look alike decides if they are tried near their diagonal first. Plans made before
-    // the strings have landed (pipelined chunks) cannot look at them and try.
+    // Unit costs: how alike the pairs look decides if they are tried near their diagonal first (`near_pays`). Plans made
+    // before the strings have landed (pipelined chunks but the first) cannot look at them and go by the first chunk.
     bool const planned_ahead = call.scoring_after && call.plan_after != call.scoring_after;
     args.near_sample_stride =
         engine.unit_levenshtein && schedule != szs_gb300_schedule_plain_k && !planned_ahead
@@ -1320,11 +1321,11 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
         // pair busy for long, so it takes batches of more pairs than the warp route scores at once (two CTAs of eight
         // warps per SM).
         int near_words = myers_max_words_k + 1, near_per_lane = 0; // first words, most words per lane it takes
-        // A pair given up early costs about an eighth of its full score, one found saves a third or more.
-        if (!plain && (!args.near_sample_stride || plan.near_alike * 3 > plan.near_sampled)) {
-            auto near_job = [&](int half, int key_begin, int key_end) {
+        if (!plain) {
+            near_sample_t const &sample = args.near_sample_stride ? plan.near : call.near_sample;
+            auto near_job = [&](int half, int key_begin, int key_end, std::uint32_t longest) {
                 std::uint64_t const pairs_here = pairs_in(key_begin, key_end);
-                if (!pairs_here) return;
+                if (!pairs_here || !near_pays(sample, pairs_here, longest, half)) return false;
                 std::uint64_t const needed = (pairs_here + myers_near_threads() - 1) / myers_near_threads();
                 int const ctas = (int)std::min<std::uint64_t>(needed, (std::uint64_t)context->sm_count * 16);
                 if (!near_list_at) {
@@ -1332,14 +1333,19 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
                     scratch_total = near_list_at + align_up(args.pairs * sizeof(std::uint32_t), 256);
                 }
                 jobs[job_count++] = {job_near_k, half, 0, key_begin, key_end, pairs_here, ctas, 0, 0};
+                return true;
             };
             int const warp_end = bin_myers_warp_begin_k + myers_warp_max_words_k * myers_warp_classes_k;
-            near_words = near_min_words_k;
-            near_job(1, bin_myers_begin_k + near_words * 16, bin_myers_begin_k + (myers_max_words_k + 1) * 16);
+            if (near_job(1, bin_myers_begin_k + near_min_words_k * 16, bin_myers_begin_k + (myers_max_words_k + 1) * 16,
+                         plan.max_myers_rows))
+                near_words = near_min_words_k;
             int const one_per_lane = warp_end - myers_warp_classes_k;
-            if (wide && pairs_in(one_per_lane, warp_end)) near_per_lane = 1, near_job(1, one_per_lane, warp_end);
-            if (myers_planes == 2 && pairs_in(bin_myers_warp_begin_k, warp_end) >= (std::uint64_t)context->sm_count * 16)
-                near_per_lane = myers_warp_max_words_k, near_job(4, bin_myers_warp_begin_k, warp_end);
+            if (wide && near_job(1, one_per_lane, warp_end, std::min<std::uint32_t>(plan.max_myers_warp_rows, 1024)))
+                near_per_lane = 1;
+            if (myers_planes == 2 &&
+                pairs_in(bin_myers_warp_begin_k, warp_end) >= (std::uint64_t)context->sm_count * 16 &&
+                near_job(4, bin_myers_warp_begin_k, warp_end, plan.max_myers_warp_rows))
+                near_per_lane = myers_warp_max_words_k;
         }
         // Longer patterns first: one warp per pair, most words per lane first.
         for (int words = myers_warp_max_words_k; words >= 1; --words) {
@@ -1580,8 +1586,14 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             float ms = 0, offset = 0;
             cudaEventElapsedTime(&ms, context->trace_events[2 * i], context->trace_events[2 * i + 1]);
             cudaEventElapsedTime(&offset, context->compute_start, context->trace_events[2 * i]);
-            std::fprintf(stderr, "[szs_gb300] %-20s %3d  pairs %10llu  start %8.3f ms  took %9.3f ms\n",
-                         names[jobs[i].kind], jobs[i].variant, (unsigned long long)jobs[i].pairs, offset, ms);
+            std::fprintf(stderr, "[szs_gb300] %-20s %3d  pairs %10llu  ctas per pair %3d  start %8.3f ms  took %9.3f ms\n",
+                         names[jobs[i].kind], jobs[i].variant, (unsigned long long)jobs[i].pairs, jobs[i].group_ctas, offset,
+                         ms);
+        }
+        if (near_list_at) {
+            std::uint32_t tried[2] = {0, 0}; // pairs tried near the diagonal, and those of them that failed
+            SZS_TRY_CUDA(cudaMemcpy(tried, &bins->near_tried, sizeof(tried), cudaMemcpyDeviceToHost));
+            std::fprintf(stderr, "[szs_gb300] near diagonal tried %u failed %u\n", tried[0], tried[1]);
         }
     }
     stats.last_launches = launches;
@@ -1783,6 +1795,7 @@ static status_t run_pipelined(engine_t const &engine, device_context_t *context,
     bool const alphabet_pass = (engine.kind == kind_levenshtein_k || !engine.dense.empty()) && !engine.utf8;
     bool const sampled = alphabet_pass && engine.unit_levenshtein;
     bool const plan_ahead = !alphabet_pass || sampled;
+    near_sample_t first_chunk {}; // how alike the first chunk's pairs look (unit costs)
     auto plan = [&](int c) -> status_t { // plans chunk c on context c % depth, once its previous chunk is settled
         int const which = c % depth;
         status_t settled = settle(which);
@@ -1798,9 +1811,11 @@ static status_t run_pipelined(engine_t const &engine, device_context_t *context,
         chunk.scoring_after = context->copied[c];
         chunk.plan_after = !alphabet_pass ? context->offsets_copied : sampled ? context->copied[0] : context->copied[c];
         if (sampled) chunk.sample_queries = &staged[0], chunk.sample_candidates = &staged[1];
+        if (c) chunk.near_sample = first_chunk;
         chunk.plan_only = true;
         chunk_stats[which].graph_replays = 0;
         status_t const planned = run_on(engine, contexts[which], streams[which], chunk, schedule, chunk_stats[which]);
+        if (!c) first_chunk = contexts[which]->bins_host()->near;
         launches += chunk_stats[which].last_launches;
         host_marks[3 * c + 1] = host_ms();
         return planned;

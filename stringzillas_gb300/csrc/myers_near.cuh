@@ -13,8 +13,8 @@
  *  stays inside, so a result of at most 64 h - (m - n) is the distance; any other pair is listed for the full kernel of
  *  its bin (myers_table.cuh, myers.cuh, myers_warp.cuh), which scores it from the start. Pairs far apart give up early:
  *  values on the final diagonal never decrease, so they stop when it passes the limit, or when its growth so far
- *  predicts that it will. Once nearly all pairs tried have failed (a batch of unrelated strings), the CTAs still to come
- *  list theirs untried.
+ *  predicts that it will. Which calls are tried at all is `near_pays`' choice, by the ends of sampled pairs; should nearly
+ *  all pairs tried fail for all that (alike at their ends only), the CTAs still to come list theirs untried.
  *
  *  Measured: 1,048,576 DNA pairs of U[100, 300], 4 % apart, 1.22 -> 0.63 ms per call (895,168 of them here in 0.50 ms,
  *  bound by the integer pipe: 34 operations a column for three words); 4,096 reads of 1,000-4,000 2.03 -> 0.78 ms (nine

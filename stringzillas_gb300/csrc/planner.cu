@@ -238,22 +238,31 @@ __device__ __forceinline__ pair_route_info_t route_of_pair(plan_args_t const &ar
     return route_pair(args, first, first_length, second, second_length, short_fine);
 }
 
-/** Whether two strings of `n` <= `m` symbols look so alike that their distance should be at most `distance`: by the
- *  share of their first and last 16 symbols that are the same in place, or of one end's where the other has fewer than 9
- *  (one insertion hides the rest of an end; unrelated DNA agrees in 4). Not the better end's of two: that promises too
- *  much near the limit, where a pair is given up late (211,388 texts of 230-435 at 20 % substitutions 1.34 ms without the
- *  trial, 1.47 with it). Decides only which kernel tries first, never a score. */
+/** Edits between the first 16 rows and the start of the text that is nearest to them (of at most 20 symbols), by the
+ *  bit-parallel step on one half word; `direction` -1: the last 16, from the strings' last symbols backwards. All loads come
+ *  first: the plan waits for them once. */
 template <typename symbol_>
-__device__ __forceinline__ bool looks_alike(symbol_ const *rows, std::uint32_t n, symbol_ const *cols, std::uint32_t m,
-                                            std::uint32_t distance) {
-    std::uint32_t head = 0, tail = 0;
+__device__ __forceinline__ int end_edits(symbol_ const *rows, symbol_ const *cols, int direction) {
+    std::uint32_t row[16], col[20], pv = 0xFFFFFFFFu, mv = 0u;
 #pragma unroll
-    for (std::uint32_t k = 0; k < 16; ++k) {
-        head += rows[k] == cols[k];
-        tail += rows[n - 1 - k] == cols[m - 1 - k];
+    for (int k = 0; k < 16; ++k) row[k] = rows[direction * k];
+#pragma unroll
+    for (int j = 0; j < 20; ++j) col[j] = cols[direction * j];
+    int score = 16, least = 16;
+#pragma unroll
+    for (int j = 0; j < 20; ++j) {
+        std::uint32_t eq = 0;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) eq |= (row[k] == col[j] ? 1u : 0u) << k;
+        std::uint32_t const xv = eq | mv, xh = (((eq & pv) + pv) ^ pv) | eq;
+        std::uint32_t const ph = mv | ~(xh | pv), mh = pv & xh;
+        score += (int)((ph >> 15) & 1u) - (int)((mh >> 15) & 1u);
+        least = min(least, score);
+        std::uint32_t const ph_shifted = ph << 1 | 1u;
+        pv = mh << 1 | ~(xv | ph_shifted);
+        mv = ph_shifted & xv;
     }
-    std::uint32_t const twice = head >= 9 && tail >= 9 ? head + tail : 2 * max(head, tail);
-    return twice >= 18 && (std::uint64_t)(32 - twice) * m <= 32ull * distance;
+    return least;
 }
 
 /** Pass 1: answer trivial pairs, count pairs per bin, track the longest column string and total cells. */
@@ -324,10 +333,11 @@ __global__ void plan_count_kernel(plan_args_t const args, plan_bins_t *__restric
     }
 }
 
-/** Whether pair @p p is one that the near-diagonal kernels would try (patterns of at least five words, up to 32 or 128
- *  symbols of difference in length), and if it is, whether it looks like a distance well inside their limits of 64 and
- *  256. */
-__device__ __forceinline__ bool near_candidate(plan_args_t const &args, std::uint64_t p, bool &alike) {
+/** What the near-diagonal kernels would find in pair @p p, by its ends: 0 it is not theirs (patterns of at least five words,
+ *  up to 8,192 rows), 1 unrelated, or of lengths too different, 2 related, 3 related and at a distance well inside their
+ *  limits of 64 and 256. `edits`: of a related pair's 32 rows at both ends (a fifth of substitutions makes 6 or 7, unrelated
+ *  DNA some 14). Two lanes per pair, one at each end (`tail`). */
+__device__ __forceinline__ int near_likeness(plan_args_t const &args, std::uint64_t p, bool tail, int &edits) {
     std::uint64_t q, c;
     pair_indices(args, p, q, c);
     std::uint8_t const *first, *second;
@@ -338,22 +348,38 @@ __device__ __forceinline__ bool near_candidate(plan_args_t const &args, std::uin
     std::uint8_t const *rows = swap ? second : first, *cols = swap ? first : second;
     std::uint64_t const n = swap ? second_length : first_length, m = swap ? first_length : second_length;
     std::uint32_t const blocks = n <= 32u * myers_max_words_k ? 1u : 4u;
-    if (n <= 32u * (near_min_words_k - 1) || n > 32u * 32u * myers_warp_max_words_k || m - n > 32u * blocks) return false;
-    alike = args.wide ? looks_alike(reinterpret_cast<std::uint16_t const *>(rows), (std::uint32_t)n,
-                                    reinterpret_cast<std::uint16_t const *>(cols), (std::uint32_t)m, 40u * blocks)
-                      : looks_alike(rows, (std::uint32_t)n, cols, (std::uint32_t)m, 40u * blocks);
-    return true;
+    if (n <= 32u * (near_min_words_k - 1) || n > 32u * 32u * myers_warp_max_words_k) return 0;
+    if (m - n > 32u * blocks) return 1;
+    std::uint64_t const row_at = tail ? n - 1 : 0, col_at = tail ? m - 1 : 0;
+    int const direction = tail ? -1 : 1;
+    int const own = args.wide ? end_edits(reinterpret_cast<std::uint16_t const *>(rows) + row_at,
+                                          reinterpret_cast<std::uint16_t const *>(cols) + col_at, direction)
+                              : end_edits(rows + row_at, cols + col_at, direction);
+    unsigned const both = 3u << (threadIdx.x & 30u);
+    int const other = __shfl_xor_sync(both, own, 1);
+    if (min(own, other) >= near_unrelated_edits_k) return 1;
+    edits = own + other;
+    return (std::uint64_t)edits * m <= 32ull * 40u * blocks ? 3 : 2;
 }
 
-/** Pass 2: exclusive scan of bin counts (one CTA of `bin_keys_k / 2` threads, two adjacent keys each). A second CTA
- *  samples the pairs' likeness meanwhile, one pair per thread. */
+/** Pass 2: exclusive scan of bin counts (one CTA of `bin_keys_k / 2` threads, two adjacent keys each). Further CTAs
+ *  sample the pairs' likeness meanwhile, two threads per pair. */
 __global__ void __launch_bounds__(bin_keys_k / 2) plan_scan_kernel(plan_args_t const args, plan_bins_t *__restrict__ bins) {
-    if (blockIdx.x == 1) {
-        std::uint64_t const p = (std::uint64_t)threadIdx.x * args.near_sample_stride;
-        bool alike = false;
-        bool const sampled = threadIdx.x < near_samples_k && p < args.pairs && near_candidate(args, p, alike);
-        int const samples = __syncthreads_count(sampled), similar = __syncthreads_count(sampled && alike);
-        if (threadIdx.x == 0) bins->near_sampled = (std::uint32_t)samples, bins->near_alike = (std::uint32_t)similar;
+    if (blockIdx.x) { // sixteen pairs on one warp: their scattered bytes would queue on a single SM
+        if (threadIdx.x >= 32) return;
+        bool const first = (threadIdx.x & 1) == 0;
+        std::uint64_t const p = ((blockIdx.x - 1) * 16u + (threadIdx.x >> 1)) * (std::uint64_t)args.near_sample_stride;
+        int edits = 0;
+        int const likeness = p < args.pairs ? near_likeness(args, p, !first, edits) : 0;
+        __syncwarp();
+        int const sum = __reduce_add_sync(0xFFFFFFFFu, first ? edits : 0);
+        unsigned const sampled = __ballot_sync(0xFFFFFFFFu, first && likeness != 0);
+        unsigned const unrelated = __ballot_sync(0xFFFFFFFFu, first && likeness == 1);
+        unsigned const alike = __ballot_sync(0xFFFFFFFFu, first && likeness == 3);
+        if (threadIdx.x == 0) {
+            atomicAdd(&bins->near.sampled, (unsigned)__popc(sampled)), atomicAdd(&bins->near.unrelated, (unsigned)__popc(unrelated));
+            atomicAdd(&bins->near.alike, (unsigned)__popc(alike)), atomicAdd(&bins->near.edits, (unsigned)sum);
+        }
         return;
     }
     constexpr int warps = bin_keys_k / 2 / 32;
@@ -585,7 +611,8 @@ cudaError_t launch_plan(plan_args_t const &args, plan_bins_t *bins, pair_task_t 
     if (args.pairs == 0) return cudaSuccess;
     status = launch_prioritised(plan_count_kernel, grid_for(args.pairs, 256, sm_count), 256, stream, args, bins, results);
     if (status != cudaSuccess) return status;
-    status = launch_prioritised(plan_scan_kernel, args.near_sample_stride ? 2 : 1, bin_keys_k / 2, stream, args, bins);
+    status = launch_prioritised(plan_scan_kernel, 1 + (args.near_sample_stride ? near_samples_k / 16 : 0), bin_keys_k / 2, stream,
+                                args, bins);
     if (status != cudaSuccess) return status;
     return launch_prioritised(plan_scatter_kernel, grid_for(args.pairs, 256, sm_count), 256, stream, args, bins, tasks);
 }

@@ -118,6 +118,8 @@ __host__ __device__ inline int short_bin(std::uint64_t n, std::uint64_t m, bool 
 static_assert(bin_myers_chain_k < bin_keys_k, "bin layout exceeds the key space");
 constexpr int near_min_words_k = 5; // patterns of the thread route that the near-diagonal kernel tries
 constexpr std::uint32_t near_samples_k = 128; // pairs sampled per call
+constexpr int near_unrelated_edits_k = 6;     // fewest edits in 16 rows at either end of a pair that counts as unrelated
+constexpr std::uint64_t near_large_pairs_k = 100000; // pairs from which the trial's left-over does not cost its chain
 constexpr std::uint32_t near_trial_k = 4096; // pairs tried near the diagonal before a batch may be found unrelated
 constexpr std::uint32_t myers_chain_max_rows_k = 1u << 20; // longest pattern a chain of warps takes
 
@@ -168,6 +170,33 @@ struct plan_args_t {
     std::uint32_t near_sample_stride;    // unit-cost calls: every so many pairs one is sampled for likeness (0: none)
 };
 
+/** What the ends of sampled pairs say about trying a call's pairs near their diagonal first (myers_near.cuh). */
+struct near_sample_t {
+    std::uint32_t sampled;   // pairs sampled that the near-diagonal kernels could take
+    std::uint32_t unrelated; // unrelated, or of lengths too different
+    std::uint32_t alike;     // at a distance well inside the kernels' limits
+    std::uint32_t edits;     // of all related ones' 32 rows at both ends
+};
+
+/**
+ *  Whether @p pairs with patterns of up to @p longest rows should be tried near their diagonal (`half` blocks either side)
+ *  before the full kernels score what is left. A pair found saves a third of its work or more, but what is left over starts
+ *  only when all have been tried, so a few failures cost a call of less than some waves of threads a whole full kernel's
+ *  chain. Such a call has to have hardly an unrelated pair, and its longest pairs at the sampled rate of edits have to stay
+ *  inside the limit; a larger one needs a third of its pairs alike and less than half unrelated. Against never trying: 20,000
+ *  DNA reads of 100-300 at 8-18 % substitutions 1.17-1.25x, at 22 % 0.80x, half of them unrelated 0.77x; 5,000 of
+ *  1,000-4,000 with a tenth unrelated 0.76x, at 8 % 1.05x, at 4 % 2.6x; 200,000 of 100-300 at 26 % 1.18x, with 35 %
+ *  unrelated 1.08x, with half 0.98x, with 65 % 0.90x.
+ */
+inline bool near_pays(near_sample_t const &sample, std::uint64_t pairs, std::uint32_t longest, int half) {
+    if (pairs >= near_large_pairs_k)
+        return sample.alike * 3 > sample.sampled && sample.unrelated * 20 <= sample.sampled * 9;
+    if (!sample.alike || sample.unrelated * 32 > sample.sampled) return false;
+    float const edits = (float)sample.edits / (32.0f * (float)(sample.sampled - sample.unrelated)) * (float)longest;
+    float const room = 64.0f * (float)half - edits;
+    return room > 0 && edits * (2.8f * 2.8f) <= room * room; // 2.8 standard deviations
+}
+
 /** Per-bin counters the planner fills. */
 struct plan_bins_t {
     std::uint32_t count[bin_keys_k];
@@ -182,7 +211,7 @@ struct plan_bins_t {
     std::uint32_t max_myers_warp_rows; // longest pattern on the warp-per-pair bit-parallel route
     std::uint32_t max_chain_rows;      // longest pattern on the chained bit-parallel route
     std::uint32_t near_tried, near_failed; // pairs the near-diagonal kernel has tried, and those it had to list
-    std::uint32_t near_sampled, near_alike; // pairs the planner sampled for likeness, and those found alike
+    near_sample_t near;                     // the planner's look at the pairs' likeness
     std::uint32_t short_fine;              // whether short pairs are cut in quarter octaves (`short_fine_rows`)
     std::uint32_t listed[32];              // pairs it listed per class of full kernel (words; 16 + words per lane)
 };

@@ -189,3 +189,34 @@ int main() {
 }
 """)
     assert not broken, broken[:5]
+
+
+def test_near_diagonal_trials_that_pay(tmp_path):
+    """The trial near the diagonal: small calls need hardly an unrelated pair and their longest pairs well inside the
+    limit, large ones enough alike; calls measured faster without it go without."""
+    broken = run_checks(tmp_path, r"""
+#include <cuda_runtime.h>
+#include <cstdio>
+#include "planner.cuh"
+using namespace szs_gb300;
+static void expect(char const *what, double unrelated, double alike, double rate, std::uint64_t pairs, unsigned longest,
+                   int half, bool want) {
+    near_sample_t const sample {128, unsigned(128 * unrelated), unsigned(128 * alike),
+                                unsigned((128 - unsigned(128 * unrelated)) * 32 * rate)};
+    if (near_pays(sample, pairs, longest, half) != want) std::printf("%s: not %d\n", what, (int)want);
+}
+int main() {
+    expect("1M reads, 4 %", 0, 1, 0.04, 1 << 20, 300, 1, true), expect("long reads, 4 %", 0, 1, 0.04, 4096, 4000, 4, true);
+    expect("65,536 CJK, 7 %", 0, 1, 0.07, 65536, 300, 1, true), expect("20,000 reads, 10 %", 0, 1, 0.10, 20000, 300, 1, true);
+    expect("20,000 reads, 17 %", 0, 0.9, 0.17, 20000, 300, 1, false);
+    expect("20,000 reads, a tenth unrelated", 0.1, 0.9, 0.02, 20000, 300, 1, false);
+    expect("200,000 reads, a third unrelated", 0.35, 0.65, 0.02, 200000, 300, 1, true);
+    expect("200,000 reads, two thirds unrelated", 0.65, 0.35, 0.02, 200000, 300, 1, false);
+    expect("5,000 long reads, a tenth unrelated", 0.1, 0.9, 0.02, 5000, 4000, 4, false);
+    expect("5,000 long reads, 9 %", 0, 0.2, 0.09, 5000, 4000, 4, false);
+    expect("unrelated", 1, 0, 0, 1 << 20, 300, 1, false), expect("20,000 unrelated", 1, 0, 0, 20000, 300, 1, false);
+    near_sample_t const none {};
+    if (near_pays(none, 1 << 20, 300, 1) || near_pays(none, 1000, 300, 1)) std::printf("nothing sampled\n");
+}
+""")
+    assert not broken, broken[:5]
