@@ -106,3 +106,23 @@ check(engine, oracle.levenshtein_costs(), first, (mutant(first[0], {rate}), firs
     jobs = [line for line in lines if "job kind 8 " in line]
     assert len(chunks) >= 4
     assert len(jobs) >= len(chunks) if tried else not jobs
+
+
+def test_largest_pairs_of_a_batch_in_groups():
+    """Many 16-bit band pairs of very different sizes: the largest size classes take groups of CTAs, the others single ones,
+    in one call."""
+    lines = trace("""
+lengths = np.concatenate([rng.integers(2050, 2400, 360), [9000, 8200, 12000]])
+other = np.concatenate([rng.integers(2050, 2600, 360), [9500, 16000, 8500]])
+table = np.zeros((32, 32), dtype=np.int8)
+table[1:5, 1:5] = -3
+np.fill_diagonal(table[1:5, 1:5], 2)
+classes = np.zeros(256, dtype=np.uint8)
+classes[DNA] = [1, 2, 3, 4]
+engine = szs.SmithWatermanScores(classes, table, open=-5, extend=-2)
+check(engine, oracle.alignment_costs(oracle.SMITH_WATERMAN, classes, table, -5, -2), tape(lengths), tape(other))
+""")
+    found = [re.search(r"band16 bits .*pairs +(\d+) +ctas per pair +(\d+)", line) for line in lines]
+    jobs = [(int(m.group(1)), int(m.group(2))) for m in found if m]
+    assert sum(pairs for pairs, _ in jobs) == 363
+    assert any(group > 1 for _, group in jobs) and any(group == 1 for _, group in jobs)
