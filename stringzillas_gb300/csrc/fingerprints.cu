@@ -43,7 +43,6 @@ constexpr int tensor_dims_k = fingerprint_group_k;           // 64 dimensions pe
 static_assert(tensor_dims_k == 8 * tensor_tiles_k, "a warp's dimensions are whole tiles");
 constexpr int tensor_chunk_k = 256;                          // window starts per staged chunk
 constexpr int tensor_staged_k = tensor_chunk_k + 2 * tensor_width_k; // byte pairs staged per chunk
-constexpr std::uint32_t tensor_windows_min_k = 128;          // texts with fewer windows are rolled
 constexpr std::uint32_t tensor_list_k = 512;                 // candidate windows a chunk may list
 constexpr int tensor_warps_k = 4;                            // warps per CTA, each on its own text and dimensions
 
@@ -117,10 +116,19 @@ struct rolling_t {
     }
 };
 
-/** Whether a text has too few windows (of its group's widest dimension) to bound the minimum by tensor-core tiles
+/** Whether a text has fewer windows (of its group's widest dimension) than pay for bounding the minimum by tensor-core tiles
  *  before its candidates are listed: it is rolled exactly. */
-__device__ __forceinline__ bool rolls(std::uint64_t length, std::uint32_t widest) {
-    return length < widest + (tensor_windows_min_k - 1u);
+__device__ __forceinline__ bool rolls(std::uint64_t length, std::uint32_t widest, std::uint32_t windows_min) {
+    return length < widest + (windows_min - 1u);
+}
+
+/** The fewest windows of a tensor-core text. The tensor kernel's chain per text is longer at the start than a short text's
+ *  rolled one, so calls that leave warp slots free roll longer texts than those that fill them. Rolled / tensor: 1 to 64
+ *  texts of 200 bytes at 64 to 1,024 dimensions 46 / 49 us, of 300 56 / 53; 1,000 of 100-200 at 64 dimensions 53 / 73; 250 of
+ *  150 at 1,024 81 / 92, of 200 102 / 83 (but 1,000 of 100-200 at 256, of which a quarter pass the line, 105 / 130); 4,000 of
+ *  150 at 1,024 815 / 688. */
+std::uint32_t tensor_windows_min(std::uint64_t items, int sm_count) {
+    return items <= 12ull * sm_count ? 224 : items <= 48ull * sm_count ? 160 : 128;
 }
 
 /** What one warp of the tensor-core kernel keeps in shared memory. */
@@ -175,8 +183,9 @@ __device__ __forceinline__ void mma_tile(float (&d)[4], std::uint32_t a0, std::u
 template <int steps_>
 __global__ void __launch_bounds__(32 * tensor_warps_k, steps_ == 1 ? 4 : 3)
     fingerprints_tensor_kernel(tape_t const texts, fingerprint_dim_t const *__restrict__ params,
-                               fingerprint_weights_t const *__restrict__ digits, std::uint32_t const dimensions, fingerprint_group_t const *__restrict__ groups,
-                               std::uint32_t const groups_count, std::uint32_t *__restrict__ hashes,
+                               fingerprint_weights_t const *__restrict__ digits, std::uint32_t const dimensions,
+                               fingerprint_group_t const *__restrict__ groups, std::uint32_t const groups_count,
+                               std::uint32_t const windows_min, std::uint32_t *__restrict__ hashes,
                                std::uint64_t const hashes_stride, std::uint32_t *__restrict__ counts,
                                std::uint64_t const counts_stride) {
     extern __shared__ __align__(16) unsigned char tensor_s[];
@@ -198,7 +207,8 @@ __global__ void __launch_bounds__(32 * tensor_warps_k, steps_ == 1 ? 4 : 3)
         for (; text < texts.count; text += 32 * slots) {
             std::uint64_t const candidate = text + lane * slots;
             bool const mine = candidate < texts.count &&
-                              !rolls(text_offset(texts, candidate + 1) - text_offset(texts, candidate), widest);
+                              !rolls(text_offset(texts, candidate + 1) - text_offset(texts, candidate), widest,
+                                     windows_min);
             if (std::uint32_t const found = __ballot_sync(0xFFFFFFFFu, mine)) return text + (__ffs(found) - 1) * slots;
         }
         return texts.count;
@@ -441,7 +451,7 @@ __global__ void __launch_bounds__(32 * tensor_warps_k, steps_ == 1 ? 4 : 3)
  */
 __global__ void __launch_bounds__(256, 5) fingerprints_kernel(
     tape_t const texts, fingerprint_dim_t const *__restrict__ params, std::uint32_t const dimensions,
-    fingerprint_group_t const *__restrict__ groups, std::uint32_t const groups_count,
+    fingerprint_group_t const *__restrict__ groups, std::uint32_t const groups_count, std::uint32_t const windows_min,
     std::uint32_t *__restrict__ hashes, std::uint64_t const hashes_stride, std::uint32_t *__restrict__ counts,
     std::uint64_t const counts_stride) {
     asm volatile("griddepcontrol.launch_dependents;"); // the tensor-core kernels take other texts: they may start
@@ -456,7 +466,7 @@ __global__ void __launch_bounds__(256, 5) fingerprints_kernel(
         fingerprint_group_t const group = groups[half / 2];
         std::uint64_t const start = text_offset(texts, text);
         std::uint64_t const length = text_offset(texts, text + 1) - start;
-        if (group.widest <= (std::uint32_t)tensor_width_k && !rolls(length, group.widest)) continue;
+        if (group.widest <= (std::uint32_t)tensor_width_k && !rolls(length, group.widest, windows_min)) continue;
         std::uint32_t const dim = group.index * fingerprint_group_k + (half & 1u) * 32 + lane;
         bool const live = dim < dimensions;
         if (!__any_sync(0xFFFFFFFFu, live)) continue;
@@ -586,8 +596,9 @@ cudaError_t launch_fingerprints(tape_t const &texts, fingerprint_dim_t const *pa
     std::uint32_t const total = groups.count[0] + groups.count[1] + groups.count[2];
     std::uint64_t const blocks = (texts.count * 2 * total + 7) / 8; // 8 warps per CTA
     unsigned const grid = (unsigned)std::min<std::uint64_t>(blocks, (std::uint64_t)sm_count * 16);
-    fingerprints_kernel<<<grid, 256, 0, stream>>>(texts, params, dimensions, group_list, total, hashes, hashes_stride,
-                                                  counts, counts_stride);
+    std::uint32_t const windows_min = tensor_windows_min(texts.count * total, sm_count);
+    fingerprints_kernel<<<grid, 256, 0, stream>>>(texts, params, dimensions, group_list, total, windows_min, hashes,
+                                                  hashes_stride, counts, counts_stride);
     cudaError_t launched = cudaGetLastError();
     cudaLaunchAttribute overlap;
     overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -611,7 +622,7 @@ cudaError_t launch_fingerprints(tape_t const &texts, fingerprint_dim_t const *pa
         config.dynamicSmemBytes = sizeof(tensor_warp_t) * (std::size_t)warps;
         launched = cudaLaunchKernelEx(
             &config, kind == 0 ? fingerprints_tensor_kernel<1> : fingerprints_tensor_kernel<2>, texts, params, weights,
-            dimensions, list, here, hashes, hashes_stride, counts, counts_stride);
+            dimensions, list, here, windows_min, hashes, hashes_stride, counts, counts_stride);
     }
     return launched;
 }

@@ -214,3 +214,22 @@ def test_window_and_chunk_edges_match_oracle(szs, dimensions, widths):
     want_h, want_c = oracle.fingerprints(dimensions, (data, offsets), widths, 3)
     np.testing.assert_array_equal(hashes, want_h)
     np.testing.assert_array_equal(counts, want_c)
+
+
+@pytest.mark.parametrize("count", [40, 2500, 8000])
+def test_shortest_tensor_texts_match_oracle(szs, count):
+    """Texts around the fewest windows that the tensor-core kernel takes in calls of few, some and many texts (224, 160 and
+    128), beside shorter and longer ones, repeats among them."""
+    rng = np.random.default_rng(count)
+    widths = [7, 16, 29]
+    windows = rng.choice([1, 100, 127, 128, 129, 159, 160, 161, 223, 224, 225, 300], size=count)
+    texts = [rng.integers(0, 256 if i % 3 else 2, int(w) + widths[i % 3] - 1).astype(np.uint8)
+             for i, w in enumerate(windows)]
+    offsets = np.zeros(count + 1, dtype=np.uint64)
+    offsets[1:] = np.cumsum([len(t) for t in texts])
+    data = np.concatenate(texts)
+    engine = szs.Fingerprints(66, np.array(widths, dtype=np.uint64), seed=9)
+    hashes, counts = engine(_strs(szs, data, offsets))
+    want_h, want_c = oracle.fingerprints(66, (data, offsets), widths, 9)
+    np.testing.assert_array_equal(hashes, want_h)
+    np.testing.assert_array_equal(counts, want_c)
