@@ -234,7 +234,8 @@ struct device_context_t {
     device_buffer_t chunk_inputs;
     static constexpr int pipeline_depth_k = 12; // chunks of a pipelined call in flight at once
     device_context_t *partners[pipeline_depth_k] = {nullptr}; // the contexts a pipelined call's chunks rotate over
-    device_buffer_t utf8;                // UTF-8 calls: code-point set, counts, offsets and transcoded tapes
+    device_buffer_t utf8;                // UTF-8 calls: code-point set, counts, and the tapes as 16-bit values
+    device_buffer_t utf8_ranks;          // the tapes as one-byte codes, for calls that recode their values
     device_buffer_t dense_table;         // the 256 x 256 table of the dense engine last run here over > 32 bytes
     std::uint64_t dense_table_id = 0;    // that engine's `dense_id` (0: none)
     bool deferred = false, deferred_compute = false;
@@ -309,7 +310,7 @@ struct device_context_t {
         if (pipe_stop) cudaEventDestroy(pipe_stop);
         if (offsets_copied) cudaEventDestroy(offsets_copied);
         chunk_inputs.release();
-        utf8.release();
+        utf8.release(), utf8_ranks.release();
         dense_table.release(), dense_table_id = 0;
         for (auto &partner : partners)
             if (partner) {
@@ -671,14 +672,14 @@ static status_t transcode_utf8(device_context_t *context, cudaStream_t stream, t
     SZS_TRY_CUDA(launch_utf8_extents(queries, has_candidates ? candidates : queries, context->spare_host(), stream));
     SZS_TRY_CUDA(cudaStreamSynchronize(stream));
     std::uint64_t const first[2] = {extents[0], extents[2]}, end[2] = {extents[1], extents[3]};
-    std::size_t layout[2][3] = {}; // counts, 16-bit values, one-byte codes
-    std::size_t cursor = align_up(sizeof(rune_set_t), 256);
+    std::size_t layout[2][2] = {}, ranks_at[2] = {0, 0}; // counts and 16-bit values; one-byte codes
+    std::size_t cursor = align_up(sizeof(rune_set_t), 256), ranks_bytes = 0;
     for (int t = 0; t < 2; ++t) {
         if (!tapes[t]) continue;
         // Room for a whole 8-byte chunk past the end of both.
         layout[t][0] = cursor, cursor += align_up(tapes[t]->count * 8, 256);
         layout[t][1] = cursor, cursor += align_up(2 * (end[t] - first[t]) + 8, 256);
-        layout[t][2] = cursor, cursor += align_up(end[t] - first[t] + 8, 256);
+        ranks_at[t] = ranks_bytes, ranks_bytes += align_up(end[t] - first[t] + 8, 256);
     }
     status_t status = context->utf8.reserve(cursor, stream);
     if (!status.ok()) return status;
@@ -700,16 +701,20 @@ static status_t transcode_utf8(device_context_t *context, cudaStream_t stream, t
     if (symbols > 65536)
         return {sz_unexpected_dimensions_k, "A UTF-8 call may use at most 65,536 distinct code points"};
     wide = symbols > 256; // 16-bit codes beyond 256 code points
+    // One-byte codes come from the 16-bit values where there is room for both; else, and for code points beyond the plane,
+    // from the strings again, in the values' place.
+    bool const recode = !wide && !beyond && context->utf8_ranks.reserve(ranks_bytes, stream).ok();
+    if (!recode) cudaGetLastError(); // a refused allocation leaves no error behind for the launches below
     for (int t = 0; t < 2; ++t) {
         if (!tapes[t]) continue;
         auto const *counts = reinterpret_cast<std::uint64_t const *>(area + layout[t][0]);
         auto *values = reinterpret_cast<std::uint16_t *>(area + layout[t][1]);
-        auto *bytes = reinterpret_cast<std::uint8_t *>(area + layout[t][2]);
-        if (beyond)
-            SZS_TRY_CUDA(launch_utf8_write(*tapes[t], end[t], counts, set, wide ? static_cast<void *>(values) : bytes, wide,
-                                           context->sm_count, stream));
-        else if (!wide)
+        auto *bytes = recode ? static_cast<std::uint8_t *>(context->utf8_ranks.data) + ranks_at[t]
+                             : reinterpret_cast<std::uint8_t *>(values);
+        if (recode)
             SZS_TRY_CUDA(launch_utf8_recode(*tapes[t], counts, set, values, bytes, context->sm_count, stream));
+        else if (beyond || !wide)
+            SZS_TRY_CUDA(launch_utf8_write(*tapes[t], end[t], counts, set, values, wide, context->sm_count, stream));
         // Kernels address `base + offsets[i]` (twice the offset for 16-bit codes); the codes start at offsets[0].
         tapes[t]->base = wide ? reinterpret_cast<std::uint8_t const *>(values) - 2 * first[t] : bytes - first[t];
         tapes[t]->lengths = counts;

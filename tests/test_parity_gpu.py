@@ -1499,3 +1499,25 @@ def test_short_pairs_in_quarter_octaves(szs, port, name, family, costs, letters)
     got = engine.pairwise(szs.Strs(first[:third]), szs.Strs(second[:third])).astype(np.int64)
     np.testing.assert_array_equal(got, want[:third])
     assert engine.stats()["last_launches"] < 20
+
+
+def test_utf8_scratch_of_many_code_points(szs):
+    """A UTF-8 call over more than 256 code points holds its tapes as 16-bit values and nothing else per byte (4,000 code
+    points a string: a warp per pair, which needs no scratch of its own)."""
+    import torch
+    rng = np.random.default_rng(8)
+    points = rng.integers(0, 2000, size=(2500, 4000)) + 0x4E00
+    data = np.stack([0xE0 | points >> 12, 0x80 | points >> 6 & 0x3F, 0x80 | points & 0x3F], axis=2).astype(np.uint8)
+    offsets = torch.arange(0, data.size + 1, 12000, dtype=torch.int64).cuda()
+    first = torch.from_numpy(data.reshape(-1).copy()).cuda()
+    data[:, 3000, 1] = 0xBF  # another ideograph, in every string
+    second = torch.from_numpy(data.reshape(-1).copy()).cuda()
+    out = torch.zeros(2500, dtype=torch.int64, device="cuda")
+    engine = szs.LevenshteinDistancesUTF8()
+    engine.pairwise(["a"], ["b"])  # contexts, streams and events
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    engine.pairwise(szs.Strs.from_buffers(first, offsets), szs.Strs.from_buffers(second, offsets), out=out)
+    held = before - torch.cuda.mem_get_info()[0]
+    assert set(out.cpu().numpy()) <= {0, 1}
+    assert held < 2.4 * (first.numel() + second.numel()), held
