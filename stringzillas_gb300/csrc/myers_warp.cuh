@@ -57,10 +57,15 @@ __device__ __forceinline__ std::uint32_t myers_warp_distance(pair_task_t const &
 #pragma unroll
     for (int w = 0; w < W; ++w) pv[w] = 0xFFFFFFFFu, mv[w] = 0u;
 
-    // Match mask of this lane's rows with one symbol.
+    // Match mask of this lane's rows with one symbol. Its selectors come from shared memory, but where a step is short (one
+    // word per lane) those of 8 planes, two 16-byte loads from scattered rows, keep the banks busy longer than the step
+    // itself: they are made from the bits of the code, which travels in the symbol's place (60,000 text pairs of 700-1,000
+    // 5.5 -> 4.6 ms, 30,000 of 520-700 2.06 -> 1.76; with two to four words per lane the loads are the faster way, 5,000 of
+    // 1,000-4,000 2.26 against 2.50).
+    constexpr bool codes = wide_ || (B >= 8 && W == 1);
     auto matches = [&](std::uint32_t symbol, std::uint32_t (&eq)[W]) {
         std::uint32_t select[B];
-        if constexpr (wide_) code_selectors<B>(symbol, select);
+        if constexpr (codes) code_selectors<B>(symbol, select);
         else {
 #pragma unroll
             for (int b = 0; b < B; ++b) select[b] = selectors->select[symbol][b];
@@ -72,7 +77,10 @@ __device__ __forceinline__ std::uint32_t myers_warp_distance(pair_task_t const &
             for (int b = 0; b < B; ++b) eq[w] &= planes[b][w] ^ select[b];
         }
     };
-    auto text = [&](std::uint32_t j) -> std::uint32_t { return j < m ? symbol_at<wide_>(task.cols, j) : 0u; };
+    auto text = [&](std::uint32_t j) -> std::uint32_t {
+        std::uint32_t const symbol = j < m ? symbol_at<wide_>(task.cols, j) : 0u;
+        return codes && !wide_ ? code[symbol] : symbol;
+    };
     std::uint32_t chunk = text(lane), chunk_ahead = text(32u + lane); // columns (t + 1 & ~31) + lane, and 32 later
     std::uint32_t symbol = lane == 0 ? chunk : 0u;
     std::uint32_t eq[W];

@@ -1521,3 +1521,20 @@ def test_utf8_scratch_of_many_code_points(szs):
     held = before - torch.cuda.mem_get_info()[0]
     assert set(out.cpu().numpy()) <= {0, 1}
     assert held < 2.4 * (first.numel() + second.numel()), held
+
+
+@pytest.mark.parametrize("letters", [40, 256])
+def test_warp_pairs_over_eight_planes(szs, port, letters):
+    """Unit-cost pairs of 513 to 1,024 rows over more than 32 symbols: one word per lane, whose codes travel from lane to lane
+    instead of the symbols; both sides of a lane's and the word's limits, texts a step shorter and longer than a chunk."""
+    rng = np.random.default_rng(letters)
+    alphabet = rng.permutation(256)[:letters].astype(np.uint8)
+    lengths = [(n, m) for n in (513, 543, 544, 545, 1023, 1024) for m in (n, n + 1, n + 31, 1055, 1056, 1057, 3000) if m >= n]
+    first = [bytes(rng.choice(alphabet, size=n)) for n, _ in lengths]
+    second = [bytes(rng.choice(alphabet, size=m)) for _, m in lengths]
+    second[::3] = [a[:200] + b"\x07" + a[200:] for a in first[::3]]
+    engine = szs.LevenshteinDistances()
+    sides = [szs.Strs(strings * 60) for strings in (first, second)]  # past the small host calls
+    got = engine.pairwise(*sides).astype(np.int64)
+    want = port.pairs(oracle.levenshtein_costs(), tape(first), tape(second))
+    np.testing.assert_array_equal(got, np.tile(want, 60))
