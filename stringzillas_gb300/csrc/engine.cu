@@ -907,10 +907,12 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
     // Unit costs: how alike the pairs look decides if they are tried near their diagonal first (`near_pays`). Plans made
     // before the strings have landed (pipelined chunks but the first) cannot look at them and go by the first chunk.
     bool const planned_ahead = call.scoring_after && call.plan_after != call.scoring_after;
+    std::uint64_t const near_long_pairs = (std::uint64_t)context->sm_count * 16; // a warp route's pairs at once
     args.near_sample_stride =
         engine.unit_levenshtein && schedule != szs_gb300_schedule_plain_k && !planned_ahead
             ? (std::uint32_t)std::max<std::uint64_t>(args.pairs / near_samples_k, 1)
             : 0;
+    args.near_long = args.pairs >= near_long_pairs ? 1 : 0;
     bool const levenshtein = engine.kind == kind_levenshtein_k;
     bool const dense = !engine.dense.empty();
     // Both score over the batch's own byte codes; 16-bit codes are already dense.
@@ -1348,7 +1350,7 @@ static status_t run_on(engine_t const &engine, device_context_t *context, cudaSt
             if (wide && near_job(1, one_per_lane, warp_end, std::min<std::uint32_t>(plan.max_myers_warp_rows, 1024)))
                 near_per_lane = 1;
             if (myers_planes == 2 &&
-                pairs_in(bin_myers_warp_begin_k, warp_end) >= (std::uint64_t)context->sm_count * 16 &&
+                pairs_in(bin_myers_warp_begin_k, warp_end) >= near_long_pairs &&
                 near_job(4, bin_myers_warp_begin_k, warp_end, plan.max_myers_warp_rows))
                 near_per_lane = myers_warp_max_words_k;
         }

@@ -349,6 +349,7 @@ __device__ __forceinline__ int near_likeness(plan_args_t const &args, std::uint6
     std::uint64_t const n = swap ? second_length : first_length, m = swap ? first_length : second_length;
     std::uint32_t const blocks = n <= 32u * myers_max_words_k ? 1u : 4u;
     if (n <= 32u * (near_min_words_k - 1) || n > 32u * 32u * myers_warp_max_words_k) return 0;
+    if (blocks > 1 && !args.wide && !args.near_long) return 0;
     if (m - n > 32u * blocks) return 1;
     std::uint64_t const row_at = tail ? n - 1 : 0, col_at = tail ? m - 1 : 0;
     int const direction = tail ? -1 : 1;

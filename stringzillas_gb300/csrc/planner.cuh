@@ -168,6 +168,7 @@ struct plan_args_t {
     int short_fine;                      // 1: quarter octaves of rows, where the profile has few classes
     int classes;                         // profile classes of the engine's table (not read for Levenshtein or dense)
     std::uint32_t near_sample_stride;    // unit-cost calls: every so many pairs one is sampled for likeness (0: none)
+    int near_long;                       // 1: pairs enough for the nine-word window of patterns past the thread route
 };
 
 /** What the ends of sampled pairs say about trying a call's pairs near their diagonal first (myers_near.cuh). */
