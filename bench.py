@@ -247,7 +247,7 @@ def ops_per_cell(kind_and_tables):
     return OPS_PER_CELL["packed_affine_local"] if kind == "sw" else OPS_PER_CELL["packed_affine"]
 
 
-def scored_share(first, second, kind_and_tables):
+def scored_share(first, second, kind_and_tables, sms):
     """Share of the matrices' cells that the kernels score: alike pairs of unit-cost workloads take a window of three words
     along the diagonal from five words of pattern on, nine beyond sixteen words in batches of 16 pairs per SM."""
     if kind_and_tables[0] != "lev":
@@ -255,7 +255,7 @@ def scored_share(first, second, kind_and_tables):
     a, b = np.diff(first[1]).astype(np.int64), np.diff(second[1]).astype(np.int64)
     n, m = np.minimum(a, b), np.maximum(a, b)
     words = (n + 31) // 32
-    window = np.where(words < 5, n, np.where(words <= 16, 96, n if len(n) < 16 * 152 else 288))
+    window = np.where(words < 5, n, np.where(words <= 16, 96, n if len(n) < 16 * sms else 288))
     return float((np.minimum(window, n) * m).sum() / max(1, (n * m).sum()))
 
 
@@ -851,7 +851,8 @@ def run_ours(args):
         step_compute_s = compute_ms / args.steps * 1e-3
         algorithmic_bytes = input_bytes + 8 * pairs
         achieved_gbs = algorithmic_bytes / step_compute_s / 1e9
-        share = scored_share(first, second, kind_and_tables)
+        share = scored_share(first, second, kind_and_tables,
+                             torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count)
         int_ops = cells_per_step * share * ops_per_cell(kind_and_tables)
         int_peak = None
         if peaks:
