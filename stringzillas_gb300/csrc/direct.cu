@@ -251,7 +251,8 @@ cudaError_t launch_myers_direct(tape_t const &queries, tape_t const &candidates,
     dim3 const grid(grid_x, grid_y);
     int const set = swapped ? 1 : 0;
     if (longest_rows <= 128)
-        myers_direct_kernel<1, 1, 4><<<grid, threads, 256 * direct_row_bytes(4), stream>>>(patterns, texts, set, out, stride);
+        myers_direct_kernel<1, 1, 4><<<grid, threads, 256 * direct_row_bytes(4), stream>>>(patterns, texts, set, out,
+                                                                                          stride);
     else if (longest_rows <= 512)
         myers_direct_kernel<2, 2, 16><<<grid, threads, 256 * direct_row_bytes(16), stream>>>(patterns, texts, set, out,
                                                                                             stride);

@@ -15,9 +15,10 @@
  *                direct, 21 at one and 190 to 250 at 16 planned, 90 in the warp-per-pair kernel.
  *
  *  Fitted to whole calls on a GB300, which does about 1.56e12 word-columns a second planned and an eighth more direct
- *  (800,000 pairs of 150 x 150: 457 us direct with six words each, 495 planned with five). Without it (queries as patterns whenever they fit) 1,000,000 x 1 strings of
- *  150 took 25.4 ms against 0.60 planned, 1,024 x 1,024 of which 3 % have 1,000 symbols and the others 20 2.86 ms against
- *  0.53, and 2,048 x 2,048 of log-normal lengths (median 100, sigma 0.7) 7.0 ms against 2.2.
+ *  (800,000 pairs of 150 x 150: 457 us direct with six words each, 495 planned with five). With the queries as patterns
+ *  whenever they fit, 1,000,000 x 1 strings of 150 took 25.4 ms against 0.60 planned (0.57 by this rule), 1,024 x 1,024 of
+ *  which 3 % have 1,000 symbols and the others 20 2.86 ms against 0.53, and 2,048 x 2,048 of log-normal lengths (median 100,
+ *  sigma 0.7) 7.0 ms against 2.2.
  */
 #pragma once
 #include <algorithm>

@@ -37,7 +37,9 @@ namespace szs_gb300 {
 #ifndef SZS_BAND_WARPS
 #define SZS_BAND_WARPS 8
 #endif
-constexpr int band_warps_k = SZS_BAND_WARPS; // warps per CTA
+// Warps per CTA. It differs between the builds of 8 and of 4 rows per lane, and `band_shared_t` with it: whatever depends on
+// it is a template over a policy (whose rows differ too) or device code of its own translation unit, and has to stay so.
+constexpr int band_warps_k = SZS_BAND_WARPS;
 constexpr int band_chunk_k = 32;                      // columns staged and published at a time
 
 template <int kind_, bool affine_, int rows_per_lane_, int columns_per_step_ = 1>

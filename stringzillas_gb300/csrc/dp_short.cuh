@@ -25,8 +25,8 @@
  *  max(m_A, m_B) + L - 1 steps; the warp runs its slowest segment's steps, so the planner bins these pairs by the
  *  length of their longer side.
  *
- *  Bound: the ALU pipe (82 % busy), so what is left to save is rows past a pair's end, fill steps and operations. Large
- *  batches therefore cut every octave of rows into quarters (a pair pads its rows by 9 % on average, by 17 % in halves),
+ *  Bound: the ALU pipe (82 % busy on protein profiles, 62-74 on the larger DNA shapes), so what is left to save is rows past a
+ *  pair's end, fill steps and operations. Large batches with rows enough (`short_fine_rows`) therefore cut every octave of rows into quarters (a pair pads its rows by 9 % on average, by 17 % in halves),
  *  with 16 to 28 rows per lane, and take pairs up to 448 rows from the whole-warp wavefront, whose strips of 128 to 512
  *  rows and 31 fill steps of two columns cost a pair of 130-300 rows as much again as its cells: 65,536 pairs of text of
  *  100-300 characters, affine distances, 1,030 -> 790 us per call (of 260-310: 1,730 -> 1,330); 1,048,576 DNA pairs of

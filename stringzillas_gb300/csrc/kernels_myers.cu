@@ -20,8 +20,8 @@ constexpr int myers_threads_k = 128;
 
 template <int words_>
 static cudaError_t myers_launch_words(bool exact, pair_task_t const *tasks, plan_bins_t const *bins, int key_begin,
-                                      int key_end, batch_alphabet_t const *alphabet, std::int64_t *results, std::uint32_t const *list, int ctas,
-                                      cudaStream_t stream) {
+                                      int key_end, batch_alphabet_t const *alphabet, std::int64_t *results,
+                                      std::uint32_t const *list, int ctas, cudaStream_t stream) {
     if (exact)
         myers_kernel<words_, SZS_MYERS_PLANES, true>
             <<<ctas, myers_threads_k, 0, stream>>>(tasks, bins, key_begin, key_end, alphabet, results, list);
@@ -34,7 +34,8 @@ static cudaError_t myers_launch_words(bool exact, pair_task_t const *tasks, plan
 cudaError_t SZS_CONCAT(launch_myers_planes, SZS_MYERS_PLANES)(int words, bool exact, pair_task_t const *tasks,
                                                                 plan_bins_t const *bins, int key_begin, int key_end,
                                                                 batch_alphabet_t const *alphabet,
-                                                                std::int64_t *results, std::uint32_t const *list, int ctas, cudaStream_t stream) {
+                                                                std::int64_t *results, std::uint32_t const *list,
+                                                                int ctas, cudaStream_t stream) {
     switch (words) {
     case 1: return myers_launch_words<1>(exact, tasks, bins, key_begin, key_end, alphabet, results, list, ctas, stream);
     case 2: return myers_launch_words<2>(exact, tasks, bins, key_begin, key_end, alphabet, results, list, ctas, stream);
@@ -58,8 +59,8 @@ cudaError_t SZS_CONCAT(launch_myers_planes, SZS_MYERS_PLANES)(int words, bool ex
 
 template <int words_>
 static cudaError_t myers_warp_launch_words(pair_task_t const *tasks, plan_bins_t *bins, int key_begin, int key_end,
-                                           batch_alphabet_t const *alphabet, std::int64_t *results, std::uint32_t const *list, int ctas,
-                                           cudaStream_t stream) {
+                                           batch_alphabet_t const *alphabet, std::int64_t *results,
+                                           std::uint32_t const *list, int ctas, cudaStream_t stream) {
     myers_warp_kernel<words_, SZS_MYERS_PLANES>
         <<<ctas, 256, 0, stream>>>(tasks, bins, key_begin, key_end, alphabet, results, list);
     return cudaGetLastError();
@@ -68,8 +69,8 @@ static cudaError_t myers_warp_launch_words(pair_task_t const *tasks, plan_bins_t
 cudaError_t SZS_CONCAT(launch_myers_warp_planes, SZS_MYERS_PLANES)(int words, pair_task_t const *tasks,
                                                                      plan_bins_t *bins, int key_begin, int key_end,
                                                                      batch_alphabet_t const *alphabet,
-                                                                     std::int64_t *results, std::uint32_t const *list, int ctas,
-                                                                     cudaStream_t stream) {
+                                                                     std::int64_t *results, std::uint32_t const *list,
+                                                                     int ctas, cudaStream_t stream) {
     switch (words) {
     case 1: return myers_warp_launch_words<1>(tasks, bins, key_begin, key_end, alphabet, results, list, ctas, stream);
     case 2: return myers_warp_launch_words<2>(tasks, bins, key_begin, key_end, alphabet, results, list, ctas, stream);

@@ -236,15 +236,15 @@ cudaError_t launch_myers_warp_wide(int words, pair_task_t const *tasks, plan_bin
  *  pairs may be shorter (the plain schedule puts every bit-parallel pair in one bin and launches the word count of
  *  the batch's longest pattern). */
 cudaError_t launch_myers(int words, int planes, bool exact, pair_task_t const *tasks, plan_bins_t const *bins,
-                         int key_begin, int key_end, batch_alphabet_t const *alphabet, std::int64_t *results, std::uint32_t const *list, int ctas,
-                         cudaStream_t stream);
+                         int key_begin, int key_end, batch_alphabet_t const *alphabet, std::int64_t *results,
+                         std::uint32_t const *list, int ctas, cudaStream_t stream);
 int myers_threads_per_cta();
 /** The shared-table bit-parallel kernel for batches over at most four symbol codes: bins [key_begin, key_end),
  *  patterns of at most 32 x `words` rows (1..16). A pair holding a byte outside `alphabet->present` sets bit 1 of
  *  `bins->error_flags` (its score is then not valid). */
 cudaError_t launch_myers_table(int words, int key_begin, int key_end, pair_task_t const *tasks,
-                               plan_bins_t *bins, batch_alphabet_t const *alphabet, std::int64_t *results, std::uint32_t const *list,
-                               int ctas, cudaStream_t stream);
+                               plan_bins_t *bins, batch_alphabet_t const *alphabet, std::int64_t *results,
+                               std::uint32_t const *list, int ctas, cudaStream_t stream);
 /** Planes actually instantiated for a requested minimum. */
 int myers_planes_for(int bits_needed);
 

@@ -48,8 +48,8 @@ __device__ __forceinline__ std::int64_t trivial_score(plan_args_t const &args, s
     return length == 0 ? 0 : (std::int64_t)args.open + (std::int64_t)args.extend * (std::int64_t)(length - 1);
 }
 
-/** Whether a profile over the call's symbols fits the 16x2 kernels' 32 classes, and over how many (`few`: codes are compared,
- *  or the classes are few enough for long segments). */
+/** Whether a profile over the call's symbols fits the 16x2 kernels' 32 classes, and over how many (`few`: codes are
+ *  compared, or the classes are few enough for long segments). */
 __device__ __forceinline__ bool profile_classes(plan_args_t const &args, bool &few) {
     bool const fits = (args.kind != kind_levenshtein_k && !args.dense) || (args.alphabet && args.alphabet->symbols <= 32);
     few = !fits || (args.alphabet ? (int)args.alphabet->symbols : args.classes) <= short_few_classes_k;
@@ -378,8 +378,10 @@ __global__ void __launch_bounds__(bin_keys_k / 2) plan_scan_kernel(plan_args_t c
         unsigned const unrelated = __ballot_sync(0xFFFFFFFFu, first && likeness == 1);
         unsigned const alike = __ballot_sync(0xFFFFFFFFu, first && likeness == 3);
         if (threadIdx.x == 0) {
-            atomicAdd(&bins->near.sampled, (unsigned)__popc(sampled)), atomicAdd(&bins->near.unrelated, (unsigned)__popc(unrelated));
-            atomicAdd(&bins->near.alike, (unsigned)__popc(alike)), atomicAdd(&bins->near.edits, (unsigned)sum);
+            atomicAdd(&bins->near.sampled, (unsigned)__popc(sampled));
+            atomicAdd(&bins->near.unrelated, (unsigned)__popc(unrelated));
+            atomicAdd(&bins->near.alike, (unsigned)__popc(alike));
+            atomicAdd(&bins->near.edits, (unsigned)sum);
         }
         return;
     }
@@ -612,8 +614,8 @@ cudaError_t launch_plan(plan_args_t const &args, plan_bins_t *bins, pair_task_t 
     if (args.pairs == 0) return cudaSuccess;
     status = launch_prioritised(plan_count_kernel, grid_for(args.pairs, 256, sm_count), 256, stream, args, bins, results);
     if (status != cudaSuccess) return status;
-    status = launch_prioritised(plan_scan_kernel, 1 + (args.near_sample_stride ? near_samples_k / 16 : 0), bin_keys_k / 2, stream,
-                                args, bins);
+    unsigned const sampling = args.near_sample_stride ? near_samples_k / 16 : 0; // sixteen pairs per CTA
+    status = launch_prioritised(plan_scan_kernel, 1 + sampling, bin_keys_k / 2, stream, args, bins);
     if (status != cudaSuccess) return status;
     return launch_prioritised(plan_scatter_kernel, grid_for(args.pairs, 256, sm_count), 256, stream, args, bins, tasks);
 }

@@ -68,8 +68,8 @@ constexpr int short_profile_rows_k = 192; // the same for large batches whose pr
 constexpr int short_row_maxima_k = 3;  // beside the compare modes: local scores with positive gap costs (dp_short.cuh)
 constexpr std::uint64_t short_row_maxima_pairs_k = 12288; // pairs from which those take the short route
 constexpr int short_few_classes_k = 8; // profiles over at most this many classes fit segments of 16-28 rows per lane
-/** Pairs, and cells by the mean sides of 32 of them, from which a call cuts its short pairs' rows in quarter octaves instead of
- *  halves and takes longer ones: 655e6 cells of text pairs of 100-300 took 334 us either way (340 here), 800e6 384 -> 370
+/** Pairs, and cells by the mean sides of 32 of them, from which a call cuts its short pairs' rows in quarter octaves
+ *  instead of halves and takes longer ones: 655e6 cells of text pairs of 100-300 took 334 us either way (340 here), 800e6 384 -> 370
  *  and 1.3e9 573 -> 515; 340e6 cells of DNA pairs of 16-128 226 -> 263. */
 constexpr std::uint64_t short_fine_pairs_k = 1 << 14;
 constexpr float short_fine_cells_k = 800e6f;
